@@ -710,7 +710,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   const bool persist = plain_riemann && ctx->wave_persist != 0;
   // face scratch: planes of every grid, then the flagged-pencil list
   std::vector<SweepArgs> rec(ng);
-  std::vector<int64_t> mpre(ng + 1, 0), rpre(ng + 1, 0), fpre(ng + 1, 0);
+  std::vector<int64_t> mpre(ng + 1, 0), rpre(ng + 1, 0), fpre(ng + 1, 0), gpre(ng + 1, 0);
   // the fused face kernel serves the same plain two-shock path, without slope corrections
   const bool fused = plain_riemann && ctx->sweep_mode == PPM_B200_SWEEP_FUSED &&
                      correction_planes(p) == 0;
@@ -758,6 +758,15 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
     mpre[k + 1] = mpre[k] + mb;
     rpre[k + 1] = rpre[k] + rb;
     fpre[k + 1] = fpre[k] + ppm::face_blocks(a.npencils, a.is, a.ie);
+  }
+  // the marching stages' segments, once the batch's pencils are known
+  bool uneven = false;
+  const bool local_select = !p->dual_energy || p->eta1 <= 0.25 * p->eta2;
+  for (int k = 0; k < ng; ++k) {
+    ppm::set_segments(rec[k], total_pencils, local_select);
+    ppm::set_uniform(rec[k], io[k].g->cell_width[dim], ct.all.data() + ct.offset[k]);
+    uneven = uneven || !rec[k].uniform;
+    gpre[k + 1] = gpre[k] + ppm::march_segment_blocks(rec[k]);
   }
   // callers that queue several sweeps size the scratch for all of them first, so this
   // never moves the buffer under a sweep prepared earlier
@@ -878,6 +887,9 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   const size_t off_f = align256(img.size());
   img.resize(off_f);
   append(img, fpre.data(), fpre.size());
+  const size_t off_g = align256(img.size());
+  img.resize(off_g);
+  append(img, gpre.data(), gpre.size());
   const int slot = kSlotSweep0 + 3 * dim + position;
   rc = mirror_put(ctx, ctx->mirror[slot], img);
   if (rc) return rc;
@@ -885,9 +897,14 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   std::memset(&plan.B.one, 0, sizeof(plan.B.one));
   if (ng == 1) plan.B.one = rec[0];
   plan.B.x_tma = 0;
-  if (ng == 1 && dim == 0) set_x_tiles(plan.B, rec[0]);
+  // the x sweep's staged update works on warps of 32 pencils
+  bool whole_warps = true;
+  for (int k = 0; k < ng; ++k) whole_warps = whole_warps && rec[k].pw_log2 >= 5;
+  plan.contiguous = dim == 0 && whole_warps;
+  if (ng == 1 && plan.contiguous) set_x_tiles(plan.B, rec[0]);
   plan.B.x_tma_extra_tx = plan.B.x_tma ? ctx->debug_tma_extra : 0u;
   plan.B.corrections = correction_planes(p) > 0 ? 1 : 0;
+  plan.B.uneven = uneven ? 1 : 0;
   plan.B.ncolour = nc;
   plan.B.solver = solver_code(p);
   plan.B.presfree = p->pressure_free == 1 ? 1 : 0;
@@ -897,6 +914,8 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.ngrids = ng;
   plan.B.march_prefix = (const int64_t*)(base + off_m);
   plan.B.riemann_prefix = (const int64_t*)(base + off_r);
+  plan.B.seg_prefix = (const int64_t*)(base + off_g);
+  plan.B.seg_blocks = gpre[ng];
   plan.B.counters = (unsigned long long*)ctx->counters.p;
   plan.B.flagged = (int64_t*)(scratch + scratch_doubles);
   plan.march_blocks = mpre[ng];
@@ -914,7 +933,6 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
     plan.riemann_blocks = std::min<int64_t>(
         rpre[ng], (int64_t)ctx->sms *
                       ppm::riemann_resident_blocks(p->dual_energy != 0, ng == 1, rt));
-  plan.contiguous = dim == 0;
   return PPM_B200_OK;
 }
 
@@ -1471,6 +1489,8 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, b.ngrids);
     key_put(k, b.march_prefix);
     key_put(k, b.riemann_prefix);
+    key_put(k, b.seg_prefix);
+    key_put(k, b.seg_blocks);
     key_put(k, b.counters);
     key_put(k, b.flagged);
     key_put(k, sp.sweep[s].march_blocks);
@@ -1479,6 +1499,7 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, b.x_tma);
     key_put(k, b.x_tma_extra_tx);
     key_put(k, b.corrections);
+    key_put(k, b.uneven);
     key_put(k, b.ncolour);
     key_put(k, b.solver);
     key_put(k, b.presfree);

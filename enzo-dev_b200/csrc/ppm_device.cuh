@@ -763,4 +763,21 @@ __device__ __forceinline__ void pgas2d_dual(Cell& c, double de_m, double de_p, c
   c.e = c.e - ge1 + ge2;
 }
 
+// The energy per volume d*e that pgas2d_dual leaves in cell c, without its neighbours.
+// They enter only through demax >= d*e of the cell itself, in the test ge1*d/demax > eta2
+// that replaces ge by ge1.  The total energy does not depend on that test where
+// ge1/e > eta1 (it is rebuilt from ge1 either way), nor where ge1*d/(d*e) is below eta2
+// (then no larger demax can pass it; half of eta2 leaves room for rounding).  known =
+// false: neither holds, and the neighbours decide.
+__device__ __forceinline__ double pgas2d_de_local(const Cell& c, const Phys& P, bool& known) {
+  double ke = 0.5 * (c.u * c.u + c.v * c.v + c.w * c.w);
+  double ge1 = c.e - ke;
+  const double own = c.d * c.e;
+  const bool rebuilt = qdiv(ge1, c.e) > P.eta1;
+  known = rebuilt || (own > 0.0 && qdiv(ge1 * c.d, own) <= 0.5 * P.eta2);
+  double ge2 = rebuilt ? ge1 : c.ge;
+  ge2 = dmax(ge2, qdiv(P.pmin, P.gm1 * c.d));
+  return c.d * (c.e - ge1 + ge2);
+}
+
 }  // namespace ppm

@@ -59,7 +59,7 @@ constexpr size_t kStaticPlaneBytes = size_t(48) << 20;            // interface s
 constexpr size_t kStaticBytes =
     kStaticCounterBytes + kStaticCoefBytes + kStaticDescBytes + kStaticPlaneBytes;
 static_assert(kStaticCoefEntries * sizeof(ppm::Coef) <= kStaticCoefBytes, "coef area");
-static_assert(sizeof(ppm::SweepArgs) <= 512, "descriptor area");
+static_assert(sizeof(ppm::SweepArgs) <= 768, "the record's place in the descriptor area");
 static_assert(ppm::kMaxCounters * sizeof(unsigned long long) <= kStaticCounterBytes, "counters");
 
 constexpr int kMaxDevices = 64;
@@ -252,25 +252,33 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   const int64_t march_blocks = (a.npencils + ppm::kMarchThreads - 1) / ppm::kMarchThreads;
   const int64_t riemann_blocks =
       (int64_t)(a.ie - a.is + 2) * ((a.npencils + ppm::kRiemannThreads - 1) / ppm::kRiemannThreads);
+  ppm::set_segments(a, a.npencils, !p->dual_energy || p->eta1 <= 0.25 * p->eta2);
+  ppm::set_uniform(a, in->cell_width[dim], table.data());
+  const int64_t seg_blocks = ppm::march_segment_blocks(a);
+  const int64_t mpre[2] = {0, march_blocks}, rpre[2] = {0, riemann_blocks},
+                gpre[2] = {0, seg_blocks};
   unsigned char img[kStaticDescBytes];
   std::memset(img, 0, sizeof(img));
   std::memcpy(img, &a, sizeof(a));
-  const int64_t mpre[2] = {0, march_blocks}, rpre[2] = {0, riemann_blocks};
-  std::memcpy(img + 512, mpre, sizeof(mpre));
-  std::memcpy(img + 768, rpre, sizeof(rpre));
+  std::memcpy(img + 768, mpre, sizeof(mpre));
+  std::memcpy(img + 832, rpre, sizeof(rpre));
+  std::memcpy(img + 896, gpre, sizeof(gpre));
   e = cudaMemcpyAsync(desc, img, sizeof(img), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpyAsync");
   ppm::BatchArgs B;
   B.one = a;
   B.grids = reinterpret_cast<const ppm::SweepArgs*>(desc);
   B.ngrids = 1;
-  B.march_prefix = reinterpret_cast<const int64_t*>(desc + 512);
-  B.riemann_prefix = reinterpret_cast<const int64_t*>(desc + 768);
+  B.march_prefix = reinterpret_cast<const int64_t*>(desc + 768);
+  B.riemann_prefix = reinterpret_cast<const int64_t*>(desc + 832);
+  B.seg_prefix = reinterpret_cast<const int64_t*>(desc + 896);
+  B.seg_blocks = seg_blocks;
+  B.uneven = a.uniform ? 0 : 1;
   B.counters = counters;
   B.flagged = reinterpret_cast<int64_t*>(planes + (size_t)(ppm::kFaceVars + ppm::kFluxVars) *
                                                       (size_t)a.plane);
   ppm::launch_sweep_batch(B, march_blocks, riemann_blocks, p->dual_energy != 0, p->gravity != 0,
-                          st, nullptr, false, dim == 0);
+                          st, nullptr, false, dim == 0 && a.pw_log2 >= 5);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail_cuda(e, "sweep launch");
 

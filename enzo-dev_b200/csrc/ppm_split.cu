@@ -36,6 +36,14 @@ enum { XDF = 0, XEF, XUF, XVF, XWF, XGEF, XUB };
 __device__ __forceinline__ double ldg0(const double* __restrict__ p, int64_t off) {
   return p ? __ldg(p + off) : 0.0;
 }
+// A field, and a face plane, holds fewer than 2^31 elements (at most 1031 cells a side),
+// so the marches index with 32 bits: one multiply-add per address instead of two 64-bit
+// additions (the segments made the indices differ between warps, and 64-bit arithmetic on
+// them had cost the v/w/ge march 12 % at 512^3).
+__device__ __forceinline__ int pencil_base(const SweepArgs& a, int pid) {
+  const int t2 = pid / a.n1;
+  return (pid - t2 * a.n1) * (int)a.s1 + t2 * (int)a.s2;
+}
 
 // Every thread of a block works on the same grid.  A batch of one grid (ONE) reads its
 // record from the kernel parameters, where the compiler uses the fields as constant
@@ -167,16 +175,25 @@ __global__ void __launch_bounds__(kMarchThreads) corrections_kernel(const __grid
 #ifndef PPM_RECON_PREFETCH
 #define PPM_RECON_PREFETCH 1
 #endif
-// COR: the batch carries slope corrections (the coefficients of the corrections kernel).
-// One pencil's march (the body of the reconstruct kernels).
+// COR: the batch carries slope corrections (the coefficients of the corrections kernel),
+// or is one of the other cases that are not the plain path: colours, PressureFree, cell
+// widths that differ along the sweep.  Without it every cell shares the coefficients a.uc,
+// constant operands instead of eight loads a step.
+// The march of one pencil segment, faces f0 .. f1 (the body of the reconstruct kernels):
+// it starts three cells left of f0 and repeats there what the segment before it computed
+// (a prep, two slopes, an edge, a parabola's right side), the same expressions on the
+// same cells.
 template <bool DUAL, bool GRAV, int ROLE, bool COR>
-__device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t pid) {
+__device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int pid, int f0,
+                                                   int f1) {
   constexpr int NV = (ROLE == 0) ? 3 : (DUAL ? 3 : 2);
   const Phys P = make_phys(a);
-  const int64_t base = (pid % a.n1) * a.s1 + (pid / a.n1) * a.s2;
-  const int64_t sa = a.sa;
-  const int is = a.is, ie = a.ie;
-  const int64_t np = a.npencils, plane = a.plane;
+  const int base = pencil_base(a, pid);
+  const int sa = (int)a.sa;
+  const int is = f0, ie = f1 - 1;  // the march's own first face and last cell
+  const int fs0 = a.is;            // face of the scratch planes' first row
+  const int np = (int)a.npencils;
+  const int64_t plane = a.plane;
   // the role's variables: ROLE 0 (d, p, u), ROLE 1 (v, w, ge)
   const double* q0p = ROLE == 0 ? a.in_d : a.in_v;
   const double* q1p = ROLE == 0 ? a.pres : a.in_w;
@@ -196,11 +213,11 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
   double lda = 0.0, ld0 = 0.0;
   AdvL aLp = {};   // left data of face t-2 (ROLE 1)
 
-  const int tend = ie + 3;  // the last face, ie+1, is assembled at t = ie+3
+  const int tend = ie + 3;  // the last face, f1, is assembled at t = f1+2
   // the next cell's loads (PPM_RECON_PREFETCH)
   double xq[3] = {0.0, 0.0, 0.0}, xu = 0.0, xg = 0.0, xd = 0.0, xp = 0.0;
   auto fetch = [&](const int t) {
-    const int64_t off = base + (int64_t)t * sa;
+    const int off = base + t * sa;
     xq[0] = ldg0(q0p, off);
     xq[1] = ldg0(q1p, off);
     xq[2] = ldg0(q2p, off);
@@ -217,7 +234,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
   auto step = [&](const int t, auto steady) {
     constexpr bool ST = decltype(steady)::value;
     constexpr bool PF = ST && PPM_RECON_PREFETCH;
-    const int64_t off = base + (int64_t)t * sa;
+    const int off = base + t * sa;
     double nq[3];
     nq[0] = PF ? xq[0] : ldg0(q0p, off);
     nq[1] = PF ? xq[1] : ldg0(q1p, off);
@@ -231,8 +248,8 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
     if (ST || (t >= is - 1 && t <= ie + 1)) {
       const double nd = ROLE == 0 ? nq[0] : (PF ? pd : __ldg(a.in_d + off));
       const double npr = ROLE == 0 ? nq[1] : (PF ? pp : __ldg(a.pres + off));
-      prC = (COR && a.presfree) ? cell_prep<true>(nd, npr, nu, a.coef[t].dx2i, P)
-                                : cell_prep(nd, npr, nu, a.coef[t].dx2i, P);
+      prC = (COR && a.presfree) ? cell_prep<true>(nd, npr, nu, (COR ? a.coef[t].dx2i : a.uc.dx2i), P)
+                                : cell_prep(nd, npr, nu, (COR ? a.coef[t].dx2i : a.uc.dx2i), P);
     }
     // slope and left edge of cell t-1 (intvar.F:82-102)
     double dqN[3], qlN[3];
@@ -241,7 +258,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
     {
       const int c = t - 1;
       if (ST || (c >= is - 2 && c <= ie + 2)) {
-        const Coef cf = a.coef[c];
+        const Coef& cf = COR ? a.coef[c] : a.uc;
 #pragma unroll
         for (int v = 0; v < NV; ++v) dqN[v] = pm_slope(wq1[v], wq2[v], nq[v], cf.c1, cf.c2);
         if (ST || c >= is - 1) {
@@ -262,7 +279,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
 #pragma unroll
         for (int v = 0; v < 3; ++v) pa[v] = Para{0.0, 0.0, 0.0, 0.0};
         if (COR) {
-          const int64_t co = (int64_t)(c - (is - 1)) * np + pid;
+          const int co = (c - (fs0 - 1)) * np + pid;
           const bool fl_on = a.flatten != 0, st_on = ROLE == 0 && a.steepen != 0;
           const double fl = fl_on ? a.flat[co] : 0.0;
 #pragma unroll
@@ -284,7 +301,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
 #pragma unroll
           for (int v = 0; v < NV; ++v) pa[v] = pm_parabola(wq0[v], wq1[v], wq2[v], qlm1[v], qlN[v]);
         }
-        double* o = a.fstate + (int64_t)(c - is) * np + pid;
+        double* o = a.fstate + (c - fs0) * np + pid;
         if (ROLE == 0) {
           // cell c's left edge gives the right side of face c, its right edge the left
           // side of face c+1; each side is solved on its own (face_side), the left one
@@ -300,7 +317,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
             const SideOut r = face_side<DUAL, GRAV, false>(Rin, GRAV ? (wg0 + wg1) : 0.0, P);
             double dl = sLp.d, dr = r.d;
             if (COR && a.fcol) {  // colours: what their face states need (kColVars planes)
-              double* oc = a.fcol + (int64_t)(c - is) * np + pid;
+              double* oc = a.fcol + (c - fs0) * np + pid;
               oc[CDLA * plane] = lda;
               oc[CDL0 * plane] = ld0;
               oc[CDRA * plane] = Rin.da;
@@ -388,7 +405,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int64_t p
   using Steady = std::integral_constant<bool, true>;
   const int t_steady0 = is + 2, t_steady1 = ie + 1;
 #pragma unroll 1
-  for (int t = 0; t < t_steady0 && t <= tend; ++t) step(t, Ramp{});
+  for (int t = f0 - 3; t < t_steady0 && t <= tend; ++t) step(t, Ramp{});
   if (PPM_RECON_PREFETCH && t_steady0 <= t_steady1) fetch(t_steady0);
 #pragma unroll 1
   for (int t = t_steady0; t <= t_steady1; ++t) step(t, Steady{});
@@ -409,16 +426,19 @@ __global__ void __launch_bounds__(kMarchThreads,
          k < nflag; k += (unsigned long long)gridDim.x * blockDim.x) {
       const int64_t code = B.flagged[k];
       const SweepArgs& a = ONE ? B.one : B.grids[(int)(code >> 40)];
-      reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, code & ((int64_t(1) << 40) - 1));
+      reconstruct_pencil<DUAL, GRAV, ROLE, COR>(
+          a, (int)(code & ((int64_t(1) << 40) - 1)), a.is, a.ie + 1);
     }
     return;
   }
   int64_t lb;
-  const int g = locate<ONE>(B.march_prefix, B.ngrids, lb);
+  const int g = locate<ONE>(B.seg_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
-  const int64_t pid = lb * kMarchThreads + threadIdx.x;
-  if (pid >= a.npencils) return;
-  reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, pid);
+  const int pid = (int)(lb << a.pw_log2) + (threadIdx.x & ((1 << a.pw_log2) - 1));
+  const int f0 = a.is + (int)(threadIdx.x >> a.pw_log2) * a.seg_faces;
+  if (pid >= a.npencils || f0 > a.ie + 1) return;
+  const int f1 = f0 + a.seg_faces - 1;
+  reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, pid, f0, f1 < a.ie + 1 ? f1 : a.ie + 1);
 }
 
 template <bool DUAL>
@@ -1045,11 +1065,11 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // ring: this thread's column of the block's ring (ring[v * kMarchThreads] is value v)
 template <bool DUAL, int PD>
-__device__ __forceinline__ void pipe_issue(const SweepArgs& a, double* ring, int64_t base,
-                                           int64_t pid, int s) {
-  if (s < a.n) {
+__device__ __forceinline__ void pipe_issue(const SweepArgs& a, double* ring, int base, int pid,
+                                           int s, int last) {
+  if (s <= last) {
     double* r = ring + (s % (PD + 1)) * (kUnitVals * kMarchThreads);
-    const int64_t off = base + (int64_t)s * a.sa;
+    const int off = base + s * (int)a.sa;
     cp_async8(r, a.in_d + off);
     cp_async8(r + kMarchThreads, a.in_e + off);
     if (a.in_u) cp_async8(r + 2 * kMarchThreads, a.in_u + off);
@@ -1057,7 +1077,7 @@ __device__ __forceinline__ void pipe_issue(const SweepArgs& a, double* ring, int
     if (a.in_w) cp_async8(r + 4 * kMarchThreads, a.in_w + off);
     if (DUAL) cp_async8(r + 5 * kMarchThreads, a.in_ge + off);
     if (s >= a.is && s <= a.ie) {
-      const double* f = a.fflux + (int64_t)(s + 1 - a.is) * a.npencils + pid;
+      const double* f = a.fflux + (s + 1 - a.is) * (int)a.npencils + pid;
       const int64_t pl = a.plane;
       cp_async8(r + 6 * kMarchThreads, f + XDF * pl);
       cp_async8(r + 7 * kMarchThreads, f + XEF * pl);
@@ -1068,7 +1088,7 @@ __device__ __forceinline__ void pipe_issue(const SweepArgs& a, double* ring, int
       cp_async8(r + 12 * kMarchThreads, f + XUB * pl);
     }
   }
-  cp_async_commit();  // one group per unit, empty past the pencil's end
+  cp_async_commit();  // one group per unit, empty past the segment's end
 }
 
 template <bool DUAL>
@@ -1145,10 +1165,12 @@ struct XTiles {
   unsigned fields;              // bit f: input field f present
   unsigned bytes;               // bytes of one chunk (all present fields)
   int row0;                     // the warp's first pencil
-  int last;                     // last chunk issued, -1: none
+  int q0;                       // the segment's first chunk (chunk q uses buffer (q - q0) % kXBuffers)
+  int last;                     // last chunk issued, relative to q0; -1: none
   bool broken;                  // a wait gave up: no further copies
 };
 
+// chunks q count from the segment's first
 __device__ __forceinline__ void x_issue(XTiles& x, int q) {
   const int b = q % kXBuffers;
   if ((threadIdx.x & 31) == 0) {
@@ -1156,17 +1178,17 @@ __device__ __forceinline__ void x_issue(XTiles& x, int q) {
 #pragma unroll
     for (int f = 0; f < 6; ++f)
       if (x.fields & (1u << f))
-        tma_load_2d(x.buf + (b * 6 + f) * kXTile, x.map + f, q * kXTileCells, x.row0, x.bar + b);
+        tma_load_2d(x.buf + (b * 6 + f) * kXTile, x.map + f, (x.q0 + q) * kXTileCells, x.row0, x.bar + b);
   }
   x.last = q;
 }
 
-// warp-uniform: called by every lane at the first step of chunk q (t = q * kXTileCells)
+// warp-uniform: called by every lane at its first step in chunk q; n: cells end (exclusive)
 __device__ __forceinline__ void x_chunk(XTiles& x, int q, int n) {
   __syncwarp();  // every lane has read chunk q-1, whose buffer the next copy reuses
   if (x.broken) return;
   const int next = q + kXBuffers - 1;
-  if (next * kXTileCells < n) x_issue(x, next);
+  if ((x.q0 + next) * kXTileCells < n) x_issue(x, next);
   const bool ok = mbar_wait_bounded(x.bar + q % kXBuffers, (unsigned)(q / kXBuffers) & 1u);
   if (__any_sync(0xffffffffu, !ok)) {
     x.broken = true;
@@ -1185,7 +1207,7 @@ __device__ __forceinline__ void x_drain(XTiles& x) {
 
 template <bool DUAL>
 __device__ __forceinline__ Cell x_cell(const XTiles& x, const SweepArgs& a, int t) {
-  const double* r = x.buf + ((t / kXTileCells) % kXBuffers) * (6 * kXTile) +
+  const double* r = x.buf + ((t / kXTileCells - x.q0) % kXBuffers) * (6 * kXTile) +
                     (threadIdx.x & 31) * kXTileCells + t % kXTileCells;
   Cell c;
   c.d = r[0];
@@ -1265,6 +1287,11 @@ __device__ __noinline__ void hll_fallback(const SweepArgs& a, int64_t pid, int64
 // the reference's order: all checks and fallbacks of a pencil precede its update, and
 // a fallback of cell i changes the right face of cell i-1.
 //
+// A segment's outputs are cells c0 .. c1 of the pencil (the whole pencil: 0 .. n-1).  It
+// also checks and updates cells c0-1 and c1+1, whose post-euler states its first and last
+// selects need.  The select of cell c reads the energy its left neighbour ended with, a
+// chain along the pencil that a segment cuts at c0-1: see pgas2d_de_local.
+//
 // FALLBACK = false is the hot pass: it stops at the first cell that fails its check
 // and flags the pencil; FALLBACK = true re-runs flagged pencils with the per-cell HLL
 // fallback.  Sweeps are out of place, so the re-run reads untouched inputs and
@@ -1280,7 +1307,7 @@ struct UpdateCounts {
 // Roles -> axes: the sweep velocity u is v[dim], v is v[dim+1], w is v[dim+2].
 template <bool DUAL>
 __device__ __forceinline__ double cell_dt1(const SweepArgs& a, const Cell& o, double dx_sweep,
-                                           int64_t t1, int64_t t2, const Phys& P) {
+                                           int t1, int t2, const Phys& P) {
   // axis x, y, z of the sweep's (u, v, w) and cell widths: (sweep, t1, t2) axes are
   // (x, y, z), (y, x, z) and (z, x, y) -- as selects, not a dynamically indexed array
   const int dim = a.dim;
@@ -1337,16 +1364,16 @@ constexpr int kStageWarp = 6 * kStageField;  // doubles per warp
 // stage: this warp's buffer; pid0: the warp's first pencil
 template <bool DUAL>
 __device__ __forceinline__ void flush_stage(const SweepArgs& a, const double* stage,
-                                            int64_t pid0, int c0, int ncells) {
+                                            int pid0, int c0, int ncells) {
   __syncwarp();  // every lane has staged its cells
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int r = 0; r < kStageCells; ++r) {
     const int q = lane + 32 * r;
     const int j = q % kStageCells, p = q / kStageCells;
-    const int64_t pid = pid0 + p;
+    const int pid = pid0 + p;
     if (j < ncells && pid < a.npencils) {
-      const int64_t off = (pid % a.n1) * a.s1 + (pid / a.n1) * a.s2 + (c0 + j);  // sa == 1
+      const int off = pencil_base(a, pid) + (c0 + j);  // sa == 1
       const double* sp = stage + j * kStageLd + p;
       a.out_d[off] = sp[0];
       a.out_e[off] = sp[kStageField];
@@ -1372,18 +1399,22 @@ __device__ __forceinline__ void flush_stage(const SweepArgs& a, const double* st
 // XT (x sweep of a single grid, with STAGED): the input cells arrive as TMA tiles (xt).
 template <bool DUAL, bool GRAV, bool FALLBACK, bool STAGED = false, int PD = 0, bool XT = false,
           bool RS = false>
-__device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, const Phys& P,
-                                              UpdateCounts& cnt, bool valid = true,
-                                              double* stage = nullptr, int64_t pid0 = 0,
+__device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const Phys& P,
+                                              UpdateCounts& cnt, int c0, int c1,
+                                              bool valid = true,
+                                              double* stage = nullptr, int pid0 = 0,
                                               double* ring = nullptr, XTiles* xt = nullptr) {
   bool live = valid, flagged = false;
-  const int64_t base = live ? (pid % a.n1) * a.s1 + (pid / a.n1) * a.s2 : 0;
-  const int64_t t1 = pid % a.n1, t2 = pid / a.n1;
+  const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
+  const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
   // the pencil's cells are active across the sweep (calc_dt covers active cells only)
   const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
   double dtmin = 1.0e20;
-  const int64_t sa = a.sa, np = a.npencils;
+  const int sa = (int)a.sa, np = (int)a.npencils;
+  const double qdx = P.dt / a.uc.dx;  // dt/dx of every cell (a.uniform)
   const int n = a.n, is = a.is, ie = a.ie;
+  // the segment's outputs are cells c0 .. c1; it reads cells cb .. ce
+  const int cb = c0 > 0 ? c0 - 1 : 0, ce = c1 < n - 1 ? c1 + 1 : n - 1;
 
   int64_t cap = 0, cap_end = 0;
   if (a.ncaptures > 0) {
@@ -1394,11 +1425,15 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
     }
     cap = cap_end = lo;
     while (cap_end < a.ncaptures && a.captures[cap_end].pencil == pid) ++cap_end;
+    while (cap < cap_end && a.captures[cap].face < c0) ++cap;
   }
 
   Flux Fm = {0, 0, 0, 0, 0, 0, 0};  // final flux at face t-1
   Flux F0 = Fm;                     // flux at face t (face is while t <= is)
-  if (live) F0 = load_flux(a, pid);
+  if (live) {
+    const int f = cb < is ? is : (cb > ie + 1 ? ie + 1 : cb);
+    F0 = load_flux(a, (f - is) * np + pid);
+  }
   Cell Cm = {0, 0, 0, 0, 0, 0};     // input state of cell t-1
   double ges_m = 0.0;               // final ges of cell t-1
   bool gov = false;                 // ges(t) was set by the fallback of cell t-1
@@ -1413,49 +1448,53 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
   if (live) {
     if (PIPE) {
 #pragma unroll
-      for (int u = 0; u < PD; ++u) pipe_issue<DUAL, PD>(a, ring, base, pid, u);
+      for (int u = 0; u < PD; ++u) pipe_issue<DUAL, PD>(a, ring, base, pid, cb + u, ce);
     } else {
-      if (!XT) Cpf = STAGED ? load_cell_keep<DUAL>(a, base) : load_cell<DUAL>(a, base);
-      if (0 >= is && 0 <= ie) Fpf = load_flux(a, (int64_t)(1 - is) * np + pid);
+      const int off = base + cb * sa;
+      if (!XT) Cpf = STAGED ? load_cell_keep<DUAL>(a, off) : load_cell<DUAL>(a, off);
+      if (cb >= is && cb <= ie) Fpf = load_flux(a, (cb + 1 - is) * np + pid);
     }
   }
   if (XT) {  // warp-wide, live or not: the first chunks
-    for (int q = 0; q < kXBuffers - 1 && q * kXTileCells < n; ++q) x_issue(*xt, q);
+    xt->q0 = cb / kXTileCells;
+    for (int q = 0; q < kXBuffers - 1 && (xt->q0 + q) * kXTileCells <= ce; ++q) x_issue(*xt, q);
   }
 
-  // One step of the march.  ST (steady): t in [is+2, ie-1], where cell t, face t+1 and
-  // cells t-1, t-2 are all inside the ranges every stage tests, so the tests drop out.
+  // One step of the march.  ST (steady): t in [is+2, ie-1] and [c0+2, c1], where cell t,
+  // face t+1 and cells t-1, t-2 are all inside the ranges every stage tests, so the tests
+  // drop out.
   bool handed = false;  // the pencil went to the fallback pass
   auto step = [&](const int t, auto steady) {
     constexpr bool ST = decltype(steady)::value;
-    if (XT && (ST || t < n) && t % kXTileCells == 0) x_chunk(*xt, t / kXTileCells, n);
+    if (XT && (ST || t <= ce) && (t % kXTileCells == 0 || (!ST && t == cb)))
+      x_chunk(*xt, t / kXTileCells - xt->q0, ce + 1);
     Cell Cn = Cm;
     double ges_n = 0.0;
     Flux F1 = F0;
     bool gov_next = false;
     double govv_next = 0.0;
     // (1) check of cell t
-    if (live && (ST || t < n)) {
+    if (live && (ST || t <= ce)) {
       if (PIPE) {
         cp_async_wait<(PD > 0 ? PD - 1 : 0)>();  // unit t has landed, t+1 .. t+PD-1 may not
         const double* r = ring + (t % (PD + 1)) * (kUnitVals * kMarchThreads);
         Cn = pipe_cell<DUAL>(a, r);
         if (ST || (t >= is && t <= ie)) F1 = pipe_flux(r);
-        pipe_issue<DUAL, PD>(a, ring, base, pid, t + PD);  // into the slot read at t-1
+        pipe_issue<DUAL, PD>(a, ring, base, pid, t + PD, ce);  // into the slot read at t-1
       } else {
         Cn = XT ? x_cell<DUAL>(*xt, a, t) : Cpf;
         if (ST || (t >= is && t <= ie)) F1 = Fpf;
-        if (ST || t + 1 < n) {
+        if (ST || t + 1 <= ce) {
           if (!XT)
-            Cpf = STAGED ? load_cell_keep<DUAL>(a, base + (int64_t)(t + 1) * sa)
-                         : load_cell<DUAL>(a, base + (int64_t)(t + 1) * sa);
-          if (ST || (t + 1 >= is && t + 1 <= ie)) Fpf = load_flux(a, (int64_t)(t + 2 - is) * np + pid);
+            Cpf = STAGED ? load_cell_keep<DUAL>(a, base + (t + 1) * sa)
+                         : load_cell<DUAL>(a, base + (t + 1) * sa);
+          if (ST || (t + 1 >= is && t + 1 <= ie)) Fpf = load_flux(a, (t + 2 - is) * np + pid);
         }
       }
       if (ST || (t >= is && t <= ie)) {
         if (DUAL) {
           const double pcent = dmax(P.gm1 * Cn.ge * Cn.d, kTiny);
-          ges_n = gov ? govv : (RS ? F0.ub : P.dt / a.coef[t].dx * pcent * (F0.ub - F1.ub));
+          ges_n = gov ? govv : (RS ? F0.ub : (a.uniform ? qdx : P.dt / a.coef[t].dx) * pcent * (F0.ub - F1.ub));
         }
         // RS (HLL, HLLC): flux_hll.F:336 / flux_hllc.F:332 test the density alone
         const bool bad = RS ? (Cn.d + F0.df - F1.df <= 0.0)
@@ -1487,7 +1526,8 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
           }
         }
         // subgrid flux capture: faces t (and ie+1 after the last check) are final
-        while (cap < cap_end && a.captures[cap].face <= t + (t == ie ? 1 : 0)) {
+        while (cap < cap_end && (ST || t <= c1) &&
+               a.captures[cap].face <= t + (t == ie ? 1 : 0)) {
           const FluxCapture& rq = a.captures[cap];
           const Flux& F = (rq.face == t) ? F0 : F1;
           double* dst = a.capture_buf + rq.dst;
@@ -1501,18 +1541,33 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
     Cell PEn = Cm;
     if (live) {
       const int c = t - 1;
-      if (ST || (c >= is && c <= ie)) {
+      if (ST || (c >= is && c <= ie && c >= cb)) {
         bool fatal = false;
         PEn = euler_update<DUAL, GRAV>(Cm, Fm, F0, ges_m,
-                                       GRAV ? __ldg(a.grav + base + (int64_t)c * sa) : 0.0, P,
+                                       GRAV ? __ldg(a.grav + base + c * sa) : 0.0, P,
                                        fatal);
-        if (fatal) cnt.fatal += 1;
+        if (fatal && (ST || (c >= c0 && c <= c1))) cnt.fatal += 1;
       }
     }
     // (3) dual-energy select of cell t-2 and store
     {
       const int c = t - 2;
-      if (live && (ST || c >= 0)) {
+      if (DUAL && !FALLBACK && !ST && live && c == c0 - 1 && c0 > 0) {
+        // the energy this cell ends with, without its own left neighbour; if that is not
+        // enough to know it, the fallback pass marches the whole pencil
+        bool known;
+        dep = pgas2d_de_local(PEm, P, known);
+        if (!known) {
+          if (!STAGED) {
+            if (PIPE) cp_async_wait<0>();
+            handed = true;
+            return;
+          }
+          live = false;
+          flagged = true;
+        }
+      }
+      if (live && (ST || c >= c0)) {
         Cell o = PEm;
         if (DUAL) {
           const double own = o.d * o.e;
@@ -1523,7 +1578,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
         }
         if (!isfinite(o.d) || !isfinite(o.e)) nonfin += 1;
         if (cfl && (ST || (c >= is && c <= ie)))
-          dtmin = dmin(dtmin, cell_dt1<DUAL>(a, o, a.coef[c].dx, t1, t2, P));
+          dtmin = dmin(dtmin, cell_dt1<DUAL>(a, o, a.uniform ? a.uc.dx : a.coef[c].dx, t1, t2, P));
         if (STAGED && PPM_X_STAGE_STORES) {
           double* sp = stage + (c % kStageCells) * kStageLd + (threadIdx.x & 31);
           sp[0] = o.d;
@@ -1533,7 +1588,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
           sp[4 * kStageField] = o.w;
           if (DUAL) sp[5 * kStageField] = o.ge;
         } else {
-          const int64_t off = base + (int64_t)c * sa;
+          const int off = base + c * sa;
           a.out_d[off] = o.d;
           a.out_e[off] = o.e;
           if (a.out_u) a.out_u[off] = o.u;
@@ -1543,7 +1598,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
         }
       }
       // warp-wide: the same steps on every lane
-      if (STAGED && PPM_X_STAGE_STORES && (ST || c >= 0) && c % kStageCells == kStageCells - 1)
+      if (STAGED && PPM_X_STAGE_STORES && (ST || c >= c0) && c % kStageCells == kStageCells - 1)
         flush_stage<DUAL>(a, stage, pid0, c - (kStageCells - 1), kStageCells);
     }
     Fm = F0;
@@ -1558,9 +1613,11 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
   using Steady = std::integral_constant<bool, true>;
   // the x sweep's update (TMA tiles) gains from the steady block; the y/z update, with
   // its cp.async ring, measured slower with it (more registers than its 128)
-  const int t_steady0 = XT ? is + 2 : n + 1, t_steady1 = XT ? ie - 1 : n;
+  const int tlast = c1 + 2 < n ? c1 + 2 : n;
+  const int t_steady0 = XT ? (c0 > is ? c0 : is) + 2 : tlast + 1;
+  const int t_steady1 = XT ? (c1 < ie - 1 ? c1 : ie - 1) : tlast;
 #pragma unroll 1
-  for (int t = 0; t < t_steady0 && t <= n; ++t) {
+  for (int t = cb; t < t_steady0 && t <= tlast; ++t) {
     step(t, Ramp{});
     if (handed) return true;
   }
@@ -1568,12 +1625,12 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
 #pragma unroll 1
     for (int t = t_steady0; t <= t_steady1; ++t) step(t, Steady{});
 #pragma unroll 1
-    for (int t = t_steady1 + 1 > t_steady0 ? t_steady1 + 1 : t_steady0; t <= n; ++t)
+    for (int t = t_steady1 + 1 > t_steady0 ? t_steady1 + 1 : t_steady0; t <= tlast; ++t)
       step(t, Ramp{});
   }
   // the last step (t = n) leaves cell n-1 unstored; it is a ghost cell, whose
   // post-euler state is its input, selected against itself and its left neighbour
-  {
+  if (c1 == n - 1) {
     const int c = n - 1;
     if (live) {
       Cell o = PEm;
@@ -1591,7 +1648,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int64_t pid, c
         sp[4 * kStageField] = o.w;
         if (DUAL) sp[5 * kStageField] = o.ge;
       } else {
-        const int64_t off = base + (int64_t)c * sa;
+        const int off = base + c * sa;
         a.out_d[off] = o.d;
         a.out_e[off] = o.e;
         if (a.out_u) a.out_u[off] = o.u;
@@ -1655,17 +1712,24 @@ __global__ void __launch_bounds__(kMarchThreads,
     update_kernel(const __grid_constant__ BatchArgs B) {
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
   __shared__ unsigned long long s_cnt[2];
+  __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
   __shared__ uint64_t s_xbar[XT ? (kMarchThreads / 32) * kXBuffers : 1];
   extern __shared__ __align__(128) double s_dyn[];
   double* const s_xtile = s_dyn;                                // XT: kXWarp per warp
   double* const s_stage = s_dyn + (XT ? kXBlock : 0);           // STAGED: kStageWarp per warp
   double* const s_ring = s_dyn;                                 // y, z: the input ring
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
+  s_flag[threadIdx.x] = 0;
   int64_t lb;
-  const int g = locate<ONE>(B.march_prefix, B.ngrids, lb);
+  const int g = locate<ONE>(B.seg_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
-  const int64_t pid = lb * kMarchThreads + threadIdx.x;
-  const int64_t wpid0 = pid - (threadIdx.x & 31);  // first pencil of this warp
+  // a block holds every segment of its pencils, so what one segment finds (a cell for the
+  // fallback pass) reaches the pencil's other segments through shared memory
+  const int pl = threadIdx.x & ((1 << a.pw_log2) - 1);
+  const int pid = (int)(lb << a.pw_log2) + pl;
+  const int wpid0 = pid - (threadIdx.x & 31);  // first pencil of this warp (STAGED)
+  const int c0 = (int)(threadIdx.x >> a.pw_log2) * a.seg_cells;
+  const int c1 = c0 + a.seg_cells - 1 < a.n - 1 ? c0 + a.seg_cells - 1 : a.n - 1;
   const int warp = threadIdx.x >> 5;
   XTiles xt;
   if (XT) {
@@ -1678,6 +1742,7 @@ __global__ void __launch_bounds__(kMarchThreads,
     xt.bytes = (unsigned)__popc(xt.fields) * kXTile * (unsigned)sizeof(double) +
                B.x_tma_extra_tx;
     xt.row0 = (int)wpid0;
+    xt.q0 = 0;
     xt.last = -1;
     xt.broken = false;
     if ((threadIdx.x & 31) == 0) {
@@ -1690,19 +1755,24 @@ __global__ void __launch_bounds__(kMarchThreads,
   if (ONE) __syncthreads();
   double my_dt = 1.0e20;
   const bool valid = pid < a.npencils;
-  if (STAGED || valid) {
+  UpdateCounts cnt = {0, 0, 0, 1.0e20};
+  if ((STAGED || valid) && c0 < a.n) {
     const Phys P = make_phys(a);
-    UpdateCounts cnt = {0, 0, 0, 1.0e20};
     if (update_pencil<DUAL, GRAV, false, STAGED, update_pipe<ONE, STAGED>(), XT, RS>(
-            a, pid, P, cnt, valid, s_stage + warp * kStageWarp, wpid0, s_ring + threadIdx.x,
-            &xt)) {
+            a, pid, P, cnt, c0, c1, valid, s_stage + warp * kStageWarp, wpid0,
+            s_ring + threadIdx.x, &xt))
+      s_flag[pl] = 1;
+  }
+  __syncthreads();
+  if (s_flag[pl]) {  // a flagged pencil's counts and time step come from the fallback pass
+    if (valid && c0 == 0) {
       const unsigned long long slot = atomicAdd(&B.counters[kCntFlagged], 1ull);
       B.flagged[slot] = ((int64_t)g << 40) | pid;
-    } else {
-      if (cnt.fatal) atomicAdd(&s_cnt[0], (unsigned long long)cnt.fatal);
-      if (cnt.nonfinite) atomicAdd(&s_cnt[1], (unsigned long long)cnt.nonfinite);
-      my_dt = cnt.dtmin;  // a flagged pencil's time step comes from the fallback pass
     }
+  } else {
+    if (cnt.fatal) atomicAdd(&s_cnt[0], (unsigned long long)cnt.fatal);
+    if (cnt.nonfinite) atomicAdd(&s_cnt[1], (unsigned long long)cnt.nonfinite);
+    my_dt = cnt.dtmin;
   }
   if (a.cfl_min_bits) {  // warp minimum, one atomic per warp (every lane reaches this)
 #pragma unroll
@@ -1727,8 +1797,8 @@ __global__ void __launch_bounds__(128) fallback_kernel(const __grid_constant__ B
     const SweepArgs& a = ONE ? B.one : B.grids[(int)(code >> 40)];
     const Phys P = make_phys(a);
     UpdateCounts cnt = {0, 0, 0, 1.0e20};
-    update_pencil<DUAL, GRAV, true, false, 0, false, RS>(a, code & ((int64_t(1) << 40) - 1), P,
-                                                        cnt);
+    update_pencil<DUAL, GRAV, true, false, 0, false, RS>(
+        a, (int)(code & ((int64_t(1) << 40) - 1)), P, cnt, 0, a.n - 1);
     if (a.cfl_min_bits && cnt.dtmin < 1.0e20)
       atomicMin(a.cfl_min_bits, (unsigned long long)__double_as_longlong(cnt.dtmin));
     if (cnt.fallbacks) atomicAdd(&B.counters[kCntFallbacks], (unsigned long long)cnt.fallbacks);
@@ -1934,7 +2004,7 @@ __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
 // per device (a function attribute is not a stream operation, so this is also legal
 // while a stream is being captured).
 template <bool DUAL, bool GRAV, bool ONE, bool STAGED, bool XT, bool RS = false>
-void launch_update(const BatchArgs& B, int64_t march_blocks, cudaStream_t st) {
+void launch_update(const BatchArgs& B, cudaStream_t st) {
   constexpr size_t bytes = update_smem_bytes<ONE, STAGED, XT>();
   if (bytes > 48 * 1024) {
     static std::atomic<unsigned long long> done{0};
@@ -1948,7 +2018,7 @@ void launch_update(const BatchArgs& B, int64_t march_blocks, cudaStream_t st) {
     }
   }
   update_kernel<DUAL, GRAV, ONE, STAGED, XT, RS>
-      <<<(unsigned)march_blocks, kMarchThreads, bytes, st>>>(B);
+      <<<(unsigned)B.seg_blocks, kMarchThreads, bytes, st>>>(B);
 }
 
 // The two-shock stage with the plain start: the block size and persistence the batch
@@ -1977,6 +2047,7 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
   auto mark = [&](int k) {
     if (ev) cudaEventRecord(ev[k], st);
   };
+  const unsigned sb = (unsigned)B.seg_blocks;
   mark(0);
   cudaMemsetAsync(B.counters + kCntFlagged, 0, sizeof(unsigned long long), st);
   if (B.fused) {  // the plain path with the fused face kernel
@@ -1985,11 +2056,11 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     mark(2);
     mark(3);
     if (PPM_X_TMA && staged && ONE && B.x_tma)
-      launch_update<DUAL, GRAV, ONE, true, ONE>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, true, ONE>(B, st);
     else if (staged)
-      launch_update<DUAL, GRAV, ONE, true, false>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, true, false>(B, st);
     else
-      launch_update<DUAL, GRAV, ONE, false, false>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, false, false>(B, st);
     mark(4);
     // the flagged pencils' interface states, then their per-cell HLL fallback
     reconstruct_kernel<DUAL, GRAV, 0, ONE, false, true><<<64, kMarchThreads, 0, st>>>(B);
@@ -1999,16 +2070,16 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     return;
   }
   if (B.ncolour > 0) cudaMemsetAsync(B.hll_flags, 0, (size_t)B.hll_bytes, st);
-  if (B.corrections || B.ncolour > 0 || B.presfree) {  // colours, PressureFree: COR too
+  if (B.corrections || B.ncolour > 0 || B.presfree || B.uneven) {  // not the plain path: COR
     if (B.corrections)
       corrections_kernel<ONE><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
-    reconstruct_kernel<DUAL, GRAV, 0, ONE, true><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
+    reconstruct_kernel<DUAL, GRAV, 0, ONE, true><<<sb, kMarchThreads, 0, st>>>(B);
     mark(1);
-    reconstruct_kernel<DUAL, GRAV, 1, ONE, true><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
+    reconstruct_kernel<DUAL, GRAV, 1, ONE, true><<<sb, kMarchThreads, 0, st>>>(B);
   } else {
-    reconstruct_kernel<DUAL, GRAV, 0, ONE><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
+    reconstruct_kernel<DUAL, GRAV, 0, ONE><<<sb, kMarchThreads, 0, st>>>(B);
     mark(1);
-    reconstruct_kernel<DUAL, GRAV, 1, ONE><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
+    reconstruct_kernel<DUAL, GRAV, 1, ONE><<<sb, kMarchThreads, 0, st>>>(B);
   }
   mark(2);
   const unsigned rb = (unsigned)riemann_blocks;
@@ -2040,20 +2111,20 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
   mark(3);
   if (B.solver != 0) {  // HLL / HLLC
     if (PPM_X_TMA && staged && ONE && B.x_tma)
-      launch_update<DUAL, GRAV, ONE, true, ONE, true>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, true, ONE, true>(B, st);
     else if (staged)
-      launch_update<DUAL, GRAV, ONE, true, false, true>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, true, false, true>(B, st);
     else
-      launch_update<DUAL, GRAV, ONE, false, false, true>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, false, false, true>(B, st);
     mark(4);
     fallback_kernel<DUAL, GRAV, ONE, true><<<64, 128, 0, st>>>(B);
   } else {
     if (PPM_X_TMA && staged && ONE && B.x_tma)
-      launch_update<DUAL, GRAV, ONE, true, ONE>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, true, ONE>(B, st);
     else if (staged)
-      launch_update<DUAL, GRAV, ONE, true, false>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, true, false>(B, st);
     else
-      launch_update<DUAL, GRAV, ONE, false, false>(B, march_blocks, st);
+      launch_update<DUAL, GRAV, ONE, false, false>(B, st);
     mark(4);
     fallback_kernel<DUAL, GRAV, ONE><<<64, 128, 0, st>>>(B);
   }

@@ -4,6 +4,7 @@
 #include <cuda.h>  // CUtensorMap
 
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 namespace ppm {
@@ -120,6 +121,13 @@ struct SweepArgs {
   // EOSType 3 (isothermal): the folded time step's pressure is rho * eos_cs^2
   int eos_type;
   double eos_cs;
+  // split of the marching stages (set_segments): a block of kMarchThreads threads takes
+  // 2^pw_log2 pencils, each cut into kMarchThreads >> pw_log2 segments of seg_faces faces
+  // (reconstruction) or seg_cells cells (update)
+  int pw_log2, seg_faces, seg_cells;
+  // one cell width along the sweep (uniform): the coefficients every cell shares
+  int uniform;
+  Coef uc;
 };
 
 enum { kFaceVars = 12, kFluxVars = 7 };
@@ -145,7 +153,8 @@ enum { kMarchThreads = PPM_MARCH_THREADS, kRiemannThreads = PPM_RIEMANN_THREADS 
 // One launch over a batch of grids (an AMR level, or a single grid).  Every block
 // belongs to one grid: grid g owns blocks [prefix[g], prefix[g+1]) of a stage; a
 // block finds its grid by binary search over the prefix table.
-//   marching stages: ceil(npencils / kMarchThreads) blocks per grid
+//   reconstruction, update: ceil(npencils / 2^pw_log2) blocks per grid
+//   corrections, colours: ceil(npencils / kMarchThreads) blocks per grid
 //   Riemann stage:   (ie - is + 2) * ceil(npencils / kRiemannThreads) blocks per grid
 struct BatchArgs {
   SweepArgs one;                     // the record itself when ngrids == 1 (read from the
@@ -153,10 +162,13 @@ struct BatchArgs {
   const SweepArgs* grids;            // device array, ngrids records
   int ngrids;
   const int64_t* march_prefix;       // ngrids + 1
+  const int64_t* seg_prefix;         // ngrids + 1
+  int64_t seg_blocks = 0;
   const int64_t* riemann_prefix;     // ngrids + 1
   unsigned long long* counters;      // kMaxCounters, shared by the batch
   int64_t* flagged;                  // pencils needing the fallback pass: (grid << 40) | pencil
   int corrections = 0;               // the batch's grids carry flattening / steepening
+  int uneven = 0;                    // a grid's cell widths differ along the sweep
   // x sweep of a single grid: the update kernel reads its input cells as TMA tiles of
   // kXTileRows pencils x kXTileCells cells, through 2-D tensor maps (cells x pencils) of
   // d, e, u, v, w, ge (absent fields: unused).  x_tma = 0: plain loads.
@@ -240,6 +252,56 @@ inline void build_coef(const double* dxi_in, int n, int is0, int ie0, std::vecto
     out[i - 1].c6 = -(dxi(i - 1) / qa * qc);
     out[i - 1].dx2i = 0.5 / dxi(i);
   }
+}
+
+// Segments of the marching stages.  A march along a whole pencil is a serial chain of n
+// steps, so a batch with few pencils leaves the chip idle and waits for the chain: the
+// pencils are cut (powers of two) until the batch has PPM_MARCH_FILL threads or a segment is
+// down to kSegMin faces, each segment repeating the few cells of its neighbours that its
+// first face and its first and last cells depend on.  Whole step, whole pencils -> cut
+// (exact build unless stated): 100 cells in one dimension 501 -> 101 us, 256x192 1608 ->
+// 161, 37x24x53 with HLLC 692 -> 240, 128^3 2703 -> 1879, 189x131x157 (tolerance) 3101 ->
+// 2404.  PPM_MARCH_FILL is the chip's resident march threads (148 SMs, 4 blocks of 128): with
+// 2, 4 and 8 times that 128^3 measured 1865, 2168 and 2170 us in its sweeps against 1835,
+// and 189x131x157 2711, 2525 and 2980 against 2339 (below 32 pencils a block the x sweep
+// loses its staged stores); batches with more pencils than that (256^3 nearly, 512^3,
+// levels) gain nothing from more threads and pay the repeated cells.
+#ifndef PPM_MARCH_FILL
+#define PPM_MARCH_FILL (148 * 4 * 128)
+#endif
+#ifndef PPM_SEG_MIN
+#define PPM_SEG_MIN 4
+#endif
+inline int64_t march_segment_blocks(const SweepArgs& a) {
+  return (a.npencils + (int64_t(1) << a.pw_log2) - 1) >> a.pw_log2;
+}
+// a: a record with its geometry; batch_pencils: pencils of all grids of the launch.
+// local_select: pgas2d_dual's energy of a cell may be formed without its left neighbour
+// (see update_pencil); without it the update needs whole pencils.
+inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select) {
+  int log_w = 0;
+  while ((1 << log_w) < kMarchThreads) ++log_w;
+  const int faces = a.ie - a.is + 2;
+  int segs = 1;
+  if (local_select)
+    while (segs < kMarchThreads && batch_pencils * segs < PPM_MARCH_FILL &&
+           faces / (2 * segs) >= PPM_SEG_MIN) {
+      segs *= 2;
+      --log_w;
+    }
+  a.pw_log2 = log_w;
+  a.seg_faces = (faces + segs - 1) / segs;
+  // whole output chunks of the x sweep's staged stores
+  const int cells = (a.n + segs - 1) / segs;
+  a.seg_cells = (cells + 3) / 4 * 4;
+}
+
+// The record's shared coefficients, from its coefficient table on the host.
+inline void set_uniform(SweepArgs& a, const double* width, const Coef* table) {
+  a.uniform = 1;
+  for (int i = 1; i < a.n; ++i)
+    if (std::memcmp(&width[i], &width[0], sizeof(double)) != 0) a.uniform = 0;
+  a.uc = table[a.is];
 }
 
 // Grid that owns block b of a stage, and the block's index inside that grid.
