@@ -1005,10 +1005,14 @@ int scatter_captures(ppm_b200_context* ctx, int dim, const ppm_b200_params* p,
 }
 
 int read_counters(ppm_b200_context* ctx, ppm_b200_stats* st, int* status) {
-  unsigned long long c[ppm::kMaxCounters];
-  CK(cudaMemcpyAsync(c, ctx->counters.p, sizeof(c), cudaMemcpyDeviceToHost, ctx->stream));
+  static_assert(sizeof(unsigned long long) * ppm::kMaxCounters * ppm::kCounterCopies ==
+                ppm::kCounterBytes, "counter copies");
+  unsigned long long copies[ppm::kCounterCopies * ppm::kMaxCounters], c[ppm::kMaxCounters];
+  CK(cudaMemcpyAsync(copies, ctx->counters.p, sizeof(copies), cudaMemcpyDeviceToHost,
+                     ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  CK(cudaMemsetAsync(ctx->counters.p, 0, sizeof(c), ctx->stream));
+  CK(cudaMemsetAsync(ctx->counters.p, 0, sizeof(copies), ctx->stream));
+  ppm::sum_counters(copies, c);
   if (st) {
     st->interfaces += (long long)c[ppm::kCntInterfaces];
     st->newton_iters += (long long)c[ppm::kCntNewton];
@@ -1582,7 +1586,7 @@ int ppm_b200_create(int device, void* cuda_stream, ppm_b200_context** out) {
     }
     ctx->own_stream = true;
   }
-  int rc = ensure(ctx, ctx->counters, ppm::kMaxCounters * sizeof(unsigned long long));
+  int rc = ensure(ctx, ctx->counters, ppm::kCounterBytes);
   if (!rc) rc = ensure(ctx, ctx->misc, 4 * sizeof(double));
   if (!rc) rc = cuda_fail(ctx, cudaMemset(ctx->counters.p, 0, ctx->counters.bytes), "cudaMemset");
   if (rc) {

@@ -51,7 +51,7 @@ void launch_sweep_batch(const BatchArgs& B, int64_t march_blocks, int64_t rieman
 
 namespace {
 
-constexpr size_t kStaticCounterBytes = 256;                       // kMaxCounters counters
+constexpr size_t kStaticCounterBytes = ppm::kCounterBytes;        // counters, in copies
 constexpr int kStaticCoefEntries = 1031;                          // longest pencil (fortran.def:1)
 constexpr size_t kStaticCoefBytes = 66560;                        // >= 1031 * sizeof(Coef), 256-aligned
 constexpr size_t kStaticDescBytes = 1024;                         // grid record + block prefixes
@@ -60,7 +60,7 @@ constexpr size_t kStaticBytes =
     kStaticCounterBytes + kStaticCoefBytes + kStaticDescBytes + kStaticPlaneBytes;
 static_assert(kStaticCoefEntries * sizeof(ppm::Coef) <= kStaticCoefBytes, "coef area");
 static_assert(sizeof(ppm::SweepArgs) <= 768, "the record's place in the descriptor area");
-static_assert(ppm::kMaxCounters * sizeof(unsigned long long) <= kStaticCounterBytes, "counters");
+static_assert(kStaticCounterBytes % 256 == 0, "alignment of the coefficient table");
 
 constexpr int kMaxDevices = 64;
 
@@ -283,11 +283,12 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   if (e != cudaSuccess) return fail_cuda(e, "sweep launch");
 
   // ---- status
-  unsigned long long c[ppm::kMaxCounters];
-  e = cudaMemcpyAsync(c, counters, sizeof(c), cudaMemcpyDeviceToHost, st);
+  unsigned long long copies[ppm::kCounterCopies * ppm::kMaxCounters], c[ppm::kMaxCounters];
+  e = cudaMemcpyAsync(copies, counters, sizeof(copies), cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpyAsync");
   e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail_cuda(e, "cudaStreamSynchronize");
+  ppm::sum_counters(copies, c);
   if (stats) {
     stats->interfaces += (long long)c[ppm::kCntInterfaces];
     stats->newton_iters += (long long)c[ppm::kCntNewton];

@@ -621,19 +621,20 @@ __global__ void __launch_bounds__(RT, (LEARNED ? PPM_RIEMANN_LEARNED_MINBLOCKS
   if (!PERSIST) break;
   }
   __syncthreads();
+  unsigned long long* const cnt = B.counters + (blockIdx.x % kCounterCopies) * kMaxCounters;
   if (threadIdx.x < 8 && s_hist[threadIdx.x])
-    atomicAdd(&B.counters[kCntHist0 + threadIdx.x], (unsigned long long)s_hist[threadIdx.x]);
+    atomicAdd(&cnt[kCntHist0 + threadIdx.x], (unsigned long long)s_hist[threadIdx.x]);
   if (threadIdx.x == 8 && s_newton) {
     unsigned long long nif = 0;
     for (int h = 0; h < 8; ++h) nif += s_hist[h];
-    atomicAdd(&B.counters[kCntInterfaces], nif);
-    atomicAdd(&B.counters[kCntNewton], (unsigned long long)s_newton);
+    atomicAdd(&cnt[kCntInterfaces], nif);
+    atomicAdd(&cnt[kCntNewton], (unsigned long long)s_newton);
   }
   if (LEARNED && threadIdx.x == 9 && s_rejected)
-    atomicAdd(&B.counters[kCntGuessRejected], (unsigned long long)s_rejected);
+    atomicAdd(&cnt[kCntGuessRejected], (unsigned long long)s_rejected);
   if (threadIdx.x == 10 && s_warps) {
-    atomicAdd(&B.counters[kCntWarpNewton], (unsigned long long)s_wtrips);
-    atomicAdd(&B.counters[kCntWarps], (unsigned long long)s_warps);
+    atomicAdd(&cnt[kCntWarpNewton], (unsigned long long)s_wtrips);
+    atomicAdd(&cnt[kCntWarps], (unsigned long long)s_warps);
   }
 }
 
@@ -867,17 +868,18 @@ __global__ void __launch_bounds__(kFaceThreads, PPM_FACE_MINBLOCKS)
     o[XUB * plane] = F.ub;
   }
   __syncthreads();
+  unsigned long long* const cnt = B.counters + (blockIdx.x % kCounterCopies) * kMaxCounters;
   if (threadIdx.x < 8 && s_hist[threadIdx.x])
-    atomicAdd(&B.counters[kCntHist0 + threadIdx.x], (unsigned long long)s_hist[threadIdx.x]);
+    atomicAdd(&cnt[kCntHist0 + threadIdx.x], (unsigned long long)s_hist[threadIdx.x]);
   if (threadIdx.x == 8 && s_newton) {
     unsigned long long nif = 0;
     for (int h = 0; h < 8; ++h) nif += s_hist[h];
-    atomicAdd(&B.counters[kCntInterfaces], nif);
-    atomicAdd(&B.counters[kCntNewton], (unsigned long long)s_newton);
+    atomicAdd(&cnt[kCntInterfaces], nif);
+    atomicAdd(&cnt[kCntNewton], (unsigned long long)s_newton);
   }
   if (threadIdx.x == 10 && s_warps) {
-    atomicAdd(&B.counters[kCntWarpNewton], (unsigned long long)s_wtrips);
-    atomicAdd(&B.counters[kCntWarps], (unsigned long long)s_warps);
+    atomicAdd(&cnt[kCntWarpNewton], (unsigned long long)s_wtrips);
+    atomicAdd(&cnt[kCntWarps], (unsigned long long)s_warps);
   }
 }
 
