@@ -712,7 +712,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   std::vector<SweepArgs> rec(ng);
   std::vector<int64_t> mpre(ng + 1, 0), rpre(ng + 1, 0), fpre(ng + 1, 0), gpre(ng + 1, 0);
   // the fused face kernel serves the same plain two-shock path, without slope corrections
-  const bool fused = plain_riemann && ctx->sweep_mode == PPM_B200_SWEEP_FUSED &&
+  bool fused = plain_riemann && ctx->sweep_mode == PPM_B200_SWEEP_FUSED &&
                      correction_planes(p) == 0;
   size_t scratch_doubles = 0, flag_bytes = 0;
   int64_t total_pencils = 0;

@@ -15,13 +15,6 @@
 
 #include "ppm_fastmath.cuh"
 
-// PPM_NEWTON_RSQRT: the tolerance build's Newton update from 1/sqrt of the shock factors
-// (one reciprocal square root each instead of a square root plus a shared reciprocal;
-// Riemann stage 0.77 -> 0.74 ms per 256^3 sweep)
-#ifndef PPM_NEWTON_RSQRT
-#define PPM_NEWTON_RSQRT 1
-#endif
-
 // PPM_FAST_ALGEBRA (the tolerance-mode build): a few quotients with a shared divisor
 // are formed from one reciprocal, and the divisions and square roots of the
 // reconstruction, the Riemann solvers and the update (not calc_dt's) go through qrcp /
@@ -61,7 +54,14 @@ template <bool PF = false>
 __device__ __forceinline__ Prep cell_prep(double d, double p, double u, double dx2i,
                                           const Phys& P) {
   Prep r;
-  double cs = qsqrt(qdiv(P.gamma * p, d));
+#if PPM_FAST_ALGEBRA
+  // sqrt(gamma p/d) = gamma p / sqrt(gamma p d): no division (0 where the product is 0)
+  const double gp = P.gamma * p, x = gp * d;
+  const double y = gp * qrsqrt_n(x);
+  double cs = fm_exponent(x) == 0u ? 0.0 : y;
+#else
+  double cs = sqrt(P.gamma * p / d);
+#endif
   if (PF) cs = kTiny;
   r.char1 = dmax(0.0, P.dt * (u + cs)) * dx2i;
   r.char2 = dmax(0.0, -(P.dt * (u - cs))) * dx2i;
@@ -72,9 +72,21 @@ __device__ __forceinline__ Prep cell_prep(double d, double p, double u, double d
 }
 
 // ---------------------------------------------------------------- intvar.F:82-94
+// UNI: one cell width along the sweep.  Then qcent is the mean of the two differences, and
+// of two numbers of one sign the harmonic mean qvanl is the smallest of the four candidates
+// (2ab/(a+b) <= 2 min(a,b) and <= (a+b)/2), so the tolerance build takes it without the
+// three minima.
+template <bool UNI = false>
 __device__ __forceinline__ double pm_slope(double qm, double q0, double qp, double c1, double c2) {
   double qplus = qp - q0;
   double qmnus = q0 - qm;
+#if PPM_FAST_ALGEBRA
+  if (UNI) {
+    const double prod = qplus * qmnus;
+    const double r = 2.0 * prod * qrcp_n(qmnus + qplus);  // NaN for a zero sum: not taken
+    return prod > 0.0 ? r : 0.0;
+  }
+#endif
   double qcent = c1 * qplus + c2 * qmnus;
   double qvanl = qdiv(2.0 * qplus * qmnus, qmnus + qplus);
   double temp1 = dmin(dmin(dmin(fabs(qcent), fabs(qvanl)), 2.0 * fabs(qmnus)), 2.0 * fabs(qplus));
@@ -192,7 +204,13 @@ struct Para {
   double ql, qr, q6, dq;
 };
 
-template <bool STEEP = false, bool FLAT = false>
+// UNI (with neither): one cell width along the sweep, where CHECK_LR has nothing to do but
+// round-off.  An edge of two neighbours a, b = a + h lies in [a + h/6, b - h/6], as the
+// limited slopes differ by at most 2h; where a != b in double precision both bounds are
+// inside, and where a == b both slopes are zero and the edge is a.  The monotonicity step
+// moves an edge only toward the cell's value.  The tolerance build leaves the eight
+// comparisons out.
+template <bool STEEP = false, bool FLAT = false, bool UNI = false>
 __device__ __forceinline__ Para pm_parabola(double qm, double q0, double qp, double ql, double qr,
                                             double st = 0.0, double dqm = 0.0,
                                             double dqp = 0.0, double fl = 0.0) {
@@ -215,11 +233,12 @@ __device__ __forceinline__ Para pm_parabola(double qm, double q0, double qp, dou
     ql = q0 * fl + ql * (1.0 - fl);
     qr = q0 * fl + qr * (1.0 - fl);
   }
-  // CHECK_LR, intvar.F:145-153
-  ql = dmax(dmin(q0, qm), ql);
-  ql = dmin(dmax(q0, qm), ql);
-  qr = dmax(dmin(q0, qp), qr);
-  qr = dmin(dmax(q0, qp), qr);
+  if (!(PPM_FAST_ALGEBRA && UNI && !STEEP && !FLAT)) {  // CHECK_LR, intvar.F:145-153
+    ql = dmax(dmin(q0, qm), ql);
+    ql = dmin(dmax(q0, qm), ql);
+    qr = dmax(dmin(q0, qp), qr);
+    qr = dmin(dmax(q0, qp), qr);
+  }
   Para r;
   r.q6 = 6.0 * (q0 - 0.5 * (ql + qr));
   r.dq = qr - ql;
@@ -295,15 +314,30 @@ struct SideOut {
 template <bool DUAL, bool GRAV, bool LEFT>
 __device__ __forceinline__ SideOut face_side(const SideIn& S, double gsum, const Phys& P) {
   SideOut o;
-  const double c = qsqrt(dmax(P.gamma * S.pa * S.da, 0.0));
-  // 0.5/c is computed as 0.5*(1/c): equal, since c is 0, inf, NaN or a square root of
-  // a double (|c| <= 2^512), so 1/c never reaches the subnormal range
-  double f1 = qrcp(c);
+#if PPM_FAST_ALGEBRA
+  // tolerance mode: 1/c from the reciprocal square root and c = c^2/c, 1/da and
+  // 1/da - 1/d0 from one reciprocal of da*d0: two reciprocals and a root less per side
+  // (d/p/u march of a 256^3 sweep, with the slopes and parabolas: 0.60 -> 0.46 ms)
+  const double c2 = dmax(P.gamma * S.pa * S.da, 0.0);
+  double f1 = qrsqrt(c2);  // inf where c2 is 0
+  const double c = fm_exponent(c2) == 0u ? 0.0 : c2 * f1;
   const double hc = 0.5 * f1;
-  const double yd = qrcp(S.da);
+  const double qd = qrcp_n(S.da * S.d0);
+  const double yd = S.d0 * qd;
   double bp = (S.ua - S.up) + (S.pa - S.pp) * f1;
   double bm = (S.ua - S.um) - (S.pa - S.pm) * f1;
-  double b0 = (S.pa - S.p0) * (f1 * f1) + yd - qrcp(S.d0);
+  double b0 = (S.pa - S.p0) * (f1 * f1) + (S.d0 - S.da) * qd;
+#else
+  const double c = sqrt(dmax(P.gamma * S.pa * S.da, 0.0)), c2 = c * c;
+  // 0.5/c is computed as 0.5*(1/c): equal, since c is 0, inf, NaN or a square root of
+  // a double (|c| <= 2^512), so 1/c never reaches the subnormal range
+  double f1 = 1.0 / c;
+  const double hc = 0.5 * f1;
+  const double yd = 1.0 / S.da;
+  double bp = (S.ua - S.up) + (S.pa - S.pp) * f1;
+  double bm = (S.ua - S.um) - (S.pa - S.pm) * f1;
+  double b0 = (S.pa - S.p0) * (f1 * f1) + yd - 1.0 / S.d0;
+#endif
   if (GRAV) {
     const double gterm = 0.25 * P.dt * gsum;
     bp = bp - gterm;
@@ -315,7 +349,7 @@ __device__ __forceinline__ SideOut face_side(const SideIn& S, double gsum, const
   if (LEFT ? S.cp <= 0.0 : S.cp >= 0.0) bp = 0.0;
   if (LEFT ? S.cm <= 0.0 : S.cm >= 0.0) bm = 0.0;
   if (LEFT ? S.c0 <= 0.0 : S.c0 >= 0.0) b0 = 0.0;
-  o.p = S.pa + (bp + bm) * (c * c);
+  o.p = S.pa + (bp + bm) * c2;
   o.u = S.ua + (bp - bm) * c;
   o.d = qrcp(yd - (b0 + bp + bm));
   o.dc = o.d;
@@ -407,32 +441,33 @@ __device__ __forceinline__ double acoustic_guess(const FaceState& s, double cl, 
 
 __device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, double cl, double cr,
                                                    double ps, const Phys& P) {
-  double old_ps = ps, ubl = 0.0, ubr = 0.0, dpdul = 0.0, dpdur = 0.0;
+  double old_ps = ps, ubl = 0.0, ubr = 0.0;
   int it = 0;
   bool active = true;
 #if PPM_FAST_ALGEBRA
-  // Tolerance-mode build: the same Newton update with the face's reciprocals 1/pl, 1/pr,
-  // 1/dl, 1/dr formed once, each pair of quotients with different divisors sharing one
-  // division (a/x, b/y = a*y*q, b*x*q with q = 1/(x*y)), and the convergence test as
-  // |dp| < tolerance * ps: three divisions per update instead of twelve.
-  const double ipl = qrcp(s.pl), ipr = qrcp(s.pr), idl = qrcp(s.dl), idr = qrcp(s.dr);
-#if PPM_NEWTON_RSQRT
-  // zl = cl sqrt(Xl) from yl = 1/sqrt(Xl): zl = cl Xl yl, 1/zl = yl / cl, zl^2 = cl^2 Xl
-  const double icl = qrcp(cl), icr = qrcp(cr), cl2 = cl * cl, cr2 = cr * cr;
+  // Tolerance-mode build: the same Newton update from X = 1 + qa (p/p_s - 1) alone, where
+  // z^2 = c^2 X.  4 z^2/d is 4 gamma p_s X, and 4 z^2/d - (gamma+1)(p - p_s) is
+  // 2 gamma p_s (1 + X), so the slope of a side is dp/du = 2 z X/(1 + X), and the update
+  // (ur - ul) R L/(R - L) with L = -dp/du of the left side is (ul - ur)/(1/dpl + 1/dpr):
+  // with y = 1/sqrt(X) and 1/z = y/c an update takes two reciprocal square roots and one
+  // reciprocal (the reference's form: two roots and eight divisions).  256^3 sweep: 1138 k
+  // issue cycles -> 828 k, 0.73 -> 0.58 ms (with the flux's shared reciprocals below).
+  const double icl = qrcp_n(cl), icr = qrcp_n(cr);
+  const double qp = P.qa * qrcp_n(s.pl * s.pr), gl = s.pr * qp, gr = s.pl * qp;
+  const double omq = 1.0 - P.qa;
+  double il = 0.0, ir = 0.0, qs = 0.0;  // 1/dpl, 1/dpr, 1/(1/dpl + 1/dpr)
 #pragma unroll 1
   for (int n = 2; n <= kNumIter; n++) {
     if (active) {
-      const double Xl = 1.0 + P.qa * (ps * ipl - 1.0), Xr = 1.0 + P.qa * (ps * ipr - 1.0);
-      const double yl = qrsqrt(Xl), yr = qrsqrt(Xr);
-      const double zl = cl * (Xl * yl), zr = cr * (Xr * yr);
-      ubl = s.ul - (ps - s.pl) * (yl * icl);
-      ubr = s.ur + (ps - s.pr) * (yr * icr);
-      const double al = 4.0 * (cl2 * Xl) * idl, ar = 4.0 * (cr2 * Xr) * idr;
-      const double dl = al - P.gp1 * (ps - s.pl), dr = ar - P.gp1 * (ps - s.pr);
-      const double qd = qrcp(dl * dr);
-      dpdul = -(zl * al * (dr * qd));
-      dpdur = zr * ar * (dl * qd);
-      ps = ps + qdiv((ubr - ubl) * dpdur * dpdul, dpdur - dpdul);
+      const double Xl = ps * gl + omq, Xr = ps * gr + omq;
+      const double yl = qrsqrt_n(Xl), yr = qrsqrt_n(Xr);
+      const double wl = yl * icl, wr = yr * icr;
+      ubl = s.ul - (ps - s.pl) * wl;
+      ubr = s.ur + (ps - s.pr) * wr;
+      il = wl * (0.5 * Xl + 0.5) * (yl * yl);
+      ir = wr * (0.5 * Xr + 0.5) * (yr * yr);
+      qs = qrcp_n(il + ir);
+      ps = ps + (ubl - ubr) * qs;
       if (ps < P.pmin) ps = P.pmin;
       const double delta_ps = ps - old_ps;
       old_ps = ps;
@@ -441,29 +476,7 @@ __device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, double cl
     }
   }
 #else
-#pragma unroll 1
-  for (int n = 2; n <= kNumIter; n++) {
-    if (active) {
-      const double zl = cl * qsqrt((1.0 + P.qa * (ps * ipl - 1.0)));
-      const double zr = cr * qsqrt((1.0 + P.qa * (ps * ipr - 1.0)));
-      const double qz = qrcp(zl * zr);
-      ubl = s.ul - (ps - s.pl) * (zr * qz);
-      ubr = s.ur + (ps - s.pr) * (zl * qz);
-      const double al = 4.0 * (zl * zl) * idl, ar = 4.0 * (zr * zr) * idr;
-      const double dl = al - P.gp1 * (ps - s.pl), dr = ar - P.gp1 * (ps - s.pr);
-      const double qd = qrcp(dl * dr);
-      dpdul = -(zl * al * (dr * qd));
-      dpdur = zr * ar * (dl * qd);
-      ps = ps + qdiv((ubr - ubl) * dpdur * dpdul, dpdur - dpdul);
-      if (ps < P.pmin) ps = P.pmin;
-      const double delta_ps = ps - old_ps;
-      old_ps = ps;
-      it++;
-      if (fabs(delta_ps) < kTolerance * ps) active = false;
-    }
-  }
-#endif
-#else
+  double dpdul = 0.0, dpdur = 0.0;
 #pragma unroll 1
   for (int n = 2; n <= kNumIter; n++) {
     if (active) {
@@ -485,7 +498,11 @@ __device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, double cl
   Riemann r;
   if (ps < P.pmin) ps = dmin(s.pl, s.pr);
   r.pbar = ps;
-  r.ubar = ubl + qdiv((ubr - ubl) * dpdur, dpdur - dpdul);
+#if PPM_FAST_ALGEBRA
+  r.ubar = ubl + (ubr - ubl) * (il * qs);
+#else
+  r.ubar = ubl + (ubr - ubl) * dpdur / (dpdur - dpdul);
+#endif
   r.iters = it;
   r.converged = !active;
   return r;
@@ -511,21 +528,21 @@ __device__ __forceinline__ Flux flux_twoshock(const FaceState& s, double pbar, d
     u0 = s.ur; p0 = s.pr; d0 = s.dr;
   }
 #if PPM_FAST_ALGEBRA
-  // tolerance mode: 1/d0 once, and gamma*pbar/dbar as gamma*pbar*(1/dbar)
-  const double id0 = qrcp(d0);
-  double c0 = qsqrt(dmax(gamma * p0 * id0, kTiny));
-  double z0 = c0 * d0 * qsqrt(dmax(1.0 + P.qa * (qdiv(pbar, p0) - 1.0), kTiny));
-  const double idbar = id0 - qdiv(pbar - p0, dmax(z0 * z0, kTiny));
-  double dbar = qrcp(idbar);
-  double cbar = qsqrt(dmax(gamma * pbar * idbar, kTiny));
-  double l0, lbar;
-  if (pbar < p0) {
-    l0 = u0 * sn + c0;
-    lbar = sn * ubar + cbar;
-  } else {
-    l0 = u0 * sn + z0 * id0;
-    lbar = l0;
-  }
+  // tolerance mode: 1/d0 and 1/p0 from one reciprocal; z0^2 = c0^2 d0^2 X without its
+  // root; dbar = d0 z0^2/(z0^2 - (pbar - p0) d0) and its reciprocal from one reciprocal
+  // of the two factors; of c0 and z0/d0 = c0 sqrt(X) only the one that l0 takes
+  const double q0 = qrcp_n(d0 * p0), id0 = p0 * q0;
+  const double c02 = dmax(gamma * p0 * id0, kTiny);
+  const double X = dmax(1.0 + P.qa * (pbar * (d0 * q0) - 1.0), kTiny);
+  const double c02X = c02 * X;
+  const double z02 = dmax(c02X * (d0 * d0), kTiny), zd = z02 - (pbar - p0) * d0;
+  const double qz = qrcp(z02 * zd);
+  const double idbar = id0 * (zd * zd * qz);
+  const double dbar = d0 * (z02 * z02 * qz);
+  const bool rare = pbar < p0;
+  const double l0 = u0 * sn + qsqrt(rare ? c02 : c02X);
+  const double cbar = qsqrt(dmax(gamma * pbar * idbar, kTiny));
+  const double lbar = rare ? sn * ubar + cbar : l0;
 #else
   double c0 = sqrt(dmax(gamma * p0 / d0, kTiny));
   double z0 = c0 * d0 * sqrt(dmax(1.0 + P.qa * (pbar / p0 - 1.0), kTiny));

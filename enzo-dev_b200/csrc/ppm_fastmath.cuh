@@ -70,6 +70,28 @@ __device__ __forceinline__ double qrcp(double x) {
 #endif
 }
 
+// 1/x and 1/sqrt(x) where x is normal and its result too (x from 2^-1022 to below 2^1021;
+// positive for the root): no special arguments to pick out, so the four or five integer
+// operations of that go (zeros and infinities give NaN)
+__device__ __forceinline__ double qrcp_n(double x) {
+#if PPM_FAST_DIVSQRT
+  const double y0 = fm_rcp_approx(x);
+  const double e = fma(-x, y0, 1.0);
+  return fma(y0, fma(e, e, e), y0);
+#else
+  return 1.0 / x;
+#endif
+}
+__device__ __forceinline__ double qrsqrt_n(double x) {
+#if PPM_FAST_DIVSQRT
+  const double y0 = fm_rsqrt_approx(x);
+  const double e = fma(-x * y0, y0, 1.0);
+  return fma(y0, e * fma(0.375, e, 0.5), y0);
+#else
+  return 1.0 / sqrt(x);
+#endif
+}
+
 // a/b
 __device__ __forceinline__ double qdiv(double a, double b) {
 #if PPM_FAST_DIVSQRT

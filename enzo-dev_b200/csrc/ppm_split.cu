@@ -260,7 +260,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int pid, 
       if (ST || (c >= is - 2 && c <= ie + 2)) {
         const Coef& cf = COR ? a.coef[c] : a.uc;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) dqN[v] = pm_slope(wq1[v], wq2[v], nq[v], cf.c1, cf.c2);
+        for (int v = 0; v < NV; ++v) dqN[v] = pm_slope<!COR>(wq1[v], wq2[v], nq[v], cf.c1, cf.c2);
         if (ST || c >= is - 1) {
 #pragma unroll
           for (int v = 0; v < NV; ++v)
@@ -299,7 +299,8 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int pid, 
           }
         } else {
 #pragma unroll
-          for (int v = 0; v < NV; ++v) pa[v] = pm_parabola(wq0[v], wq1[v], wq2[v], qlm1[v], qlN[v]);
+          for (int v = 0; v < NV; ++v)
+            pa[v] = pm_parabola<false, false, true>(wq0[v], wq1[v], wq2[v], qlm1[v], qlN[v]);
         }
         double* o = a.fstate + (c - fs0) * np + pid;
         if (ROLE == 0) {
@@ -670,15 +671,15 @@ __device__ __forceinline__ void face_parabolas(const double q[3], const double q
   for (int v = 0; v < 3; ++v) pa[v] = Para{0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    const double dq = pm_slope(qm[v], q[v], qp[v], cf.c1, cf.c2);
+    const double dq = pm_slope<true>(qm[v], q[v], qp[v], cf.c1, cf.c2);
     double dqm = shfl_up1(dq);
     double dqp = shfl_dn1(dq);
-    if (lane == 0) dqm = pm_slope(qmm[v], qm[v], q[v], cfm.c1, cfm.c2);
-    if (lane == 31) dqp = pm_slope(q[v], qp[v], qpp[v], cfp.c1, cfp.c2);
+    if (lane == 0) dqm = pm_slope<true>(qmm[v], qm[v], q[v], cfm.c1, cfm.c2);
+    if (lane == 31) dqp = pm_slope<true>(q[v], qp[v], qpp[v], cfp.c1, cfp.c2);
     const double ql = pm_edge(qm[v], q[v], dqm, dq, cf.c3, cf.c4, cf.c5, cf.c6);
     double qr = shfl_dn1(ql);
     if (lane == 31) qr = pm_edge(q[v], qp[v], dq, dqp, cfp.c3, cfp.c4, cfp.c5, cfp.c6);
-    pa[v] = pm_parabola(qm[v], q[v], qp[v], ql, qr);
+    pa[v] = pm_parabola<false, false, true>(qm[v], q[v], qp[v], ql, qr);
   }
 }
 
