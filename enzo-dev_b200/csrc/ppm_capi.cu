@@ -528,8 +528,8 @@ void set_x_tiles(BatchArgs& B, const SweepArgs& a) {
     return;
   const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) return;
-  const double* f[6] = {a.in_d, a.in_e, a.in_u, a.in_v, a.in_w, a.in_ge};
-  for (int k = 0; k < 6; ++k) {
+  const double* f[7] = {a.in_d, a.in_e, a.in_u, a.in_v, a.in_w, a.in_ge, a.pres};
+  for (int k = 0; k < 7; ++k) {
     std::memset(&B.xin[k], 0, sizeof(B.xin[k]));
     if (!f[k]) continue;
     if ((uintptr_t)f[k] % 16 != 0) return;
@@ -710,12 +710,13 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   const bool persist = plain_riemann && ctx->wave_persist != 0;
   // face scratch: planes of every grid, then the flagged-pencil list
   std::vector<SweepArgs> rec(ng);
-  std::vector<int64_t> mpre(ng + 1, 0), rpre(ng + 1, 0), fpre(ng + 1, 0), gpre(ng + 1, 0);
+  std::vector<int64_t> mpre(ng + 1, 0), rpre(ng + 1, 0), fpre(ng + 1, 0), gpre(ng + 1, 0),
+      upre(ng + 1, 0);
   // the fused face kernel serves the same plain two-shock path, without slope corrections
   bool fused = plain_riemann && ctx->sweep_mode == PPM_B200_SWEEP_FUSED &&
                      correction_planes(p) == 0;
   size_t scratch_doubles = 0, flag_bytes = 0;
-  int64_t total_pencils = 0;
+  int64_t total_pencils = 0, total_cells = 0;
   // colour field pointers of every grid, ncolour per grid
   const int nc = p->number_of_colours;
   double* const* col_dev = nullptr;
@@ -752,6 +753,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
                        (size_t)a.plane;
     scratch_doubles += correction_planes(p) * (size_t)(a.ie - a.is + 3) * (size_t)a.npencils;
     total_pencils += a.npencils;
+    total_cells += a.npencils * a.n;
     if (nc > 0) flag_bytes += (size_t)a.plane;
     const int64_t mb = (a.npencils + ppm::kMarchThreads - 1) / ppm::kMarchThreads;
     const int64_t rb = (int64_t)(a.ie - a.is + 2) * ((a.npencils + rt - 1) / rt);
@@ -759,14 +761,20 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
     rpre[k + 1] = rpre[k] + rb;
     fpre[k + 1] = fpre[k] + ppm::face_blocks(a.npencils, a.is, a.ie);
   }
-  // the marching stages' segments, once the batch's pencils are known
+  // the marching stages' path and segments, once the batch's pencils are known
   bool uneven = false;
-  const bool local_select = !p->dual_energy || p->eta1 <= 0.25 * p->eta2;
   for (int k = 0; k < ng; ++k) {
-    ppm::set_segments(rec[k], total_pencils, local_select);
     ppm::set_uniform(rec[k], io[k].g->cell_width[dim], ct.all.data() + ct.offset[k]);
     uneven = uneven || !rec[k].uniform;
-    gpre[k + 1] = gpre[k] + ppm::march_segment_blocks(rec[k]);
+  }
+  fused = fused && !uneven;  // the face kernel is the plain path's: one cell width
+  const bool transport = solver_code(p) == 0 && p->pressure_free != 1 && nc == 0 && !fused &&
+                         ppm::use_transport(total_cells);
+  const bool local_select = !p->dual_energy || p->eta1 <= 0.25 * p->eta2;
+  for (int k = 0; k < ng; ++k) {
+    ppm::set_segments(rec[k], total_pencils, local_select, transport);
+    gpre[k + 1] = gpre[k] + ppm::segment_blocks(rec[k], rec[k].pw_log2);
+    upre[k + 1] = upre[k] + ppm::segment_blocks(rec[k], rec[k].uw_log2);
   }
   // callers that queue several sweeps size the scratch for all of them first, so this
   // never moves the buffer under a sweep prepared earlier
@@ -890,6 +898,9 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   const size_t off_g = align256(img.size());
   img.resize(off_g);
   append(img, gpre.data(), gpre.size());
+  const size_t off_u = align256(img.size());
+  img.resize(off_u);
+  append(img, upre.data(), upre.size());
   const int slot = kSlotSweep0 + 3 * dim + position;
   rc = mirror_put(ctx, ctx->mirror[slot], img);
   if (rc) return rc;
@@ -899,7 +910,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.x_tma = 0;
   // the x sweep's staged update works on warps of 32 pencils
   bool whole_warps = true;
-  for (int k = 0; k < ng; ++k) whole_warps = whole_warps && rec[k].pw_log2 >= 5;
+  for (int k = 0; k < ng; ++k) whole_warps = whole_warps && rec[k].uw_log2 >= 5;
   plan.contiguous = dim == 0 && whole_warps;
   if (ng == 1 && plan.contiguous) set_x_tiles(plan.B, rec[0]);
   plan.B.x_tma_extra_tx = plan.B.x_tma ? ctx->debug_tma_extra : 0u;
@@ -916,6 +927,9 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.riemann_prefix = (const int64_t*)(base + off_r);
   plan.B.seg_prefix = (const int64_t*)(base + off_g);
   plan.B.seg_blocks = gpre[ng];
+  plan.B.upd_prefix = (const int64_t*)(base + off_u);
+  plan.B.upd_blocks = upre[ng];
+  plan.B.transport = transport ? 1 : 0;
   plan.B.counters = (unsigned long long*)ctx->counters.p;
   plan.B.flagged = (int64_t*)(scratch + scratch_doubles);
   plan.march_blocks = mpre[ng];
@@ -1495,6 +1509,9 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, b.riemann_prefix);
     key_put(k, b.seg_prefix);
     key_put(k, b.seg_blocks);
+    key_put(k, b.upd_prefix);
+    key_put(k, b.upd_blocks);
+    key_put(k, b.transport);
     key_put(k, b.counters);
     key_put(k, b.flagged);
     key_put(k, sp.sweep[s].march_blocks);

@@ -513,12 +513,13 @@ struct Flux {
   double df, ef, uf, vf, wf, gef, ub;
 };
 
-// db_out (optional): the Godunov density db, which the colour fluxes scale by
-// (flux_twoshock.F:251-259)
-template <bool DUAL>
-__device__ __forceinline__ Flux flux_twoshock(const FaceState& s, double pbar, double ubar,
-                                              double qc, const Phys& P,
-                                              double* db_out = nullptr) {
+// The state at the face (flux_twoshock.F:84-350): pressure, density, normal velocity.
+struct Godunov {
+  double pb, db, ub;
+};
+
+__device__ __forceinline__ Godunov godunov_state(const FaceState& s, double pbar, double ubar,
+                                                 const Phys& P) {
   const double gamma = P.gamma;
   double sn = copysign(1.0, -ubar);
   double u0, p0, d0;
@@ -570,29 +571,52 @@ __device__ __forceinline__ Flux flux_twoshock(const FaceState& s, double pbar, d
   if (l0 < 0.0) {
     pb = p0; db = d0; ub = u0;
   }
-  if (db_out) *db_out = db;
+  return Godunov{pb, db, ub};
+}
+
+// Its flux with the advected states of the side the velocity comes from (:351-396).
+template <bool DUAL>
+__device__ __forceinline__ Flux godunov_flux(const Godunov& G, const AdvState& s, double qc,
+                                             const Phys& P) {
+  const double pb = G.pb, db = G.db, ub = G.ub;
   double vb, wb, geb;
   if (ub > 0.0) {
     vb = s.vl; wb = s.wl; geb = s.gel;
   } else {
     vb = s.vr; wb = s.wr; geb = s.ger;
   }
-  double eb = qdiv(pb, P.gm1 * db) + 0.5 * (ub * ub + vb * vb + wb * wb);
-  double upb = pb * ub;
-  double dub = ub * db;
-  double duub = dub * ub;
-  double duvb = dub * vb;
-  double duwb = dub * wb;
-  double dueb = dub * eb;
+  // The multiply-adds of the tolerance build are written out and the products by dt/dx
+  // rounded, so that a flux is the same double whether it is stored to a plane or used
+  // where it is formed (the compiler would fuse that product into the update).
+  const double dub = ub * db;
+#if PPM_FAST_ALGEBRA
+  const double ke = fma(ub, ub, fma(vb, vb, __dmul_rn(wb, wb)));
+  const double eb = fma(0.5, ke, qdiv(pb, P.gm1 * db));
+  const double efl = fma(dub, eb, __dmul_rn(pb, ub)), ufl = fma(dub, ub, pb);
+#else
+  const double eb = pb / (P.gm1 * db) + 0.5 * (ub * ub + vb * vb + wb * wb);
+  const double efl = dub * eb + pb * ub, ufl = dub * ub + pb;
+#endif
   Flux f;
-  f.df = qc * dub;
-  f.ef = qc * (dueb + upb);
-  f.uf = qc * (duub + pb);
-  f.vf = qc * duvb;
-  f.wf = qc * duwb;
-  f.gef = DUAL ? qc * (dub * geb) : 0.0;
+  f.df = __dmul_rn(qc, dub);
+  f.ef = __dmul_rn(qc, efl);
+  f.uf = __dmul_rn(qc, ufl);
+  f.vf = __dmul_rn(qc, __dmul_rn(dub, vb));
+  f.wf = __dmul_rn(qc, __dmul_rn(dub, wb));
+  f.gef = DUAL ? __dmul_rn(qc, __dmul_rn(dub, geb)) : 0.0;
   f.ub = ub;
   return f;
+}
+
+// db_out (optional): the Godunov density db, which the colour fluxes scale by
+// (flux_twoshock.F:251-259)
+template <bool DUAL>
+__device__ __forceinline__ Flux flux_twoshock(const FaceState& s, double pbar, double ubar,
+                                              double qc, const Phys& P,
+                                              double* db_out = nullptr) {
+  const Godunov G = godunov_state(s, pbar, ubar, P);
+  if (db_out) *db_out = G.db;
+  return godunov_flux<DUAL>(G, AdvState{s.vl, s.vr, s.wl, s.wr, s.gel, s.ger}, qc, P);
 }
 
 // ------------------------------------------ flux_hll.F:111-258 for one face (no diffusion)

@@ -252,17 +252,20 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   const int64_t march_blocks = (a.npencils + ppm::kMarchThreads - 1) / ppm::kMarchThreads;
   const int64_t riemann_blocks =
       (int64_t)(a.ie - a.is + 2) * ((a.npencils + ppm::kRiemannThreads - 1) / ppm::kRiemannThreads);
-  ppm::set_segments(a, a.npencils, !p->dual_energy || p->eta1 <= 0.25 * p->eta2);
+  const bool transport = ppm::use_transport(a.npencils * a.n);
+  ppm::set_segments(a, a.npencils, !p->dual_energy || p->eta1 <= 0.25 * p->eta2, transport);
   ppm::set_uniform(a, in->cell_width[dim], table.data());
-  const int64_t seg_blocks = ppm::march_segment_blocks(a);
+  const int64_t seg_blocks = ppm::segment_blocks(a, a.pw_log2);
+  const int64_t upd_blocks = ppm::segment_blocks(a, a.uw_log2);
   const int64_t mpre[2] = {0, march_blocks}, rpre[2] = {0, riemann_blocks},
-                gpre[2] = {0, seg_blocks};
+                gpre[2] = {0, seg_blocks}, upre[2] = {0, upd_blocks};
   unsigned char img[kStaticDescBytes];
   std::memset(img, 0, sizeof(img));
   std::memcpy(img, &a, sizeof(a));
   std::memcpy(img + 768, mpre, sizeof(mpre));
   std::memcpy(img + 832, rpre, sizeof(rpre));
   std::memcpy(img + 896, gpre, sizeof(gpre));
+  std::memcpy(img + 960, upre, sizeof(upre));
   e = cudaMemcpyAsync(desc, img, sizeof(img), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return fail_cuda(e, "cudaMemcpyAsync");
   ppm::BatchArgs B;
@@ -273,12 +276,15 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   B.riemann_prefix = reinterpret_cast<const int64_t*>(desc + 832);
   B.seg_prefix = reinterpret_cast<const int64_t*>(desc + 896);
   B.seg_blocks = seg_blocks;
+  B.upd_prefix = reinterpret_cast<const int64_t*>(desc + 960);
+  B.upd_blocks = upd_blocks;
+  B.transport = transport ? 1 : 0;
   B.uneven = a.uniform ? 0 : 1;
   B.counters = counters;
   B.flagged = reinterpret_cast<int64_t*>(planes + (size_t)(ppm::kFaceVars + ppm::kFluxVars) *
                                                       (size_t)a.plane);
   ppm::launch_sweep_batch(B, march_blocks, riemann_blocks, p->dual_energy != 0, p->gravity != 0,
-                          st, nullptr, false, dim == 0 && a.pw_log2 >= 5);
+                          st, nullptr, false, dim == 0 && a.uw_log2 >= 5);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail_cuda(e, "sweep launch");
 

@@ -32,6 +32,8 @@ namespace split {
 enum { VD = 0, VP = 1, VU = 2, VV = 3, VW = 4, VGE = 5 };
 enum { SDL = 0, SDR, SPL, SPR, SUL, SUR, SVL, SVR, SWL, SWR, SGEL, SGER };
 enum { XDF = 0, XEF, XUF, XVF, XWF, XGEF, XUB };
+// the transport path's planes: the Godunov state of the face in place of its fluxes
+enum { XDB = XDF, XPB = XEF };
 
 __device__ __forceinline__ double ldg0(const double* __restrict__ p, int64_t off) {
   return p ? __ldg(p + off) : 0.0;
@@ -86,6 +88,41 @@ __device__ __forceinline__ Phys make_phys(const SweepArgs& a) {
   P.gp1 = a.gamma + 1.0;
   P.gm1 = a.gamma - 1.0;
   return P;
+}
+
+template <bool DUAL>
+__device__ __forceinline__ FaceState load_face(const SweepArgs& a, int64_t idx) {
+  const double* s = a.fstate + idx;
+  const int64_t pl = a.plane;
+  FaceState f;
+  f.dl = s[SDL * pl];
+  f.dr = s[SDR * pl];
+  f.pl = s[SPL * pl];
+  f.pr = s[SPR * pl];
+  f.ul = s[SUL * pl];
+  f.ur = s[SUR * pl];
+  f.vl = s[SVL * pl];
+  f.vr = s[SVR * pl];
+  f.wl = s[SWL * pl];
+  f.wr = s[SWR * pl];
+  f.gel = DUAL ? s[SGEL * pl] : 0.0;
+  f.ger = DUAL ? s[SGER * pl] : 0.0;
+  return f;
+}
+
+// The advected states (v, w, ge) of a face, which only the flux needs: the Riemann
+// kernel loads them after the Newton iteration, so they hold no registers during it.
+template <bool DUAL>
+__device__ __forceinline__ void load_face_advected(const SweepArgs& a, int64_t idx,
+                                                   FaceState& f) {
+  const double* s = a.fstate + idx;
+  const int64_t pl = a.plane;
+  f.vl = s[SVL * pl];
+  f.vr = s[SVR * pl];
+  f.wl = s[SWL * pl];
+  f.wr = s[SWR * pl];
+  f.gel = DUAL ? s[SGEL * pl] : 0.0;
+  f.ger = DUAL ? s[SGER * pl] : 0.0;
 }
 
 // ------------------------------------------------------------------ stage 0 (optional)
@@ -427,8 +464,8 @@ __global__ void __launch_bounds__(kMarchThreads,
          k < nflag; k += (unsigned long long)gridDim.x * blockDim.x) {
       const int64_t code = B.flagged[k];
       const SweepArgs& a = ONE ? B.one : B.grids[(int)(code >> 40)];
-      reconstruct_pencil<DUAL, GRAV, ROLE, COR>(
-          a, (int)(code & ((int64_t(1) << 40) - 1)), a.is, a.ie + 1);
+      const int pid = (int)(code & ((int64_t(1) << 40) - 1));
+      reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, pid, a.is, a.ie + 1);
     }
     return;
   }
@@ -440,41 +477,6 @@ __global__ void __launch_bounds__(kMarchThreads,
   if (pid >= a.npencils || f0 > a.ie + 1) return;
   const int f1 = f0 + a.seg_faces - 1;
   reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, pid, f0, f1 < a.ie + 1 ? f1 : a.ie + 1);
-}
-
-template <bool DUAL>
-__device__ __forceinline__ FaceState load_face(const SweepArgs& a, int64_t idx) {
-  const double* s = a.fstate + idx;
-  const int64_t pl = a.plane;
-  FaceState f;
-  f.dl = s[SDL * pl];
-  f.dr = s[SDR * pl];
-  f.pl = s[SPL * pl];
-  f.pr = s[SPR * pl];
-  f.ul = s[SUL * pl];
-  f.ur = s[SUR * pl];
-  f.vl = s[SVL * pl];
-  f.vr = s[SVR * pl];
-  f.wl = s[SWL * pl];
-  f.wr = s[SWR * pl];
-  f.gel = DUAL ? s[SGEL * pl] : 0.0;
-  f.ger = DUAL ? s[SGER * pl] : 0.0;
-  return f;
-}
-
-// The advected states (v, w, ge) of a face, which only the flux needs: the Riemann
-// kernel loads them after the Newton iteration, so they hold no registers during it.
-template <bool DUAL>
-__device__ __forceinline__ void load_face_advected(const SweepArgs& a, int64_t idx,
-                                                   FaceState& f) {
-  const double* s = a.fstate + idx;
-  const int64_t pl = a.plane;
-  f.vl = s[SVL * pl];
-  f.vr = s[SVR * pl];
-  f.wl = s[SWL * pl];
-  f.wr = s[SWR * pl];
-  f.gel = DUAL ? s[SGEL * pl] : 0.0;
-  f.ger = DUAL ? s[SGER * pl] : 0.0;
 }
 
 // ------------------------------------------------------------------ stage 2
@@ -500,10 +502,12 @@ __device__ __forceinline__ void load_face_advected(const SweepArgs& a, int64_t i
 // block list (B.riemann_total entries) with a stride of the grid, keeping each grid's
 // record in shared memory while consecutive blocks belong to it.  RT and PERSIST are the
 // level autotuner's choices per size class (ppm_b200_autotune_level).
+// STATE: write the Godunov state of the face (pressure, density, velocity: three planes)
+// for the transport kernel, which forms the flux; without it the seven flux planes.
 // PLANE (with LEARNED): the net's output and |x|^2 of each face come from the guess
 // pass, in the face's slot of the XUB plane.
 template <bool DUAL, bool ONE, bool LEARNED, bool COL = false, int RT = kRiemannThreads,
-          bool PERSIST = false, bool PLANE = false>
+          bool PERSIST = false, bool PLANE = false, bool STATE = false>
 __global__ void __launch_bounds__(RT, (LEARNED ? PPM_RIEMANN_LEARNED_MINBLOCKS
                                                : PPM_RIEMANN_MINBLOCKS) * kRiemannThreads / RT)
     riemann_kernel(const __grid_constant__ BatchArgs B) {
@@ -593,20 +597,27 @@ __global__ void __launch_bounds__(RT, (LEARNED ? PPM_RIEMANN_LEARNED_MINBLOCKS
         }
       }
     }
-    const double qc = qdiv(P.dt, a.coef[a.is + fi].dx);
-    load_face_advected<DUAL>(a, idx, s);
-    double db;
-    const Flux F = flux_twoshock<DUAL>(s, rs.pbar, rs.ubar, qc, P, COL ? &db : nullptr);
     double* o = a.fflux + idx;
     const int64_t pl = a.plane;
-    if (COL) a.fcol[CDB * pl + idx] = db;
-    o[XDF * pl] = F.df;
-    o[XEF * pl] = F.ef;
-    o[XUF * pl] = F.uf;
-    o[XVF * pl] = F.vf;
-    o[XWF * pl] = F.wf;
-    if (DUAL) o[XGEF * pl] = F.gef;
-    o[XUB * pl] = F.ub;
+    if (STATE) {
+      const Godunov G = godunov_state(s, rs.pbar, rs.ubar, P);
+      o[XPB * pl] = G.pb;
+      o[XDB * pl] = G.db;
+      o[XUB * pl] = G.ub;
+    } else {
+      const double qc = qdiv(P.dt, a.coef[a.is + fi].dx);
+      load_face_advected<DUAL>(a, idx, s);
+      double db;
+      const Flux F = flux_twoshock<DUAL>(s, rs.pbar, rs.ubar, qc, P, COL ? &db : nullptr);
+      if (COL) a.fcol[CDB * pl + idx] = db;
+      o[XDF * pl] = F.df;
+      o[XEF * pl] = F.ef;
+      o[XUF * pl] = F.uf;
+      o[XVF * pl] = F.vf;
+      o[XWF * pl] = F.wf;
+      if (DUAL) o[XGEF * pl] = F.gef;
+      o[XUB * pl] = F.ub;
+    }
     atomicAdd(&s_hist[rs.iters & 7], 1u);
     atomicAdd(&s_newton, (unsigned)rs.iters + spent);
     trips = (unsigned)rs.iters + spent;
@@ -1118,7 +1129,10 @@ __device__ __forceinline__ Cell pipe_cell(const SweepArgs& a, const double* r) {
 #define PPM_X_TMA 1
 #endif
 constexpr int kXTile = kXTileRows * kXTileCells;       // doubles per field and buffer
-constexpr int kXWarp = kXBuffers * 6 * kXTile;         // doubles per warp
+template <int NF>
+__host__ __device__ constexpr int x_warp_doubles() {   // NF fields: doubles per warp
+  return kXBuffers * NF * kXTile;
+}
 constexpr long long kXWaitCycles = 2000000000ll;       // ~1 s at the B200's clocks
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
@@ -1174,28 +1188,51 @@ struct XTiles {
 };
 
 // chunks q count from the segment's first
+template <int NF>
 __device__ __forceinline__ void x_issue(XTiles& x, int q) {
   const int b = q % kXBuffers;
   if ((threadIdx.x & 31) == 0) {
     mbar_expect_tx(x.bar + b, x.bytes);
 #pragma unroll
-    for (int f = 0; f < 6; ++f)
+    for (int f = 0; f < NF; ++f)
       if (x.fields & (1u << f))
-        tma_load_2d(x.buf + (b * 6 + f) * kXTile, x.map + f, (x.q0 + q) * kXTileCells, x.row0, x.bar + b);
+        tma_load_2d(x.buf + (b * NF + f) * kXTile, x.map + f, (x.q0 + q) * kXTileCells, x.row0, x.bar + b);
   }
   x.last = q;
 }
 
 // warp-uniform: called by every lane at its first step in chunk q; n: cells end (exclusive)
+template <int NF>
 __device__ __forceinline__ void x_chunk(XTiles& x, int q, int n) {
   __syncwarp();  // every lane has read chunk q-1, whose buffer the next copy reuses
   if (x.broken) return;
   const int next = q + kXBuffers - 1;
-  if ((x.q0 + next) * kXTileCells < n) x_issue(x, next);
+  if ((x.q0 + next) * kXTileCells < n) x_issue<NF>(x, next);
   const bool ok = mbar_wait_bounded(x.bar + q % kXBuffers, (unsigned)(q / kXBuffers) & 1u);
   if (__any_sync(0xffffffffu, !ok)) {
     x.broken = true;
     if ((threadIdx.x & 31) == 0) atomicAdd(x.timeouts, 1ull);
+  }
+}
+
+// one warp's tiles of the fields (bits into B.xin), pencils row0 .. row0+31
+__device__ __forceinline__ void x_setup(XTiles& x, const BatchArgs& B, double* buf,
+                                        uint64_t* bar, int row0, unsigned fields) {
+  x.buf = buf;
+  x.bar = bar;
+  x.map = B.xin;
+  x.timeouts = B.counters + kCntTimeout;
+  x.fields = fields;
+  x.bytes = (unsigned)__popc(fields) * kXTile * (unsigned)sizeof(double) + B.x_tma_extra_tx;
+  x.row0 = row0;
+  x.q0 = 0;
+  x.last = -1;
+  x.broken = false;
+  if ((threadIdx.x & 31) == 0) {
+    for (int b = 0; b < kXBuffers; ++b) mbar_init(bar + b, 1);
+    // the barriers' initialisation is visible to the tensor-memory accelerator
+    asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::
+                     : "memory");
   }
 }
 
@@ -1208,10 +1245,16 @@ __device__ __forceinline__ void x_drain(XTiles& x) {
   }
 }
 
+// this lane's row of the tile of cell t
+template <int NF>
+__device__ __forceinline__ const double* x_row(const XTiles& x, int t) {
+  return x.buf + ((t / kXTileCells - x.q0) % kXBuffers) * (NF * kXTile) +
+         (threadIdx.x & 31) * kXTileCells + t % kXTileCells;
+}
+
 template <bool DUAL>
 __device__ __forceinline__ Cell x_cell(const XTiles& x, const SweepArgs& a, int t) {
-  const double* r = x.buf + ((t / kXTileCells - x.q0) % kXBuffers) * (6 * kXTile) +
-                    (threadIdx.x & 31) * kXTileCells + t % kXTileCells;
+  const double* r = x_row<6>(x, t);
   Cell c;
   c.d = r[0];
   c.e = r[kXTile];
@@ -1460,7 +1503,8 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
   }
   if (XT) {  // warp-wide, live or not: the first chunks
     xt->q0 = cb / kXTileCells;
-    for (int q = 0; q < kXBuffers - 1 && (xt->q0 + q) * kXTileCells <= ce; ++q) x_issue(*xt, q);
+    for (int q = 0; q < kXBuffers - 1 && (xt->q0 + q) * kXTileCells <= ce; ++q)
+      x_issue<6>(*xt, q);
   }
 
   // One step of the march.  ST (steady): t in [is+2, ie-1] and [c0+2, c1], where cell t,
@@ -1470,7 +1514,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
   auto step = [&](const int t, auto steady) {
     constexpr bool ST = decltype(steady)::value;
     if (XT && (ST || t <= ce) && (t % kXTileCells == 0 || (!ST && t == cb)))
-      x_chunk(*xt, t / kXTileCells - xt->q0, ce + 1);
+      x_chunk<6>(*xt, t / kXTileCells - xt->q0, ce + 1);
     Cell Cn = Cm;
     double ges_n = 0.0;
     Flux F1 = F0;
@@ -1695,13 +1739,45 @@ __host__ __device__ constexpr int update_pipe() {
   return STAGED ? 0 : (ONE ? PPM_UPDATE_PIPE_ONE : PPM_UPDATE_PIPE_BATCH);
 }
 constexpr int kStageBlock = (kMarchThreads / 32) * kStageWarp;
-constexpr int kXBlock = (kMarchThreads / 32) * kXWarp;
+constexpr int kXBlock = (kMarchThreads / 32) * x_warp_doubles<6>();
 // dynamic shared memory of the update kernel: the x sweep's TMA tiles (XT) and output
 // staging, one of each per warp, or the y and z sweeps' input ring
 template <bool ONE, bool STAGED, bool XT>
 constexpr size_t update_smem_bytes() {
   return sizeof(double) * ((XT ? kXBlock : 0) + (STAGED ? kStageBlock : 0) +
                            ring_doubles<update_pipe<ONE, STAGED>()>());
+}
+
+// The end of an update or transport block: flagged pencils onto the fallback list (their
+// counts and time step come from the fallback pass), the other threads' counts and the
+// block's smallest time step.  first: the thread of its pencil that lists it.
+__device__ __forceinline__ void finish_block(const BatchArgs& B, const SweepArgs& a, int g,
+                                             int pid, bool first, const unsigned char* s_flag,
+                                             int pl, unsigned long long* s_cnt,
+                                             const UpdateCounts& cnt) {
+  double my_dt = 1.0e20;
+  __syncthreads();
+  if (s_flag[pl]) {
+    if (first) {
+      const unsigned long long slot = atomicAdd(&B.counters[kCntFlagged], 1ull);
+      B.flagged[slot] = ((int64_t)g << 40) | pid;
+    }
+  } else {
+    if (cnt.fatal) atomicAdd(&s_cnt[0], (unsigned long long)cnt.fatal);
+    if (cnt.nonfinite) atomicAdd(&s_cnt[1], (unsigned long long)cnt.nonfinite);
+    my_dt = cnt.dtmin;
+  }
+  if (a.cfl_min_bits) {  // warp minimum, one atomic per warp (every lane reaches this)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) my_dt = dmin(my_dt, __shfl_xor_sync(0xffffffffu, my_dt, o));
+    if ((threadIdx.x & 31) == 0 && my_dt < 1.0e20)
+      atomicMin(a.cfl_min_bits, (unsigned long long)__double_as_longlong(my_dt));
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_cnt[0]) atomicAdd(&B.counters[kCntFatal], s_cnt[0]);
+    if (s_cnt[1]) atomicAdd(&B.counters[kCntNonFinite], s_cnt[1]);
+  }
 }
 
 // STAGED: the x sweep (pencils along the contiguous axis) with staged outputs; XT: its
@@ -1724,39 +1800,23 @@ __global__ void __launch_bounds__(kMarchThreads,
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
   s_flag[threadIdx.x] = 0;
   int64_t lb;
-  const int g = locate<ONE>(B.seg_prefix, B.ngrids, lb);
+  const int g = locate<ONE>(B.upd_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
   // a block holds every segment of its pencils, so what one segment finds (a cell for the
   // fallback pass) reaches the pencil's other segments through shared memory
-  const int pl = threadIdx.x & ((1 << a.pw_log2) - 1);
-  const int pid = (int)(lb << a.pw_log2) + pl;
+  const int pl = threadIdx.x & ((1 << a.uw_log2) - 1);
+  const int pid = (int)(lb << a.uw_log2) + pl;
   const int wpid0 = pid - (threadIdx.x & 31);  // first pencil of this warp (STAGED)
-  const int c0 = (int)(threadIdx.x >> a.pw_log2) * a.seg_cells;
+  const int c0 = (int)(threadIdx.x >> a.uw_log2) * a.seg_cells;
   const int c1 = c0 + a.seg_cells - 1 < a.n - 1 ? c0 + a.seg_cells - 1 : a.n - 1;
   const int warp = threadIdx.x >> 5;
   XTiles xt;
   if (XT) {
-    xt.buf = s_xtile + warp * kXWarp;
-    xt.bar = s_xbar + warp * kXBuffers;
-    xt.map = B.xin;
-    xt.timeouts = B.counters + kCntTimeout;
-    xt.fields = 3u | (a.in_u ? 4u : 0u) | (a.in_v ? 8u : 0u) | (a.in_w ? 16u : 0u) |
-                ((DUAL && a.in_ge) ? 32u : 0u);
-    xt.bytes = (unsigned)__popc(xt.fields) * kXTile * (unsigned)sizeof(double) +
-               B.x_tma_extra_tx;
-    xt.row0 = (int)wpid0;
-    xt.q0 = 0;
-    xt.last = -1;
-    xt.broken = false;
-    if ((threadIdx.x & 31) == 0) {
-      for (int b = 0; b < kXBuffers; ++b) mbar_init(xt.bar + b, 1);
-      // the barriers' initialisation is visible to the tensor-memory accelerator
-      asm volatile("fence.mbarrier_init.release.cluster;\n\tfence.proxy.async.shared::cta;" ::
-                       : "memory");
-    }
+    x_setup(xt, B, s_xtile + warp * x_warp_doubles<6>(), s_xbar + warp * kXBuffers, wpid0,
+            3u | (a.in_u ? 4u : 0u) | (a.in_v ? 8u : 0u) | (a.in_w ? 16u : 0u) |
+                ((DUAL && a.in_ge) ? 32u : 0u));
   }
   if (ONE) __syncthreads();
-  double my_dt = 1.0e20;
   const bool valid = pid < a.npencils;
   UpdateCounts cnt = {0, 0, 0, 1.0e20};
   if ((STAGED || valid) && c0 < a.n) {
@@ -1766,38 +1826,43 @@ __global__ void __launch_bounds__(kMarchThreads,
             s_ring + threadIdx.x, &xt))
       s_flag[pl] = 1;
   }
-  __syncthreads();
-  if (s_flag[pl]) {  // a flagged pencil's counts and time step come from the fallback pass
-    if (valid && c0 == 0) {
-      const unsigned long long slot = atomicAdd(&B.counters[kCntFlagged], 1ull);
-      B.flagged[slot] = ((int64_t)g << 40) | pid;
-    }
-  } else {
-    if (cnt.fatal) atomicAdd(&s_cnt[0], (unsigned long long)cnt.fatal);
-    if (cnt.nonfinite) atomicAdd(&s_cnt[1], (unsigned long long)cnt.nonfinite);
-    my_dt = cnt.dtmin;
-  }
-  if (a.cfl_min_bits) {  // warp minimum, one atomic per warp (every lane reaches this)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) my_dt = dmin(my_dt, __shfl_xor_sync(0xffffffffu, my_dt, o));
-    if ((threadIdx.x & 31) == 0 && my_dt < 1.0e20)
-      atomicMin(a.cfl_min_bits, (unsigned long long)__double_as_longlong(my_dt));
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (s_cnt[0]) atomicAdd(&B.counters[kCntFatal], s_cnt[0]);
-    if (s_cnt[1]) atomicAdd(&B.counters[kCntNonFinite], s_cnt[1]);
+  finish_block(B, a, g, pid, valid && c0 == 0, s_flag, pl, s_cnt, cnt);
+}
+
+// The transport path's planes of one pencil made the fallback pass's: its advected states,
+// which the transport kernel keeps to itself, and its fluxes in place of the Godunov states.
+template <bool DUAL, bool GRAV, bool COR>
+__device__ __noinline__ void fill_pencil(const SweepArgs& a, int pid) {
+  reconstruct_pencil<DUAL, GRAV, 1, COR>(a, pid, a.is, a.ie + 1);
+  const Phys P = make_phys(a);
+  const int64_t pl = a.plane;
+  for (int f = a.is; f <= a.ie + 1; ++f) {
+    const int64_t idx = (int64_t)(f - a.is) * a.npencils + pid;
+    double* o = a.fflux + idx;
+    const Godunov G{o[XPB * pl], o[XDB * pl], o[XUB * pl]};
+    FaceState s;
+    load_face_advected<DUAL>(a, idx, s);
+    const Flux F = godunov_flux<DUAL>(G, AdvState{s.vl, s.vr, s.wl, s.wr, s.gel, s.ger},
+                                      qdiv(P.dt, a.coef[f].dx), P);
+    o[XDF * pl] = F.df;
+    o[XEF * pl] = F.ef;
+    o[XUF * pl] = F.uf;
+    o[XVF * pl] = F.vf;
+    o[XWF * pl] = F.wf;
+    if (DUAL) o[XGEF * pl] = F.gef;
   }
 }
 
-// The fallback pass: a fixed grid that walks the list of flagged pencils.
-template <bool DUAL, bool GRAV, bool ONE, bool RS = false>
+// The fallback pass: a fixed grid that walks the list of flagged pencils.  TRANS: after the
+// transport kernel.
+template <bool DUAL, bool GRAV, bool ONE, bool RS = false, bool TRANS = false, bool COR = false>
 __global__ void __launch_bounds__(128) fallback_kernel(const __grid_constant__ BatchArgs B) {
   const unsigned long long nflag = *(volatile unsigned long long*)&B.counters[kCntFlagged];
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
        k < nflag; k += (unsigned long long)gridDim.x * blockDim.x) {
     const int64_t code = B.flagged[k];
     const SweepArgs& a = ONE ? B.one : B.grids[(int)(code >> 40)];
+    if (TRANS) fill_pencil<DUAL, GRAV, COR>(a, (int)(code & ((int64_t(1) << 40) - 1)));
     const Phys P = make_phys(a);
     UpdateCounts cnt = {0, 0, 0, 1.0e20};
     update_pencil<DUAL, GRAV, true, false, 0, false, RS>(
@@ -1808,6 +1873,441 @@ __global__ void __launch_bounds__(128) fallback_kernel(const __grid_constant__ B
     if (cnt.fatal) atomicAdd(&B.counters[kCntFatal], (unsigned long long)cnt.fatal);
     if (cnt.nonfinite) atomicAdd(&B.counters[kCntNonFinite], (unsigned long long)cnt.nonfinite);
   }
+}
+
+// ------------------------------------------------------------------ stages 1b+3 fused
+// The transport kernel of the plain path (two-shock solver, no colours): the advected
+// states (v, w, ge), the fluxes and the update of a pencil segment in one march, so
+// neither the six advected state planes nor the flux planes exist: it reads the Godunov
+// state of every face (three planes), 128 bytes a cell with the fields, where the two
+// kernels it stands for moved 150 and the Riemann kernel 85 more than it does now.
+// A step t loads cell t, reconstructs v, w, ge at cell t-2 and face t-2 (the body of
+// reconstruct_pencil's ROLE 1), forms that face's flux, checks and updates cell t-3
+// (update_pencil's stages 1 and 2) and selects and stores cell t-4 (its stage 3).
+// Segments as in update_pencil: outputs c0 .. c1, updates of cells cb .. ce, faces
+// fa .. fb, loads from three cells left of cb to three right of ce.  A pencil with a cell
+// that fails its check goes to the fallback pass.
+// PD: the inputs arrive through a cp.async ring PD steps ahead, as in update_pencil;
+// STAGED: the x sweep's staged stores, with plain loads a step ahead, or XT, its input
+// cells as TMA tiles.
+enum { UD = 0, UP, UU, UV, UW, UGE, UE, UPB, UDB, UUB, UG, kTransVals };
+template <int PD>
+__host__ __device__ constexpr int trans_ring_doubles() {
+  return PD > 0 ? (PD + 1) * kTransVals * kMarchThreads : 0;
+}
+constexpr int kTransTiles = 7;  // TMA tiles: d, e, u, v, w, ge, p (BatchArgs::xin)
+
+template <bool DUAL, bool GRAV, bool COR, bool STAGED, int PD, bool XT>
+__device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, const Phys& P,
+                                                 UpdateCounts& cnt, int c0, int c1, bool valid,
+                                                 double* stage, int pid0, double* ring,
+                                                 XTiles* xt) {
+  static_assert(!(PD > 0 && STAGED), "the ring serves the y and z sweeps");
+  constexpr int NV = DUAL ? 3 : 2;
+  bool live = valid, flagged = false, handed = false;
+  const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
+  const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
+  const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
+  double dtmin = 1.0e20;
+  const int sa = (int)a.sa, np = (int)a.npencils;
+  const int n = a.n, is = a.is, ie = a.ie;
+  const int cb = c0 > 0 ? c0 - 1 : 0, ce = c1 < n - 1 ? c1 + 1 : n - 1;
+  const int fa = cb > is ? cb : is, fb = ce < ie ? ce + 1 : ie + 1;
+  const int lo = cb > 3 ? cb - 3 : 0, hi = ce + 3 < n - 1 ? ce + 3 : n - 1;
+  const double qdx = P.dt / a.uc.dx, qcx = qdiv(P.dt, a.uc.dx);
+  const int64_t pl = a.plane;
+  const double* const god = a.fflux + pid;
+
+  int64_t cap = 0, cap_end = 0;
+  if (a.ncaptures > 0) {
+    int64_t l = 0, h = a.ncaptures;
+    while (l < h) {
+      int64_t mid = (l + h) >> 1;
+      if (a.captures[mid].pencil < pid) l = mid + 1; else h = mid;
+    }
+    cap = cap_end = l;
+    while (cap_end < a.ncaptures && a.captures[cap_end].pencil == pid) ++cap_end;
+    while (cap < cap_end && a.captures[cap].face < c0) ++cap;
+  }
+
+  // inputs of step t: cell t, the energy (and acceleration) of cell t-3, face t-2
+  double in[kTransVals];  // the next step's values (neither PD nor XT)
+#pragma unroll
+  for (int k = 0; k < kTransVals; ++k) in[k] = 0.0;
+  auto fetch = [&](const int t, auto steady) {
+    constexpr bool ST = decltype(steady)::value;
+    double* r = PD > 0 ? ring + (t % (PD + 1)) * (kTransVals * kMarchThreads) : nullptr;
+    auto get = [&](int k, const double* p) {
+      if (PD > 0)
+        cp_async8(r + k * kMarchThreads, p);
+      else if (STAGED && k < UPB)
+        in[k] = ldg_keep(p);
+      else
+        in[k] = __ldcs(p);
+    };
+    if (!XT && (ST || t <= hi)) {
+      const int off = base + t * sa;
+      get(UD, a.in_d + off);
+      get(UP, a.pres + off);
+      if (a.in_u) get(UU, a.in_u + off);
+      if (a.in_v) get(UV, a.in_v + off);
+      if (a.in_w) get(UW, a.in_w + off);
+      if (DUAL) get(UGE, a.in_ge + off);
+    }
+    if (ST || (t - 3 >= cb && t - 3 <= ce)) {
+      const int off = base + (t - 3) * sa;
+      if (!XT) get(UE, a.in_e + off);
+      if (GRAV) get(UG, a.grav + off);
+    }
+    if (ST || (t - 2 >= fa && t - 2 <= fb)) {
+      const double* f = god + (t - 2 - is) * np;
+      get(UPB, f + XPB * pl);
+      get(UDB, f + XDB * pl);
+      get(UUB, f + XUB * pl);
+    }
+    if (PD > 0) cp_async_commit();
+  };
+
+  double wq0[3], wq1[3], wq2[3];  // v, w, ge of cells t-3, t-2, t-1
+  double dqm1[3], qlm1[3];        // dq(t-2), ql(t-2)
+#pragma unroll
+  for (int v = 0; v < 3; ++v) wq0[v] = wq1[v] = wq2[v] = dqm1[v] = qlm1[v] = 0.0;
+  double wu0 = 0.0, wu1 = 0.0, wu2 = 0.0, wd0 = 0.0, wd1 = 0.0, wd2 = 0.0;  // u, d: same cells
+  double we0 = 0.0, we1 = 0.0, we2 = 0.0;                                   // e (XT)
+  Prep prA = {0, 0, 0, 0, 0}, prB = {0, 0, 0, 0, 0};                        // cells t-2, t-1
+  AdvL aL = {};                     // left data of face t-2
+  Flux F0 = {0, 0, 0, 0, 0, 0, 0};  // flux at face t-3
+  Cell PEm = {0, 0, 0, 0, 0, 0};    // post-euler state of cell t-4
+  double dep = 0.0;                 // post-select d*e of cell t-5
+  unsigned int nonfin = 0;
+
+  auto store = [&](const int c, const Cell& o) {
+    if (STAGED) {
+      double* sp = stage + (c % kStageCells) * kStageLd + (threadIdx.x & 31);
+      sp[0] = o.d;
+      sp[kStageField] = o.e;
+      sp[2 * kStageField] = o.u;
+      sp[3 * kStageField] = o.v;
+      sp[4 * kStageField] = o.w;
+      if (DUAL) sp[5 * kStageField] = o.ge;
+    } else {
+      const int off = base + c * sa;
+      a.out_d[off] = o.d;
+      a.out_e[off] = o.e;
+      if (a.out_u) a.out_u[off] = o.u;
+      if (a.out_v) a.out_v[off] = o.v;
+      if (a.out_w) a.out_w[off] = o.w;
+      if (DUAL) a.out_ge[off] = o.ge;
+    }
+  };
+
+  // One step.  ST (steady): every range test below holds, and the next fetch is whole.
+  auto step = [&](const int t, auto steady) {
+    constexpr bool ST = decltype(steady)::value;
+    double nq[3] = {wq2[0], wq2[1], wq2[2]}, nu = wu2, nd = wd2, np_ = 0.0, ne = 0.0;
+    double e3 = we0, g3 = 0.0;
+    Godunov G = {0.0, 0.0, 0.0};
+    if (XT && (ST || t <= hi) && (t % kXTileCells == 0 || (!ST && t == lo)))
+      x_chunk<kTransTiles>(*xt, t / kXTileCells - xt->q0, hi + 1);
+    if (live) {
+      if (PD > 0) {
+        cp_async_wait<(PD > 0 ? PD - 1 : 0)>();
+        const double* r = ring + (t % (PD + 1)) * (kTransVals * kMarchThreads);
+        if (ST || t <= hi) {
+          nd = r[UD * kMarchThreads];
+          np_ = r[UP * kMarchThreads];
+          nu = a.in_u ? r[UU * kMarchThreads] : 0.0;
+          nq[0] = a.in_v ? r[UV * kMarchThreads] : 0.0;
+          nq[1] = a.in_w ? r[UW * kMarchThreads] : 0.0;
+          nq[2] = DUAL ? r[UGE * kMarchThreads] : 0.0;
+        }
+        if (ST || (t - 3 >= cb && t - 3 <= ce)) {
+          e3 = r[UE * kMarchThreads];
+          if (GRAV) g3 = r[UG * kMarchThreads];
+        }
+        if (ST || (t - 2 >= fa && t - 2 <= fb))
+          G = Godunov{r[UPB * kMarchThreads], r[UDB * kMarchThreads], r[UUB * kMarchThreads]};
+        fetch(t + PD, steady);
+      } else {
+        if (XT) {
+          if (ST || t <= hi) {
+            const double* r = x_row<kTransTiles>(*xt, t);
+            nd = r[0];
+            ne = r[kXTile];
+            nu = a.in_u ? r[2 * kXTile] : 0.0;
+            nq[0] = a.in_v ? r[3 * kXTile] : 0.0;
+            nq[1] = a.in_w ? r[4 * kXTile] : 0.0;
+            nq[2] = DUAL ? r[5 * kXTile] : 0.0;
+            np_ = r[6 * kXTile];
+          }
+        } else {
+          nd = in[UD];
+          np_ = in[UP];
+          nu = in[UU];
+          nq[0] = in[UV];
+          nq[1] = in[UW];
+          nq[2] = in[UGE];
+          e3 = in[UE];
+        }
+        g3 = in[UG];
+        G = Godunov{in[UPB], in[UDB], in[UUB]};
+        fetch(t + 1, steady);
+      }
+    }
+    // ---- reconstruction of v, w, ge (reconstruct_pencil, ROLE 1)
+    Prep prC = prB;
+    if (ST || (t >= fa - 1 && t <= fb)) prC = cell_prep(nd, np_, nu, COR ? a.coef[t].dx2i : a.uc.dx2i, P);
+    double dqN[3], qlN[3];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) dqN[v] = qlN[v] = 0.0;
+    if (ST || (t - 1 >= fa - 2 && t - 1 <= fb + 1)) {
+      const Coef& cf = COR ? a.coef[t - 1] : a.uc;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        dqN[v] = pm_slope<!COR>(wq1[v], wq2[v], nq[v], cf.c1, cf.c2);
+        if (ST || t - 1 >= fa - 1)
+          qlN[v] = pm_edge(wq1[v], wq2[v], dqm1[v], dqN[v], cf.c3, cf.c4, cf.c5, cf.c6);
+      }
+    }
+    Flux F1 = F0;
+    AdvL aN = aL;
+    if (ST || (t - 2 >= fa - 1 && t - 2 <= fb)) {
+      const int c = t - 2;
+      Para pa[3];
+      pa[2] = Para{0.0, 0.0, 0.0, 0.0};
+      if (COR && a.flatten != 0 && live) {
+        const double fl = a.flat[(c - (is - 1)) * np + pid];
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          pa[v] = pm_parabola<false, true>(wq0[v], wq1[v], wq2[v], qlm1[v], qlN[v], 0.0, 0.0,
+                                           0.0, fl);
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+          pa[v] = pm_parabola<false, false, !COR>(wq0[v], wq1[v], wq2[v], qlm1[v], qlN[v]);
+      }
+      if (ST || c >= fa) {
+        AdvR R;
+        R.vra = pm_C(pa[0], prA.char2);
+        R.vr0 = pm_B(pa[0], prA.c0);
+        R.wra = pm_C(pa[1], prA.char2);
+        R.wr0 = pm_B(pa[1], prA.c0);
+        R.gera = DUAL ? pm_C(pa[2], prA.char2) : 0.0;
+        R.ger0 = DUAL ? pm_B(pa[2], prA.c0) : 0.0;
+        F1 = godunov_flux<DUAL>(G, face_advected(aL, R, wu0, wu1),
+                                COR ? qdiv(P.dt, a.coef[c].dx) : qcx, P);
+      }
+      aN.vla = pm_A(pa[0], prA.char1);
+      aN.vl0 = pm_A(pa[0], prA.c0);
+      aN.wla = pm_A(pa[1], prA.char1);
+      aN.wl0 = pm_A(pa[1], prA.c0);
+      aN.gela = DUAL ? pm_A(pa[2], prA.char1) : 0.0;
+      aN.gel0 = DUAL ? pm_A(pa[2], prA.c0) : 0.0;
+    }
+    // ---- check and update of cell t-3 (update_pencil)
+    const int c = t - 3;
+    Cell PEn = {wd0, e3, wu0, wq0[0], wq0[1], wq0[2]};
+    if (live && (ST || (c >= is && c <= ie && c >= cb))) {
+      const Cell C = PEn;
+      double ges = 0.0;
+      if (DUAL) {
+        const double pcent = dmax(P.gm1 * C.ge * C.d, kTiny);
+        ges = (COR && !a.uniform ? P.dt / a.coef[c].dx : qdx) * pcent * (F0.ub - F1.ub);
+      }
+      if (C.d + (F0.df - F1.df) <= 0.0 || C.e < 0.0) {  // to the fallback pass
+        if (!STAGED) {
+          if (PD > 0) cp_async_wait<0>();
+          handed = true;
+          return;
+        }
+        live = false;
+        flagged = true;
+      }
+      // subgrid flux capture: face c, and face ie+1 with the last cell
+      while (cap < cap_end && (ST || c <= c1) && a.captures[cap].face <= c + (c == ie ? 1 : 0)) {
+        const FluxCapture& rq = a.captures[cap];
+        const Flux& F = (rq.face == c) ? F0 : F1;
+        double* dst = a.capture_buf + rq.dst;
+        dst[0] = F.df; dst[1] = F.ef; dst[2] = F.uf;
+        dst[3] = F.vf; dst[4] = F.wf; dst[5] = DUAL ? F.gef : 0.0;
+        ++cap;
+      }
+      bool fatal = false;
+      PEn = euler_update<DUAL, GRAV>(C, F0, F1, ges, g3, P, fatal);
+      if (fatal && live && (ST || (c >= c0 && c <= c1))) cnt.fatal += 1;
+    }
+    // ---- select and store of cell t-4
+    {
+      const int k = t - 4;
+      if (DUAL && !ST && live && k == c0 - 1 && c0 > 0) {
+        bool known;
+        dep = pgas2d_de_local(PEm, P, known);
+        if (!known) {
+          if (!STAGED) {
+            if (PD > 0) cp_async_wait<0>();
+            handed = true;
+            return;
+          }
+          live = false;
+          flagged = true;
+        }
+      }
+      if (live && (ST || k >= c0)) {
+        Cell o = PEm;
+        if (DUAL) {
+          const double own = o.d * o.e;
+          const double de_m = (!ST && k == 0) ? own : dep;
+          pgas2d_dual(o, de_m, PEn.d * PEn.e, P);  // k < n-1 here
+          dep = o.d * o.e;
+        }
+        if (!isfinite(o.d) || !isfinite(o.e)) nonfin += 1;
+        if (cfl && (ST || (k >= is && k <= ie)))
+          dtmin = dmin(dtmin, cell_dt1<DUAL>(a, o, COR && !a.uniform ? a.coef[k].dx : a.uc.dx,
+                                             t1, t2, P));
+        store(k, o);
+      }
+      if (STAGED && (ST || k >= c0) && k % kStageCells == kStageCells - 1)
+        flush_stage<DUAL>(a, stage, pid0, k - (kStageCells - 1), kStageCells);
+    }
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+      wq0[v] = wq1[v];
+      wq1[v] = wq2[v];
+      wq2[v] = nq[v];
+      dqm1[v] = dqN[v];
+      qlm1[v] = qlN[v];
+    }
+    wu0 = wu1;
+    wu1 = wu2;
+    wu2 = nu;
+    wd0 = wd1;
+    wd1 = wd2;
+    wd2 = nd;
+    if (XT) {
+      we0 = we1;
+      we1 = we2;
+      we2 = ne;
+    }
+    prA = prB;
+    prB = prC;
+    aL = aN;
+    F0 = F1;
+    PEm = PEn;
+  };
+  using Ramp = std::integral_constant<bool, false>;
+  using Steady = std::integral_constant<bool, true>;
+  if (XT) {
+    xt->q0 = lo / kXTileCells;
+    for (int q = 0; q < kXBuffers - 1 && (xt->q0 + q) * kXTileCells <= hi; ++q)
+      x_issue<kTransTiles>(*xt, q);
+  }
+  constexpr int AHEAD = PD > 0 ? PD : 1;
+  if (live) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) fetch(lo + u, Ramp{});
+  }
+  const int tlast = ce + 3;
+  auto max2 = [](int x, int y) { return x > y ? x : y; };
+  auto min2 = [](int x, int y) { return x < y ? x : y; };
+  // every range of a steady step, and of the steps it fetches for
+  const int s0 = max2(max2(fa + 2, is + 3), c0 + 4);
+  const int s1 = min2(min2(hi, fb + 2), min2(ie + 3, c1 + 3)) - AHEAD;
+#pragma unroll 1
+  for (int t = lo; t < s0 && t <= tlast; ++t) {
+    step(t, Ramp{});
+    if (handed) return true;
+  }
+#pragma unroll 1
+  for (int t = s0; t <= s1; ++t) {
+    step(t, Steady{});
+    if (!STAGED && handed) return true;
+  }
+#pragma unroll 1
+  for (int t = s1 + 1 > s0 ? s1 + 1 : s0; t <= tlast; ++t) {
+    step(t, Ramp{});
+    if (handed) return true;
+  }
+  if (c1 == n - 1) {  // the pencil's last cell, a ghost, against itself
+    const int k = n - 1;
+    if (live) {
+      Cell o = PEm;
+      if (DUAL) {
+        const double own = o.d * o.e;
+        pgas2d_dual(o, (k == 0) ? own : dep, own, P);
+      }
+      if (!isfinite(o.d) || !isfinite(o.e)) nonfin += 1;
+      store(k, o);
+    }
+    if (STAGED) {
+      const int k0 = k - k % kStageCells;
+      flush_stage<DUAL>(a, stage, pid0, k0, k - k0 + 1);
+    }
+  }
+  if (PD > 0) cp_async_wait<0>();
+  if (XT) x_drain(*xt);
+  cnt.nonfinite += nonfin;
+  cnt.dtmin = dtmin;
+  return flagged;
+}
+
+#ifndef PPM_TRANS_MINBLOCKS
+#define PPM_TRANS_MINBLOCKS (2 * 128 / PPM_MARCH_THREADS)
+#endif
+#ifndef PPM_TRANS_X_MINBLOCKS
+#define PPM_TRANS_X_MINBLOCKS (2 * 128 / PPM_MARCH_THREADS)
+#endif
+#ifndef PPM_TRANS_PIPE
+#define PPM_TRANS_PIPE 2
+#endif
+template <bool STAGED>
+__host__ __device__ constexpr int trans_pipe() {
+  return STAGED ? 0 : PPM_TRANS_PIPE;
+}
+constexpr int kTransXBlock = (kMarchThreads / 32) * x_warp_doubles<kTransTiles>();
+template <bool STAGED, bool XT>
+constexpr size_t trans_smem_bytes() {
+  return sizeof(double) * ((XT ? kTransXBlock : 0) + (STAGED ? kStageBlock : 0) +
+                           trans_ring_doubles<trans_pipe<STAGED>()>());
+}
+
+template <bool DUAL, bool GRAV, bool ONE, bool COR, bool STAGED, bool XT>
+__global__ void __launch_bounds__(kMarchThreads,
+                                  STAGED ? PPM_TRANS_X_MINBLOCKS : PPM_TRANS_MINBLOCKS)
+    transport_kernel(const __grid_constant__ BatchArgs B) {
+  static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
+  __shared__ unsigned long long s_cnt[2];
+  __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
+  __shared__ uint64_t s_xbar[XT ? (kMarchThreads / 32) * kXBuffers : 1];
+  extern __shared__ __align__(128) double s_dyn[];
+  double* const s_stage = s_dyn + (XT ? kTransXBlock : 0);
+  if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
+  s_flag[threadIdx.x] = 0;
+  int64_t lb;
+  const int g = locate<ONE>(B.upd_prefix, B.ngrids, lb);
+  PPM_BIND_RECORD(a, g)
+  const int pl = threadIdx.x & ((1 << a.uw_log2) - 1);
+  const int pid = (int)(lb << a.uw_log2) + pl;
+  const int wpid0 = pid - (threadIdx.x & 31);
+  const int c0 = (int)(threadIdx.x >> a.uw_log2) * a.seg_cells;
+  const int c1 = c0 + a.seg_cells - 1 < a.n - 1 ? c0 + a.seg_cells - 1 : a.n - 1;
+  const int warp = threadIdx.x >> 5;
+  XTiles xt;
+  if (XT)
+    x_setup(xt, B, s_dyn + warp * x_warp_doubles<kTransTiles>(), s_xbar + warp * kXBuffers,
+            wpid0,
+            67u | (a.in_u ? 4u : 0u) | (a.in_v ? 8u : 0u) | (a.in_w ? 16u : 0u) |
+                ((DUAL && a.in_ge) ? 32u : 0u));
+  if (ONE) __syncthreads();
+  const bool valid = pid < a.npencils;
+  UpdateCounts cnt = {0, 0, 0, 1.0e20};
+  if ((STAGED || valid) && c0 < a.n) {
+    const Phys P = make_phys(a);
+    if (transport_pencil<DUAL, GRAV, COR, STAGED, trans_pipe<STAGED>(), XT>(
+            a, pid, P, cnt, c0, c1, valid, s_stage + warp * kStageWarp, wpid0,
+            s_dyn + threadIdx.x, &xt))
+      s_flag[pl] = 1;
+  }
+  finish_block(B, a, g, pid, valid && c0 == 0, s_flag, pl, s_cnt, cnt);
 }
 
 // ------------------------------------------------------------------ stage 5 (colours)
@@ -2021,28 +2521,59 @@ void launch_update(const BatchArgs& B, cudaStream_t st) {
     }
   }
   update_kernel<DUAL, GRAV, ONE, STAGED, XT, RS>
-      <<<(unsigned)B.seg_blocks, kMarchThreads, bytes, st>>>(B);
+      <<<(unsigned)B.upd_blocks, kMarchThreads, bytes, st>>>(B);
+}
+
+template <bool DUAL, bool GRAV, bool ONE, bool COR, bool STAGED, bool XT>
+void launch_transport_kernel(const BatchArgs& B, cudaStream_t st) {
+  constexpr size_t bytes = trans_smem_bytes<STAGED, XT>();
+  if (bytes > 48 * 1024) {
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(done.load(std::memory_order_acquire) & bit)) {
+      cudaFuncSetAttribute(transport_kernel<DUAL, GRAV, ONE, COR, STAGED, XT>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      done.fetch_or(bit, std::memory_order_release);
+    }
+  }
+  transport_kernel<DUAL, GRAV, ONE, COR, STAGED, XT>
+      <<<(unsigned)B.upd_blocks, kMarchThreads, bytes, st>>>(B);
+}
+
+template <bool DUAL, bool GRAV, bool ONE, bool COR>
+void launch_transport(const BatchArgs& B, cudaStream_t st, bool staged) {
+  if (PPM_X_TMA && staged && ONE && B.x_tma)
+    launch_transport_kernel<DUAL, GRAV, ONE, COR, true, ONE>(B, st);
+  else if (staged)
+    launch_transport_kernel<DUAL, GRAV, ONE, COR, true, false>(B, st);
+  else
+    launch_transport_kernel<DUAL, GRAV, ONE, COR, false, false>(B, st);
 }
 
 // The two-shock stage with the plain start: the block size and persistence the batch
 // asks for.  riemann_blocks: the launch's grid (the resident blocks when persistent).
-template <bool DUAL, bool ONE, int RT>
+template <bool DUAL, bool ONE, bool STATE, int RT>
 void launch_riemann_rt(const BatchArgs& B, unsigned rb, cudaStream_t st) {
   if (B.persistent)
-    riemann_kernel<DUAL, ONE, false, false, RT, true><<<rb, RT, 0, st>>>(B);
+    riemann_kernel<DUAL, ONE, false, false, RT, true, false, STATE><<<rb, RT, 0, st>>>(B);
   else
-    riemann_kernel<DUAL, ONE, false, false, RT, false><<<rb, RT, 0, st>>>(B);
+    riemann_kernel<DUAL, ONE, false, false, RT, false, false, STATE><<<rb, RT, 0, st>>>(B);
 }
 
-template <bool DUAL, bool ONE>
+template <bool DUAL, bool ONE, bool STATE>
 void launch_riemann_plain(const BatchArgs& B, unsigned rb, cudaStream_t st) {
   if (B.riemann_threads == 64)
-    launch_riemann_rt<DUAL, ONE, 64>(B, rb, st);
+    launch_riemann_rt<DUAL, ONE, STATE, 64>(B, rb, st);
   else if (B.riemann_threads == 256)
-    launch_riemann_rt<DUAL, ONE, 256>(B, rb, st);
+    launch_riemann_rt<DUAL, ONE, STATE, 256>(B, rb, st);
   else
-    launch_riemann_rt<DUAL, ONE, kRiemannThreads>(B, rb, st);
+    launch_riemann_rt<DUAL, ONE, STATE, kRiemannThreads>(B, rb, st);
 }
+
+// The list of flagged pencils starts empty.
+__global__ void clear_flagged_kernel(unsigned long long* counters) { counters[kCntFlagged] = 0ull; }
 
 template <bool DUAL, bool GRAV, bool ONE>
 void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
@@ -2052,6 +2583,41 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
   };
   const unsigned sb = (unsigned)B.seg_blocks;
   mark(0);
+  if (B.transport) {
+    const bool cor = B.corrections || B.uneven;
+    const unsigned rb = (unsigned)riemann_blocks;
+    clear_flagged_kernel<<<1, 1, 0, st>>>(B.counters);
+    if (B.corrections)
+      corrections_kernel<ONE><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
+    if (cor)
+      reconstruct_kernel<DUAL, GRAV, 0, ONE, true><<<sb, kMarchThreads, 0, st>>>(B);
+    else
+      reconstruct_kernel<DUAL, GRAV, 0, ONE><<<sb, kMarchThreads, 0, st>>>(B);
+    mark(1);
+    mark(2);
+    if (learned && B.learned_pass) {
+      launch_guess_pass(B, B.sms, st);
+      riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, true, true>
+          <<<rb, kRiemannThreads, 0, st>>>(B);
+    } else if (learned) {
+      riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, false, true>
+          <<<rb, kRiemannThreads, 0, st>>>(B);
+    } else {
+      launch_riemann_plain<DUAL, ONE, true>(B, rb, st);
+    }
+    mark(3);
+    if (cor)
+      launch_transport<DUAL, GRAV, ONE, true>(B, st, staged);
+    else
+      launch_transport<DUAL, GRAV, ONE, false>(B, st, staged);
+    mark(4);
+    if (cor)
+      fallback_kernel<DUAL, GRAV, ONE, false, true, true><<<64, 128, 0, st>>>(B);
+    else
+      fallback_kernel<DUAL, GRAV, ONE, false, true, false><<<64, 128, 0, st>>>(B);
+    mark(5);
+    return;
+  }
   cudaMemsetAsync(B.counters + kCntFlagged, 0, sizeof(unsigned long long), st);
   if (B.fused) {  // the plain path with the fused face kernel
     face_kernel<DUAL, GRAV, ONE><<<(unsigned)B.face_blocks, kFaceThreads, 0, st>>>(B);
@@ -2099,7 +2665,7 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     hll_riemann_kernel<DUAL, ONE, true, true><<<rb, kRiemannThreads, 0, st>>>(B);
   else if (B.solver == 2)
     hll_riemann_kernel<DUAL, ONE, true, false><<<rb, kRiemannThreads, 0, st>>>(B);
-  else if (learned && B.ncolour > 0)
+  else if (learned && col)
     riemann_kernel<DUAL, ONE, true, true><<<rb, kRiemannThreads, 0, st>>>(B);
   else if (learned && B.learned_pass) {
     launch_guess_pass(B, B.sms, st);
@@ -2107,10 +2673,10 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
         <<<rb, kRiemannThreads, 0, st>>>(B);
   } else if (learned)
     riemann_kernel<DUAL, ONE, true><<<rb, kRiemannThreads, 0, st>>>(B);
-  else if (B.ncolour > 0)
+  else if (col)
     riemann_kernel<DUAL, ONE, false, true><<<rb, kRiemannThreads, 0, st>>>(B);
   else
-    launch_riemann_plain<DUAL, ONE>(B, rb, st);
+    launch_riemann_plain<DUAL, ONE, false>(B, rb, st);
   mark(3);
   if (B.solver != 0) {  // HLL / HLLC
     if (PPM_X_TMA && staged && ONE && B.x_tma)
@@ -2172,21 +2738,21 @@ int riemann_resident_blocks(bool dual, bool one, int threads) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, rt, 0);
   };
   if (threads == 64) {
-    if (dual) one ? occ(split::riemann_kernel<true, true, false, false, 64, true>, 64)
-              : occ(split::riemann_kernel<true, false, false, false, 64, true>, 64);
-    else one ? occ(split::riemann_kernel<false, true, false, false, 64, true>, 64)
-             : occ(split::riemann_kernel<false, false, false, false, 64, true>, 64);
+    if (dual) one ? occ(split::riemann_kernel<true, true, false, false, 64, true, false, true>, 64)
+              : occ(split::riemann_kernel<true, false, false, false, 64, true, false, true>, 64);
+    else one ? occ(split::riemann_kernel<false, true, false, false, 64, true, false, true>, 64)
+             : occ(split::riemann_kernel<false, false, false, false, 64, true, false, true>, 64);
   } else if (threads == 256) {
-    if (dual) one ? occ(split::riemann_kernel<true, true, false, false, 256, true>, 256)
-              : occ(split::riemann_kernel<true, false, false, false, 256, true>, 256);
-    else one ? occ(split::riemann_kernel<false, true, false, false, 256, true>, 256)
-             : occ(split::riemann_kernel<false, false, false, false, 256, true>, 256);
+    if (dual) one ? occ(split::riemann_kernel<true, true, false, false, 256, true, false, true>, 256)
+              : occ(split::riemann_kernel<true, false, false, false, 256, true, false, true>, 256);
+    else one ? occ(split::riemann_kernel<false, true, false, false, 256, true, false, true>, 256)
+             : occ(split::riemann_kernel<false, false, false, false, 256, true, false, true>, 256);
   } else {
     constexpr int rt = kRiemannThreads;
-    if (dual) one ? occ(split::riemann_kernel<true, true, false, false, rt, true>, rt)
-              : occ(split::riemann_kernel<true, false, false, false, rt, true>, rt);
-    else one ? occ(split::riemann_kernel<false, true, false, false, rt, true>, rt)
-             : occ(split::riemann_kernel<false, false, false, false, rt, true>, rt);
+    if (dual) one ? occ(split::riemann_kernel<true, true, false, false, rt, true, false, true>, rt)
+              : occ(split::riemann_kernel<true, false, false, false, rt, true, false, true>, rt);
+    else one ? occ(split::riemann_kernel<false, true, false, false, rt, true, false, true>, rt)
+             : occ(split::riemann_kernel<false, false, false, false, rt, true, false, true>, rt);
   }
   return n > 0 ? n : 1;
 }

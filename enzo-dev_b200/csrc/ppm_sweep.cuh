@@ -138,8 +138,9 @@ struct SweepArgs {
   double eos_cs;
   // split of the marching stages (set_segments): a block of kMarchThreads threads takes
   // 2^pw_log2 pencils, each cut into kMarchThreads >> pw_log2 segments of seg_faces faces
-  // (reconstruction) or seg_cells cells (update)
-  int pw_log2, seg_faces, seg_cells;
+  // (reconstruction); uw_log2 and seg_cells the same for the update and transport kernels,
+  // whose segments are of cells
+  int pw_log2, seg_faces, uw_log2, seg_cells;
   // one cell width along the sweep (uniform): the coefficients every cell shares
   int uniform;
   Coef uc;
@@ -168,7 +169,8 @@ enum { kMarchThreads = PPM_MARCH_THREADS, kRiemannThreads = PPM_RIEMANN_THREADS 
 // One launch over a batch of grids (an AMR level, or a single grid).  Every block
 // belongs to one grid: grid g owns blocks [prefix[g], prefix[g+1]) of a stage; a
 // block finds its grid by binary search over the prefix table.
-//   reconstruction, update: ceil(npencils / 2^pw_log2) blocks per grid
+//   reconstruction: ceil(npencils / 2^pw_log2) blocks per grid
+//   update, transport: ceil(npencils / 2^uw_log2) blocks per grid
 //   corrections, colours: ceil(npencils / kMarchThreads) blocks per grid
 //   Riemann stage:   (ie - is + 2) * ceil(npencils / kRiemannThreads) blocks per grid
 struct BatchArgs {
@@ -177,8 +179,11 @@ struct BatchArgs {
   const SweepArgs* grids;            // device array, ngrids records
   int ngrids;
   const int64_t* march_prefix;       // ngrids + 1
-  const int64_t* seg_prefix;         // ngrids + 1
+  const int64_t* seg_prefix;         // ngrids + 1 (reconstruction)
   int64_t seg_blocks = 0;
+  const int64_t* upd_prefix;         // ngrids + 1 (update, transport)
+  int64_t upd_blocks = 0;
+  int transport = 0;                 // the transport path (see transport_kernel)
   const int64_t* riemann_prefix;     // ngrids + 1
   unsigned long long* counters;      // kCounterCopies x kMaxCounters, shared by the batch
   int64_t* flagged;                  // pencils needing the fallback pass: (grid << 40) | pencil
@@ -215,7 +220,7 @@ struct BatchArgs {
   // interface states before the Riemann kernel, instead of inside it
   int learned_pass = 0;
   int sms = 148;
-  CUtensorMap xin[6];
+  CUtensorMap xin[7];                // d, e, u, v, w, ge, pressure
 };
 
 // The fused face kernel: a warp takes one pencil and kFaceSeg consecutive faces, lane
@@ -287,25 +292,48 @@ inline void build_coef(const double* dxi_in, int n, int is0, int ie0, std::vecto
 #ifndef PPM_SEG_MIN
 #define PPM_SEG_MIN 4
 #endif
-inline int64_t march_segment_blocks(const SweepArgs& a) {
-  return (a.npencils + (int64_t(1) << a.pw_log2) - 1) >> a.pw_log2;
+// The transport path (transport_kernel) holds half the resident threads of the kernels it
+// replaces, so it pays where a batch fills the chip all the same.  Whole step, the two
+// kernels -> transport (us): exact 80^3 622 -> 700, 96^3 979 -> 949, 128^3 1879 -> 1650,
+// 900x900 690 -> 680, levels of 0.53 M cells 604 -> 657, of 1.5 M 1295 -> 1240; tolerance
+// 64^3 283 -> 328, 80^3 403 -> 430, 900x900 (0.82 M cells) 573 -> 451, 96^3 673 -> 540.
+#ifndef PPM_TRANSPORT_CELLS
+#define PPM_TRANSPORT_CELLS 750000
+#endif
+inline bool use_transport(int64_t batch_cells) { return batch_cells >= PPM_TRANSPORT_CELLS; }
+// The transport kernel's resident threads: two blocks of 128 an SM.
+#ifndef PPM_TRANS_FILL
+#define PPM_TRANS_FILL (148 * 2 * 128)
+#endif
+inline int64_t segment_blocks(const SweepArgs& a, int log_w) {
+  return (a.npencils + (int64_t(1) << log_w) - 1) >> log_w;
 }
 // a: a record with its geometry; batch_pencils: pencils of all grids of the launch.
 // local_select: pgas2d_dual's energy of a cell may be formed without its left neighbour
 // (see update_pencil); without it the update needs whole pencils.
-inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select) {
-  int log_w = 0;
-  while ((1 << log_w) < kMarchThreads) ++log_w;
+inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select,
+                         bool transport) {
+  int whole = 0;
+  while ((1 << whole) < kMarchThreads) ++whole;
   const int faces = a.ie - a.is + 2;
-  int segs = 1;
-  if (local_select)
-    while (segs < kMarchThreads && batch_pencils * segs < PPM_MARCH_FILL &&
+  auto split = [&](int64_t fill, int& log_w) {
+    int segs = 1;
+    log_w = whole;
+    while (segs < kMarchThreads && batch_pencils * segs < fill &&
            faces / (2 * segs) >= PPM_SEG_MIN) {
       segs *= 2;
       --log_w;
     }
-  a.pw_log2 = log_w;
+    return segs;
+  };
+  int segs = split(PPM_MARCH_FILL, a.pw_log2);
   a.seg_faces = (faces + segs - 1) / segs;
+  if (local_select) {
+    segs = split(transport ? PPM_TRANS_FILL : PPM_MARCH_FILL, a.uw_log2);
+  } else {
+    segs = 1;
+    a.uw_log2 = whole;
+  }
   // whole output chunks of the x sweep's staged stores
   const int cells = (a.n + segs - 1) / segs;
   a.seg_cells = (cells + 3) / 4 * 4;
