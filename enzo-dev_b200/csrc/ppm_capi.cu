@@ -59,7 +59,6 @@ struct ElemBatch {
   double eos_cs;
 };
 void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st);
-void launch_cfl_reset(unsigned long long* min_bits, cudaStream_t st);
 void launch_cfl_finalize(const unsigned long long* min_bits, double courant, double* dt_out,
                          cudaStream_t st);
 void launch_sweep_batch(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
@@ -644,10 +643,12 @@ int solver_code(const ppm_b200_params* p) {
          : p->riemann_solver == PPM_B200_RIEMANN_HLLC ? 2 : 0;
 }
 
-// kernels one sweep launches: reconstruct x2, Riemann, update, fallback, and the
-// corrections and colour kernels when present
-int sweep_kernels(const ppm_b200_params* p) {
-  return 5 + (correction_planes(p) > 0 ? 1 : 0) + (p->number_of_colours > 0 ? 1 : 0);
+// kernels one sweep launches: reconstruct x2 (or the clearing kernel and both in one),
+// Riemann, update, fallback; on the transport path reconstruct, Riemann, transport,
+// fallback; and the corrections and colour kernels when present
+int sweep_kernels(const ppm_b200_params* p, const BatchArgs& B) {
+  return (B.transport ? 4 : 5) + (correction_planes(p) > 0 ? 1 : 0) +
+         (p->number_of_colours > 0 ? 1 : 0);
 }
 
 size_t sweep_scratch_bytes(int dim, const std::vector<GridIO>& io, const ppm_b200_params* p) {
@@ -930,6 +931,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.upd_prefix = (const int64_t*)(base + off_u);
   plan.B.upd_blocks = upre[ng];
   plan.B.transport = transport ? 1 : 0;
+  plan.B.both_roles = ppm::use_both_roles(gpre[ng], transport) ? 1 : 0;
   plan.B.counters = (unsigned long long*)ctx->counters.p;
   plan.B.flagged = (int64_t*)(scratch + scratch_doubles);
   plan.march_blocks = mpre[ng];
@@ -950,8 +952,9 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   return PPM_B200_OK;
 }
 
+// clear_bits: the folded time step's minimum, reset before this sweep (null: not here)
 int enqueue_sweep(ppm_b200_context* ctx, const SweepPlan& plan, const ppm_b200_params* p,
-                  bool capturing) {
+                  bool capturing, unsigned long long* clear_bits = nullptr) {
   cudaEvent_t* ev = nullptr;
   if (ctx->profiling && !capturing) {
     while (ctx->ev_pool.size() < ctx->ev_used + kSweepEvents) {
@@ -962,10 +965,12 @@ int enqueue_sweep(ppm_b200_context* ctx, const SweepPlan& plan, const ppm_b200_p
     ev = &ctx->ev_pool[ctx->ev_used];
     ctx->ev_used += kSweepEvents;
   }
-  ppm::launch_sweep_batch(plan.B, plan.march_blocks, plan.riemann_blocks, p->dual_energy != 0,
+  BatchArgs B = plan.B;
+  B.clear_bits = clear_bits;
+  ppm::launch_sweep_batch(B, plan.march_blocks, plan.riemann_blocks, p->dual_energy != 0,
                           p->gravity != 0, ctx->stream, ev, p->learned_guess != 0,
                           plan.contiguous);
-  ctx->launches += sweep_kernels(p);
+  ctx->launches += sweep_kernels(p, B);
   CK(cudaGetLastError());
   return PPM_B200_OK;
 }
@@ -1326,8 +1331,7 @@ int enqueue_solve(ppm_b200_context* ctx, const ppm_b200_params* p, const std::ve
   unsigned long long* cfl_bits = ((unsigned long long*)ctx->misc.p) + 2;
   for (int s = 0; s < sp.nsweeps; ++s) {
     const bool cfl = ctx->cfl_dt != nullptr && s == sp.nsweeps - 1;
-    if (cfl && cfl_first) ppm::launch_cfl_reset(cfl_bits, ctx->stream);
-    int rc = enqueue_sweep(ctx, sp.sweep[s], p, capturing);
+    int rc = enqueue_sweep(ctx, sp.sweep[s], p, capturing, cfl && cfl_first ? cfl_bits : nullptr);
     if (rc) return rc;
     if (cfl && cfl_last) {
       ppm::launch_cfl_finalize(cfl_bits, ctx->cfl_courant, ctx->cfl_dt, ctx->stream);
@@ -1512,6 +1516,7 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, b.upd_prefix);
     key_put(k, b.upd_blocks);
     key_put(k, b.transport);
+    key_put(k, b.both_roles);
     key_put(k, b.counters);
     key_put(k, b.flagged);
     key_put(k, sp.sweep[s].march_blocks);
@@ -1996,8 +2001,10 @@ int ppm_b200_solve_level(ppm_b200_context* ctx, const ppm_b200_params* p, int cy
       it = ctx->graphs.emplace(key, ex).first;
     }
     CK(cudaGraphLaunch(it->second, ctx->stream));
-    for (const auto& sp : plans)
-      ctx->launches += 1 + sweep_kernels(p) * sp.nsweeps + (p->eos_type > 0 ? 1 : 0);
+    for (const auto& sp : plans) {
+      ctx->launches += 1 + (p->eos_type > 0 ? 1 : 0);
+      for (int s = 0; s < sp.nsweeps; ++s) ctx->launches += sweep_kernels(p, sp.sweep[s].B);
+    }
     if (ctx->cfl_dt) ctx->launches += 1;  // the folded time step's finalize kernel
   } else {
     rc = enqueue_all(false);

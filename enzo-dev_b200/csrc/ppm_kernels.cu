@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "ppm_device.cuh"
+#include "ppm_launch.cuh"
 #include "ppm_sweep.cuh"
 
 namespace ppm {
@@ -92,6 +93,7 @@ __device__ __forceinline__ double eos_pressure(const ElemGrid& G, int64_t i, con
 }
 
 __global__ void __launch_bounds__(256) pressure_kernel(const __grid_constant__ ElemBatch B) {
+  pdl_begin();
   int64_t lb;
   const ElemGrid& G = B.grids[batch_locate(B.size_prefix, B.ngrids, blockIdx.x, lb)];
   const int64_t i = lb * 256 + threadIdx.x;
@@ -102,6 +104,7 @@ __global__ void __launch_bounds__(256) pressure_kernel(const __grid_constant__ E
 
 // calc_dt (ihydro = 0) over the active cells of every grid; min over the batch
 __global__ void __launch_bounds__(256) timestep_kernel(const __grid_constant__ ElemBatch B) {
+  pdl_begin();
   int64_t lb;
   const ElemGrid& G = B.grids[batch_locate(B.active_prefix, B.ngrids, blockIdx.x, lb)];
   const int64_t c = lb * 256 + threadIdx.x;
@@ -150,6 +153,7 @@ __global__ void __launch_bounds__(256) timestep_kernel(const __grid_constant__ E
 // min_bits starts as all ones (set by a memset); every block has folded in a value <= huge.
 __global__ void timestep_finalize_kernel(const unsigned long long* min_bits, double courant,
                                          double* dt_out) {
+  pdl_begin();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const unsigned long long b = *min_bits;
     double dt = (b == ~0ull) ? 1.0e20 : __longlong_as_double((long long)b);
@@ -187,6 +191,7 @@ __device__ __forceinline__ void copy_cell(double* const (&f)[6], int64_t dst, in
 // warps each) stride over its rows, about four per warp, so that the block-to-grid search
 // and the record's fields are amortised over several rows.
 __global__ void __launch_bounds__(256) boundary_kernel(const __grid_constant__ ElemBatch B) {
+  pdl_begin();
   int64_t lb;
   const int gi = batch_locate(B.row_prefix, B.ngrids, blockIdx.x, lb);
   const ElemGrid& G = B.grids[gi];
@@ -445,6 +450,7 @@ __device__ __forceinline__ double cell_pressure_interp(const ElemGrid& G, int64_
 }
 
 __global__ void __launch_bounds__(256) expansion_kernel(const __grid_constant__ ElemBatch B) {
+  pdl_begin();
   int64_t lb;
   const ElemGrid& G = B.grids[batch_locate(B.size_prefix, B.ngrids, blockIdx.x, lb)];
   const int64_t i = lb * 256 + threadIdx.x;
@@ -470,32 +476,29 @@ __global__ void __launch_bounds__(256) expansion_kernel(const __grid_constant__ 
 
 // ------------------------------------------------------------------ launchers
 void launch_pressure_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  pressure_kernel<<<(unsigned)blocks, 256, 0, st>>>(B);
+  launch_chain(pressure_kernel, blocks, 256, 0, st, B);
 }
 
 void launch_timestep_batch(const ElemBatch& B, int64_t blocks, double courant, double* dt_out,
                            cudaStream_t st) {
   cudaMemsetAsync(B.min_bits, 0xFF, sizeof(unsigned long long), st);
-  timestep_kernel<<<(unsigned)blocks, 256, 0, st>>>(B);
-  timestep_finalize_kernel<<<1, 32, 0, st>>>(B.min_bits, courant, dt_out);
+  launch_chain(timestep_kernel, blocks, 256, 0, st, B);
+  const unsigned long long* bits = B.min_bits;
+  launch_chain(timestep_finalize_kernel, 1, 32, 0, st, bits, courant, dt_out);
 }
 
-// The time step folded into a solve's last sweep: reset before it, finalise after it.
-void launch_cfl_reset(unsigned long long* min_bits, cudaStream_t st) {
-  cudaMemsetAsync(min_bits, 0xFF, sizeof(unsigned long long), st);
-}
-
+// The time step folded into a solve's last sweep (reset in that sweep's first kernel).
 void launch_cfl_finalize(const unsigned long long* min_bits, double courant, double* dt_out,
                          cudaStream_t st) {
-  timestep_finalize_kernel<<<1, 32, 0, st>>>(min_bits, courant, dt_out);
+  launch_chain(timestep_finalize_kernel, 1, 32, 0, st, min_bits, courant, dt_out);
 }
 
 void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  expansion_kernel<<<(unsigned)blocks, 256, 0, st>>>(B);
+  launch_chain(expansion_kernel, blocks, 256, 0, st, B);
 }
 
 void launch_boundary_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  boundary_kernel<<<(unsigned)blocks, 256, 0, st>>>(B);
+  launch_chain(boundary_kernel, blocks, 256, 0, st, B);
 }
 
 }  // namespace ppm

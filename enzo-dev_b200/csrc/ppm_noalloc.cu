@@ -279,6 +279,7 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   B.upd_prefix = reinterpret_cast<const int64_t*>(desc + 960);
   B.upd_blocks = upd_blocks;
   B.transport = transport ? 1 : 0;
+  B.both_roles = ppm::use_both_roles(seg_blocks, transport) ? 1 : 0;
   B.uneven = a.uniform ? 0 : 1;
   B.counters = counters;
   B.flagged = reinterpret_cast<int64_t*>(planes + (size_t)(ppm::kFaceVars + ppm::kFluxVars) *

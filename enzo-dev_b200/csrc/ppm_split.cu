@@ -23,6 +23,7 @@
 
 #include "ppm_device.cuh"
 #include "ppm_guess.cuh"
+#include "ppm_launch.cuh"
 #include "ppm_sweep.cuh"
 
 namespace ppm {
@@ -133,6 +134,7 @@ __device__ __forceinline__ void load_face_advected(const SweepArgs& a, int64_t i
 // flattemp values are computed once each and kept for the max of eq. A2.
 template <bool ONE>
 __global__ void __launch_bounds__(kMarchThreads) corrections_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   int64_t lb;
   const int g = locate<ONE>(B.march_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
@@ -452,12 +454,34 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int pid, 
     step(t, Ramp{});
 }
 
+// This thread's segment of block lb of a grid.
+template <bool DUAL, bool GRAV, int ROLE, bool COR>
+__device__ __forceinline__ void reconstruct_segment(const SweepArgs& a, int64_t lb) {
+  const int pid = (int)(lb << a.pw_log2) + (threadIdx.x & ((1 << a.pw_log2) - 1));
+  const int f0 = a.is + (int)(threadIdx.x >> a.pw_log2) * a.seg_faces;
+  if (pid >= a.npencils || f0 > a.ie + 1) return;
+  const int f1 = f0 + a.seg_faces - 1;
+  reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, pid, f0, f1 < a.ie + 1 ? f1 : a.ie + 1);
+}
+
+// What a sweep starts from, by one thread before its update kernel is launched: an empty
+// list of flagged pencils and, where the batch asks for it, no folded time step yet.
+__device__ __forceinline__ void clear_sweep(const BatchArgs& B) {
+  B.counters[kCntFlagged] = 0ull;
+  if (B.clear_bits) *B.clear_bits = ~0ull;
+}
+__global__ void clear_sweep_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
+  clear_sweep(B);
+}
+
 // FLAG: only the pencils of the batch's flagged list (the fused sweep's fallback pass,
 // which needs the interface states of those pencils): a fixed grid walks the list.
 template <bool DUAL, bool GRAV, int ROLE, bool ONE, bool COR = false, bool FLAG = false>
 __global__ void __launch_bounds__(kMarchThreads,
                                   ROLE == 0 ? PPM_RECON0_MINBLOCKS : PPM_RECON_MINBLOCKS)
     reconstruct_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   if (FLAG) {
     const unsigned long long nflag = *(volatile unsigned long long*)&B.counters[kCntFlagged];
     for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -469,14 +493,29 @@ __global__ void __launch_bounds__(kMarchThreads,
     }
     return;
   }
+  if (ROLE == 0 && blockIdx.x == 0 && threadIdx.x == 0) clear_sweep(B);
   int64_t lb;
   const int g = locate<ONE>(B.seg_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
-  const int pid = (int)(lb << a.pw_log2) + (threadIdx.x & ((1 << a.pw_log2) - 1));
-  const int f0 = a.is + (int)(threadIdx.x >> a.pw_log2) * a.seg_faces;
-  if (pid >= a.npencils || f0 > a.ie + 1) return;
-  const int f1 = f0 + a.seg_faces - 1;
-  reconstruct_pencil<DUAL, GRAV, ROLE, COR>(a, pid, f0, f1 < a.ie + 1 ? f1 : a.ie + 1);
+  reconstruct_segment<DUAL, GRAV, ROLE, COR>(a, lb);
+}
+
+// Both roles in one launch, role 0 in the first half of the blocks: for batches whose
+// blocks are all resident together, which then pay one launch and the longer of the two
+// marches instead of their sum.
+template <bool DUAL, bool GRAV, bool ONE, bool COR>
+__global__ void __launch_bounds__(kMarchThreads, PPM_RECON_MINBLOCKS)
+    reconstruct_both_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
+  const bool first = blockIdx.x < B.seg_blocks;
+  const int64_t blk = blockIdx.x - (first ? 0 : B.seg_blocks);
+  int64_t lb = blk;
+  const int g = ONE ? 0 : batch_locate(B.seg_prefix, B.ngrids, blk, lb);
+  PPM_BIND_RECORD(a, g)
+  if (first)
+    reconstruct_segment<DUAL, GRAV, 0, COR>(a, lb);
+  else
+    reconstruct_segment<DUAL, GRAV, 1, COR>(a, lb);
 }
 
 // ------------------------------------------------------------------ stage 2
@@ -511,6 +550,7 @@ template <bool DUAL, bool ONE, bool LEARNED, bool COL = false, int RT = kRiemann
 __global__ void __launch_bounds__(RT, (LEARNED ? PPM_RIEMANN_LEARNED_MINBLOCKS
                                                : PPM_RIEMANN_MINBLOCKS) * kRiemannThreads / RT)
     riemann_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   __shared__ unsigned int s_hist[8];
   __shared__ unsigned int s_newton;
   __shared__ unsigned int s_rejected;
@@ -697,6 +737,7 @@ __device__ __forceinline__ void face_parabolas(const double q[3], const double q
 template <bool DUAL, bool GRAV, bool ONE>
 __global__ void __launch_bounds__(kFaceThreads, PPM_FACE_MINBLOCKS)
     face_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   __shared__ unsigned int s_hist[8];
   __shared__ unsigned int s_newton, s_wtrips, s_warps;
   if (threadIdx.x < 8) s_hist[threadIdx.x] = 0u;
@@ -900,6 +941,7 @@ __global__ void __launch_bounds__(kFaceThreads, PPM_FACE_MINBLOCKS)
 // (twoshock.F:124-130).  COL: the Godunov density for the colour kernel.
 template <bool DUAL, bool ONE, bool COL>
 __global__ void __launch_bounds__(kRiemannThreads) presfree_riemann_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   int64_t lb;
   const int g = locate<ONE>(B.riemann_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
@@ -950,6 +992,7 @@ __device__ __forceinline__ HllFace hll_any(const FaceState& s, const Phys& P) {
 template <bool DUAL, bool ONE, bool HLLC, bool COL>
 __global__ void __launch_bounds__(kRiemannThreads, PPM_HLL_MINBLOCKS)
     hll_riemann_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   int64_t lb;
   const int g = locate<ONE>(B.riemann_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
@@ -1789,6 +1832,7 @@ __global__ void __launch_bounds__(kMarchThreads,
                                          : (ONE ? PPM_UPDATE_YZ_MINBLOCKS
                                                 : PPM_UPDATE_YZ_BATCH_MINBLOCKS))
     update_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
   __shared__ unsigned long long s_cnt[2];
   __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
@@ -1857,6 +1901,7 @@ __device__ __noinline__ void fill_pencil(const SweepArgs& a, int pid) {
 // transport kernel.
 template <bool DUAL, bool GRAV, bool ONE, bool RS = false, bool TRANS = false, bool COR = false>
 __global__ void __launch_bounds__(128) fallback_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   const unsigned long long nflag = *(volatile unsigned long long*)&B.counters[kCntFlagged];
   for (unsigned long long k = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
        k < nflag; k += (unsigned long long)gridDim.x * blockDim.x) {
@@ -2274,6 +2319,7 @@ template <bool DUAL, bool GRAV, bool ONE, bool COR, bool STAGED, bool XT>
 __global__ void __launch_bounds__(kMarchThreads,
                                   STAGED ? PPM_TRANS_X_MINBLOCKS : PPM_TRANS_MINBLOCKS)
     transport_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
   __shared__ unsigned long long s_cnt[2];
   __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
@@ -2344,6 +2390,7 @@ constexpr double kMinColour = 1.0e-5 * kTiny;   // min_color, euler.F:104-105
 template <bool DUAL, bool ONE, int CPT>
 __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
     colour_kernel(const __grid_constant__ BatchArgs B) {
+  pdl_begin();
   const int nc = B.ncolour;
   const int nchunk = (nc + CPT - 1) / CPT;
   const int64_t mb = blockIdx.x / nchunk;
@@ -2520,8 +2567,8 @@ void launch_update(const BatchArgs& B, cudaStream_t st) {
       done.fetch_or(bit, std::memory_order_release);
     }
   }
-  update_kernel<DUAL, GRAV, ONE, STAGED, XT, RS>
-      <<<(unsigned)B.upd_blocks, kMarchThreads, bytes, st>>>(B);
+  launch_chain(update_kernel<DUAL, GRAV, ONE, STAGED, XT, RS>,
+               B.upd_blocks, kMarchThreads, bytes, st, B);
 }
 
 template <bool DUAL, bool GRAV, bool ONE, bool COR, bool STAGED, bool XT>
@@ -2538,8 +2585,8 @@ void launch_transport_kernel(const BatchArgs& B, cudaStream_t st) {
       done.fetch_or(bit, std::memory_order_release);
     }
   }
-  transport_kernel<DUAL, GRAV, ONE, COR, STAGED, XT>
-      <<<(unsigned)B.upd_blocks, kMarchThreads, bytes, st>>>(B);
+  launch_chain(transport_kernel<DUAL, GRAV, ONE, COR, STAGED, XT>,
+               B.upd_blocks, kMarchThreads, bytes, st, B);
 }
 
 template <bool DUAL, bool GRAV, bool ONE, bool COR>
@@ -2557,9 +2604,11 @@ void launch_transport(const BatchArgs& B, cudaStream_t st, bool staged) {
 template <bool DUAL, bool ONE, bool STATE, int RT>
 void launch_riemann_rt(const BatchArgs& B, unsigned rb, cudaStream_t st) {
   if (B.persistent)
-    riemann_kernel<DUAL, ONE, false, false, RT, true, false, STATE><<<rb, RT, 0, st>>>(B);
+    launch_chain(riemann_kernel<DUAL, ONE, false, false, RT, true, false, STATE>,
+                 rb, RT, 0, st, B);
   else
-    riemann_kernel<DUAL, ONE, false, false, RT, false, false, STATE><<<rb, RT, 0, st>>>(B);
+    launch_chain(riemann_kernel<DUAL, ONE, false, false, RT, false, false, STATE>,
+                 rb, RT, 0, st, B);
 }
 
 template <bool DUAL, bool ONE, bool STATE>
@@ -2572,9 +2621,6 @@ void launch_riemann_plain(const BatchArgs& B, unsigned rb, cudaStream_t st) {
     launch_riemann_rt<DUAL, ONE, STATE, kRiemannThreads>(B, rb, st);
 }
 
-// The list of flagged pencils starts empty.
-__global__ void clear_flagged_kernel(unsigned long long* counters) { counters[kCntFlagged] = 0ull; }
-
 template <bool DUAL, bool GRAV, bool ONE>
 void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
                    cudaStream_t st, cudaEvent_t* ev, bool learned, bool staged) {
@@ -2586,22 +2632,21 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
   if (B.transport) {
     const bool cor = B.corrections || B.uneven;
     const unsigned rb = (unsigned)riemann_blocks;
-    clear_flagged_kernel<<<1, 1, 0, st>>>(B.counters);
     if (B.corrections)
-      corrections_kernel<ONE><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
+      launch_chain(corrections_kernel<ONE>, march_blocks, kMarchThreads, 0, st, B);
     if (cor)
-      reconstruct_kernel<DUAL, GRAV, 0, ONE, true><<<sb, kMarchThreads, 0, st>>>(B);
+      launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads, 0, st, B);
     else
-      reconstruct_kernel<DUAL, GRAV, 0, ONE><<<sb, kMarchThreads, 0, st>>>(B);
+      launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE>, sb, kMarchThreads, 0, st, B);
     mark(1);
     mark(2);
     if (learned && B.learned_pass) {
       launch_guess_pass(B, B.sms, st);
-      riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, true, true>
-          <<<rb, kRiemannThreads, 0, st>>>(B);
+      launch_chain(riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, true, true>,
+                   rb, kRiemannThreads, 0, st, B);
     } else if (learned) {
-      riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, false, true>
-          <<<rb, kRiemannThreads, 0, st>>>(B);
+      launch_chain(riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, false, true>,
+                   rb, kRiemannThreads, 0, st, B);
     } else {
       launch_riemann_plain<DUAL, ONE, true>(B, rb, st);
     }
@@ -2612,15 +2657,16 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
       launch_transport<DUAL, GRAV, ONE, false>(B, st, staged);
     mark(4);
     if (cor)
-      fallback_kernel<DUAL, GRAV, ONE, false, true, true><<<64, 128, 0, st>>>(B);
+      launch_chain(fallback_kernel<DUAL, GRAV, ONE, false, true, true>, 64, 128, 0, st, B);
     else
-      fallback_kernel<DUAL, GRAV, ONE, false, true, false><<<64, 128, 0, st>>>(B);
+      launch_chain(fallback_kernel<DUAL, GRAV, ONE, false, true, false>, 64, 128, 0, st, B);
     mark(5);
     return;
   }
-  cudaMemsetAsync(B.counters + kCntFlagged, 0, sizeof(unsigned long long), st);
   if (B.fused) {  // the plain path with the fused face kernel
-    face_kernel<DUAL, GRAV, ONE><<<(unsigned)B.face_blocks, kFaceThreads, 0, st>>>(B);
+    cudaMemsetAsync(B.counters + kCntFlagged, 0, sizeof(unsigned long long), st);
+    if (B.clear_bits) cudaMemsetAsync(B.clear_bits, 0xFF, sizeof(unsigned long long), st);
+    launch_chain(face_kernel<DUAL, GRAV, ONE>, B.face_blocks, kFaceThreads, 0, st, B);
     mark(1);
     mark(2);
     mark(3);
@@ -2632,49 +2678,60 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
       launch_update<DUAL, GRAV, ONE, false, false>(B, st);
     mark(4);
     // the flagged pencils' interface states, then their per-cell HLL fallback
-    reconstruct_kernel<DUAL, GRAV, 0, ONE, false, true><<<64, kMarchThreads, 0, st>>>(B);
-    reconstruct_kernel<DUAL, GRAV, 1, ONE, false, true><<<64, kMarchThreads, 0, st>>>(B);
-    fallback_kernel<DUAL, GRAV, ONE><<<64, 128, 0, st>>>(B);
+    launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE, false, true>,
+                 64, kMarchThreads, 0, st, B);
+    launch_chain(reconstruct_kernel<DUAL, GRAV, 1, ONE, false, true>,
+                 64, kMarchThreads, 0, st, B);
+    launch_chain(fallback_kernel<DUAL, GRAV, ONE>, 64, 128, 0, st, B);
     mark(5);
     return;
   }
   if (B.ncolour > 0) cudaMemsetAsync(B.hll_flags, 0, (size_t)B.hll_bytes, st);
-  if (B.corrections || B.ncolour > 0 || B.presfree || B.uneven) {  // not the plain path: COR
-    if (B.corrections)
-      corrections_kernel<ONE><<<(unsigned)march_blocks, kMarchThreads, 0, st>>>(B);
-    reconstruct_kernel<DUAL, GRAV, 0, ONE, true><<<sb, kMarchThreads, 0, st>>>(B);
+  const bool cor = B.corrections || B.ncolour > 0 || B.presfree || B.uneven;
+  if (B.corrections) launch_chain(corrections_kernel<ONE>, march_blocks, kMarchThreads, 0, st, B);
+  if (B.both_roles) {
+    launch_chain(clear_sweep_kernel, 1, 1, 0, st, B);
     mark(1);
-    reconstruct_kernel<DUAL, GRAV, 1, ONE, true><<<sb, kMarchThreads, 0, st>>>(B);
+    if (cor)
+      launch_chain(reconstruct_both_kernel<DUAL, GRAV, ONE, true>, 2 * B.seg_blocks,
+                   kMarchThreads, 0, st, B);
+    else
+      launch_chain(reconstruct_both_kernel<DUAL, GRAV, ONE, false>, 2 * B.seg_blocks,
+                   kMarchThreads, 0, st, B);
+  } else if (cor) {
+    launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads, 0, st, B);
+    mark(1);
+    launch_chain(reconstruct_kernel<DUAL, GRAV, 1, ONE, true>, sb, kMarchThreads, 0, st, B);
   } else {
-    reconstruct_kernel<DUAL, GRAV, 0, ONE><<<sb, kMarchThreads, 0, st>>>(B);
+    launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE>, sb, kMarchThreads, 0, st, B);
     mark(1);
-    reconstruct_kernel<DUAL, GRAV, 1, ONE><<<sb, kMarchThreads, 0, st>>>(B);
+    launch_chain(reconstruct_kernel<DUAL, GRAV, 1, ONE>, sb, kMarchThreads, 0, st, B);
   }
   mark(2);
   const unsigned rb = (unsigned)riemann_blocks;
   const bool col = B.ncolour > 0;
   if (B.solver == 0 && B.presfree && col)
-    presfree_riemann_kernel<DUAL, ONE, true><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(presfree_riemann_kernel<DUAL, ONE, true>, rb, kRiemannThreads, 0, st, B);
   else if (B.solver == 0 && B.presfree)
-    presfree_riemann_kernel<DUAL, ONE, false><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(presfree_riemann_kernel<DUAL, ONE, false>, rb, kRiemannThreads, 0, st, B);
   else if (B.solver == 1 && col)
-    hll_riemann_kernel<DUAL, ONE, false, true><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(hll_riemann_kernel<DUAL, ONE, false, true>, rb, kRiemannThreads, 0, st, B);
   else if (B.solver == 1)
-    hll_riemann_kernel<DUAL, ONE, false, false><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(hll_riemann_kernel<DUAL, ONE, false, false>, rb, kRiemannThreads, 0, st, B);
   else if (B.solver == 2 && col)
-    hll_riemann_kernel<DUAL, ONE, true, true><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(hll_riemann_kernel<DUAL, ONE, true, true>, rb, kRiemannThreads, 0, st, B);
   else if (B.solver == 2)
-    hll_riemann_kernel<DUAL, ONE, true, false><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(hll_riemann_kernel<DUAL, ONE, true, false>, rb, kRiemannThreads, 0, st, B);
   else if (learned && col)
-    riemann_kernel<DUAL, ONE, true, true><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(riemann_kernel<DUAL, ONE, true, true>, rb, kRiemannThreads, 0, st, B);
   else if (learned && B.learned_pass) {
     launch_guess_pass(B, B.sms, st);
-    riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, true>
-        <<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(riemann_kernel<DUAL, ONE, true, false, kRiemannThreads, false, true>,
+                 rb, kRiemannThreads, 0, st, B);
   } else if (learned)
-    riemann_kernel<DUAL, ONE, true><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(riemann_kernel<DUAL, ONE, true>, rb, kRiemannThreads, 0, st, B);
   else if (col)
-    riemann_kernel<DUAL, ONE, false, true><<<rb, kRiemannThreads, 0, st>>>(B);
+    launch_chain(riemann_kernel<DUAL, ONE, false, true>, rb, kRiemannThreads, 0, st, B);
   else
     launch_riemann_plain<DUAL, ONE, false>(B, rb, st);
   mark(3);
@@ -2686,7 +2743,7 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     else
       launch_update<DUAL, GRAV, ONE, false, false, true>(B, st);
     mark(4);
-    fallback_kernel<DUAL, GRAV, ONE, true><<<64, 128, 0, st>>>(B);
+    launch_chain(fallback_kernel<DUAL, GRAV, ONE, true>, 64, 128, 0, st, B);
   } else {
     if (PPM_X_TMA && staged && ONE && B.x_tma)
       launch_update<DUAL, GRAV, ONE, true, ONE>(B, st);
@@ -2695,16 +2752,16 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     else
       launch_update<DUAL, GRAV, ONE, false, false>(B, st);
     mark(4);
-    fallback_kernel<DUAL, GRAV, ONE><<<64, 128, 0, st>>>(B);
+    launch_chain(fallback_kernel<DUAL, GRAV, ONE>, 64, 128, 0, st, B);
   }
   if (B.ncolour > 0) {
     constexpr int cpt = PPM_COLOURS_PER_THREAD;
     const int64_t chunks = (B.ncolour + cpt - 1) / cpt;
     if (march_blocks * B.ncolour < PPM_COLOUR_WIDE_BLOCKS)
-      colour_kernel<DUAL, ONE, 1>
-          <<<(unsigned)(march_blocks * B.ncolour), kMarchThreads, 0, st>>>(B);
+      launch_chain(colour_kernel<DUAL, ONE, 1>, march_blocks * B.ncolour, kMarchThreads, 0, st,
+                   B);
     else
-      colour_kernel<DUAL, ONE, cpt><<<(unsigned)(march_blocks * chunks), kMarchThreads, 0, st>>>(B);
+      launch_chain(colour_kernel<DUAL, ONE, cpt>, march_blocks * chunks, kMarchThreads, 0, st, B);
   }
   mark(5);
 }

@@ -184,6 +184,8 @@ struct BatchArgs {
   const int64_t* upd_prefix;         // ngrids + 1 (update, transport)
   int64_t upd_blocks = 0;
   int transport = 0;                 // the transport path (see transport_kernel)
+  int both_roles = 0;                // both reconstructions in one launch
+  unsigned long long* clear_bits = nullptr;  // folded time step to reset before this sweep
   const int64_t* riemann_prefix;     // ngrids + 1
   unsigned long long* counters;      // kCounterCopies x kMaxCounters, shared by the batch
   int64_t* flagged;                  // pencils needing the fallback pass: (grid << 40) | pencil
@@ -301,6 +303,10 @@ inline void build_coef(const double* dxi_in, int n, int is0, int ie0, std::vecto
 #define PPM_TRANSPORT_CELLS 750000
 #endif
 inline bool use_transport(int64_t batch_cells) { return batch_cells >= PPM_TRANSPORT_CELLS; }
+// Both reconstructions in one launch, where their blocks are resident together.
+inline bool use_both_roles(int64_t seg_blocks, bool transport) {
+  return !transport && 2 * seg_blocks <= 148 * 4;
+}
 // The transport kernel's resident threads: two blocks of 128 an SM.
 #ifndef PPM_TRANS_FILL
 #define PPM_TRANS_FILL (148 * 2 * 128)
