@@ -57,7 +57,14 @@ struct ElemBatch {
   int presfree;
   int eos_type;
   double eos_cs;
+  ElemGrid one;
 };
+struct FieldCopy {
+  double* dst[6];
+  const double* src[6];
+  int64_t size;
+};
+void launch_copy_back(const FieldCopy& X, cudaStream_t st);
 void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st);
 void launch_cfl_finalize(const unsigned long long* min_bits, double courant, double* dt_out,
                          cudaStream_t st);
@@ -884,7 +891,8 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
     if (nc > 0) a.col_capture = (double*)ctx->col_capture.p;
   }
 
-  // descriptor image: records | march prefix | riemann prefix
+  // descriptor image: records | block prefixes.  A batch of one grid needs neither on the
+  // device: its record travels in the kernel parameters.
   std::vector<unsigned char> img;
   append(img, rec.data(), rec.size());
   const size_t off_m = align256(img.size());
@@ -903,11 +911,13 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   img.resize(off_u);
   append(img, upre.data(), upre.size());
   const int slot = kSlotSweep0 + 3 * dim + position;
-  rc = mirror_put(ctx, ctx->mirror[slot], img);
-  if (rc) return rc;
-  unsigned char* base = (unsigned char*)ctx->mirror[slot].dev.p;
+  if (ng > 1) {
+    rc = mirror_put(ctx, ctx->mirror[slot], img);
+    if (rc) return rc;
+  }
+  unsigned char* base = ng > 1 ? (unsigned char*)ctx->mirror[slot].dev.p : nullptr;
   std::memset(&plan.B.one, 0, sizeof(plan.B.one));
-  if (ng == 1) plan.B.one = rec[0];
+  if (ng == 1) std::memcpy(&plan.B.one, &rec[0], sizeof(rec[0]));  // padding too: a graph's key
   plan.B.x_tma = 0;
   // the x sweep's staged update works on warps of 32 pencils
   bool whole_warps = true;
@@ -1128,9 +1138,15 @@ int prepare_elem(ppm_b200_context* ctx, int slot, const ppm_b200_params* p,
   const size_t off_r = align256(img.size());
   img.resize(off_r);
   append(img, rpre.data(), rpre.size());
-  int rc = mirror_put(ctx, ctx->mirror[slot], img);
-  if (rc) return rc;
-  unsigned char* base = (unsigned char*)ctx->mirror[slot].dev.p;
+  // one grid's record travels in the kernel parameters (the zone copy reads the device's)
+  const bool one = ng == 1 && slot != kSlotCopy;
+  if (!one) {
+    int rc = mirror_put(ctx, ctx->mirror[slot], img);
+    if (rc) return rc;
+  }
+  std::memset(&plan.B.one, 0, sizeof(plan.B.one));
+  if (one) std::memcpy(&plan.B.one, &rec[0], sizeof(rec[0]));
+  unsigned char* base = one ? nullptr : (unsigned char*)ctx->mirror[slot].dev.p;
   plan.B.grids = (const ElemGrid*)base;
   plan.B.ngrids = ng;
   plan.B.size_prefix = (const int64_t*)(base + off_s);
@@ -1319,6 +1335,30 @@ int prepare_solve(ppm_b200_context* ctx, const ppm_b200_params* p, int cycle,
   return PPM_B200_OK;
 }
 
+// A single sweep's outputs from the grid's first ring set into its own fields: one kernel
+// below 65536 cells (a copy costs about 2 us of the stream each), copies above.
+constexpr int64_t kCopyKernelCells = 65536;
+int copy_back(ppm_b200_context* ctx, const GridIO& x) {
+  const int64_t cells = grid_size(x.g);
+  if (cells < kCopyKernelCells) {
+    ppm::FieldCopy c;
+    c.size = cells;
+    for (int k = 0; k < 6; ++k) {
+      c.dst[k] = x.user.f[k];
+      c.src[k] = x.ring[0].f[k];
+    }
+    ppm::launch_copy_back(c, ctx->stream);
+    ctx->launches += 1;
+    CK(cudaGetLastError());
+    return PPM_B200_OK;
+  }
+  for (int k = 0; k < 6; ++k)
+    if (x.user.f[k])
+      CK(cudaMemcpyAsync(x.user.f[k], x.ring[0].f[k], (size_t)cells * sizeof(double),
+                         cudaMemcpyDeviceToDevice, ctx->stream));
+  return PPM_B200_OK;
+}
+
 // cfl_first / cfl_last: this solve is the first / last of a level's waves, which share
 // one folded time step: the minimum is reset before the first wave's last sweep and the
 // time step written after the last wave's (every wave reads the old one until then).
@@ -1339,15 +1379,11 @@ int enqueue_solve(ppm_b200_context* ctx, const ppm_b200_params* p, const std::ve
       CK(cudaGetLastError());
     }
   }
-  if (sp.nsweeps == 1) {
+  if (sp.nsweeps == 1)
     for (const auto& x : io) {
-      const size_t bytes = (size_t)grid_size(x.g) * sizeof(double);
-      for (int k = 0; k < 6; ++k)
-        if (x.user.f[k])
-          CK(cudaMemcpyAsync(x.user.f[k], x.ring[0].f[k], bytes, cudaMemcpyDeviceToDevice,
-                             ctx->stream));
+      int rc = copy_back(ctx, x);
+      if (rc) return rc;
     }
-  }
   if (p->eos_type > 0) {  // energies consistent with the EOS again (Grid_SolvePPM_DE.C:155-157)
     ppm::launch_pressure_batch(sp.pressure.B, sp.pressure.size_blocks, ctx->stream);
     ctx->launches += 1;
@@ -1494,6 +1530,7 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
   const ElemBatch& e = sp.pressure.B;
   key_put(k, e.grids);
   key_put(k, e.ngrids);
+  if (e.ngrids == 1) key_put(k, e.one);
   key_put(k, e.size_prefix);
   key_put(k, e.active_prefix);
   key_put(k, e.row_prefix);
@@ -1509,6 +1546,7 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, sp.order[s]);
     key_put(k, b.grids);
     key_put(k, b.ngrids);
+    if (b.ngrids == 1) key_put(k, b.one);
     key_put(k, b.march_prefix);
     key_put(k, b.riemann_prefix);
     key_put(k, b.seg_prefix);
@@ -2005,6 +2043,8 @@ int ppm_b200_solve_level(ppm_b200_context* ctx, const ppm_b200_params* p, int cy
       ctx->launches += 1 + (p->eos_type > 0 ? 1 : 0);
       for (int s = 0; s < sp.nsweeps; ++s) ctx->launches += sweep_kernels(p, sp.sweep[s].B);
     }
+    if (plans[0].nsweeps == 1)
+      for (const auto& x : io) ctx->launches += grid_size(x.g) < kCopyKernelCells ? 1 : 0;
     if (ctx->cfl_dt) ctx->launches += 1;  // the folded time step's finalize kernel
   } else {
     rc = enqueue_all(false);
@@ -2052,11 +2092,8 @@ int ppm_b200_euler_sweep(ppm_b200_context* ctx, int dim, const ppm_b200_params* 
   if (rc) return rc;
   rc = scatter_captures(ctx, dim, p, g, plan, sub);
   if (rc) return rc;
-  const size_t bytes = (size_t)grid_size(g) * sizeof(double);
-  for (int k = 0; k < 6; ++k)
-    if (io[0].user.f[k])
-      CK(cudaMemcpyAsync(io[0].user.f[k], io[0].ring[0].f[k], bytes, cudaMemcpyDeviceToDevice,
-                         ctx->stream));
+  rc = copy_back(ctx, io[0]);
+  if (rc) return rc;
   if (memory == PPM_B200_MEM_HOST) {
     rc = stage_out(ctx, p, g, io[0].user);
     if (rc) return rc;

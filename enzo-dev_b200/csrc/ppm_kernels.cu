@@ -51,7 +51,20 @@ struct ElemBatch {
   // p/((gamma-1) rho) + v^2/2 wherever the pressure is computed (Grid_ComputePressure.C:112-124)
   int eos_type;
   double eos_cs;
+  ElemGrid one;                  // the record itself when ngrids == 1 (no upload, no table)
 };
+
+// The block's grid, and its index among that grid's blocks.  A batch of one grid (ONE)
+// reads its record from the kernel parameters.
+template <bool ONE>
+__device__ __forceinline__ const ElemGrid& elem_grid(const ElemBatch& B, const int64_t* prefix,
+                                                     int64_t& lb) {
+  if (ONE) {
+    lb = blockIdx.x;
+    return B.one;
+  }
+  return B.grids[batch_locate(prefix, B.ngrids, blockIdx.x, lb)];
+}
 
 // grid::ComputePressure at time == Time (Grid_ComputePressure.C:96-164)
 __device__ __forceinline__ double cell_pressure(const ElemGrid& G, int64_t i, double gamma,
@@ -92,10 +105,11 @@ __device__ __forceinline__ double eos_pressure(const ElemGrid& G, int64_t i, con
   return p;
 }
 
+template <bool ONE>
 __global__ void __launch_bounds__(256) pressure_kernel(const __grid_constant__ ElemBatch B) {
   pdl_begin();
   int64_t lb;
-  const ElemGrid& G = B.grids[batch_locate(B.size_prefix, B.ngrids, blockIdx.x, lb)];
+  const ElemGrid& G = elem_grid<ONE>(B, B.size_prefix, lb);
   const int64_t i = lb * 256 + threadIdx.x;
   if (i < G.size)
     G.p[i] = B.eos_type == 3 ? eos_pressure<true>(G, i, B)
@@ -103,10 +117,11 @@ __global__ void __launch_bounds__(256) pressure_kernel(const __grid_constant__ E
 }
 
 // calc_dt (ihydro = 0) over the active cells of every grid; min over the batch
+template <bool ONE>
 __global__ void __launch_bounds__(256) timestep_kernel(const __grid_constant__ ElemBatch B) {
   pdl_begin();
   int64_t lb;
-  const ElemGrid& G = B.grids[batch_locate(B.active_prefix, B.ngrids, blockIdx.x, lb)];
+  const ElemGrid& G = elem_grid<ONE>(B, B.active_prefix, lb);
   const int64_t c = lb * 256 + threadIdx.x;
   double best = 1.0e20;  // calc_dt.F:71 (huge)
   if (c < G.active) {
@@ -190,12 +205,14 @@ __device__ __forceinline__ void copy_cell(double* const (&f)[6], int64_t dst, in
 // in-place fill has no read-after-write hazard.  A grid's blocks (ceil(rows / 32), 8
 // warps each) stride over its rows, about four per warp, so that the block-to-grid search
 // and the record's fields are amortised over several rows.
+template <bool ONE>
 __global__ void __launch_bounds__(256) boundary_kernel(const __grid_constant__ ElemBatch B) {
   pdl_begin();
   int64_t lb;
-  const int gi = batch_locate(B.row_prefix, B.ngrids, blockIdx.x, lb);
-  const ElemGrid& G = B.grids[gi];
-  const int64_t warps = (B.row_prefix[gi + 1] - B.row_prefix[gi]) * 8;
+  const int gi = ONE ? 0 : batch_locate(B.row_prefix, B.ngrids, blockIdx.x, lb);
+  if (ONE) lb = blockIdx.x;
+  const ElemGrid& G = ONE ? B.one : B.grids[gi];
+  const int64_t warps = (ONE ? (int64_t)gridDim.x : B.row_prefix[gi + 1] - B.row_prefix[gi]) * 8;
   const int n0 = G.dims[0], n1 = G.dims[1], n2 = G.dims[2];
   const int s0 = G.start[0], e0 = G.end[0], bc0 = G.bc[0];
   const int s1 = G.start[1], e1 = G.end[1], bc1 = G.bc[1];
@@ -449,10 +466,11 @@ __device__ __forceinline__ double cell_pressure_interp(const ElemGrid& G, int64_
   return p;
 }
 
+template <bool ONE>
 __global__ void __launch_bounds__(256) expansion_kernel(const __grid_constant__ ElemBatch B) {
   pdl_begin();
   int64_t lb;
-  const ElemGrid& G = B.grids[batch_locate(B.size_prefix, B.ngrids, blockIdx.x, lb)];
+  const ElemGrid& G = elem_grid<ONE>(B, B.size_prefix, lb);
   const int64_t i = lb * 256 + threadIdx.x;
   if (i >= G.size) return;
   const double p = B.interpolate ? cell_pressure_interp(G, i, B)
@@ -474,15 +492,34 @@ __global__ void __launch_bounds__(256) expansion_kernel(const __grid_constant__ 
   }
 }
 
+// The updated fields of a small grid's single sweep back into the caller's arrays (one
+// launch of the chain instead of up to six copies between its kernels).
+struct FieldCopy {
+  double* dst[6];  // null entries skipped
+  const double* src[6];
+  int64_t size;
+};
+__global__ void __launch_bounds__(256) copy_back_kernel(const __grid_constant__ FieldCopy X) {
+  pdl_begin();
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= X.size) return;
+#pragma unroll
+  for (int k = 0; k < 6; ++k)
+    if (X.dst[k]) X.dst[k][i] = X.src[k][i];
+}
+void launch_copy_back(const FieldCopy& X, cudaStream_t st) {
+  launch_chain(copy_back_kernel, (X.size + 255) / 256, 256, 0, st, X);
+}
+
 // ------------------------------------------------------------------ launchers
 void launch_pressure_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  launch_chain(pressure_kernel, blocks, 256, 0, st, B);
+  launch_chain(B.ngrids == 1 ? pressure_kernel<true> : pressure_kernel<false>, blocks, 256, 0, st, B);
 }
 
 void launch_timestep_batch(const ElemBatch& B, int64_t blocks, double courant, double* dt_out,
                            cudaStream_t st) {
   cudaMemsetAsync(B.min_bits, 0xFF, sizeof(unsigned long long), st);
-  launch_chain(timestep_kernel, blocks, 256, 0, st, B);
+  launch_chain(B.ngrids == 1 ? timestep_kernel<true> : timestep_kernel<false>, blocks, 256, 0, st, B);
   const unsigned long long* bits = B.min_bits;
   launch_chain(timestep_finalize_kernel, 1, 32, 0, st, bits, courant, dt_out);
 }
@@ -494,11 +531,11 @@ void launch_cfl_finalize(const unsigned long long* min_bits, double courant, dou
 }
 
 void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  launch_chain(expansion_kernel, blocks, 256, 0, st, B);
+  launch_chain(B.ngrids == 1 ? expansion_kernel<true> : expansion_kernel<false>, blocks, 256, 0, st, B);
 }
 
 void launch_boundary_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  launch_chain(boundary_kernel, blocks, 256, 0, st, B);
+  launch_chain(B.ngrids == 1 ? boundary_kernel<true> : boundary_kernel<false>, blocks, 256, 0, st, B);
 }
 
 }  // namespace ppm
