@@ -211,6 +211,10 @@ __global__ void __launch_bounds__(kMarchThreads) corrections_kernel(const __grid
 #endif
 // PPM_RECON_PREFETCH: a steady step of the march loads the next cell's values while it
 // computes with this one (v/w/ge march 0.55 -> 0.48 ms per 256^3 sweep)
+#ifndef PPM_RECON_UNROLL
+#define PPM_RECON_UNROLL 1
+#endif
+constexpr int kReconUnroll = PPM_RECON_UNROLL;
 #ifndef PPM_RECON_PREFETCH
 #define PPM_RECON_PREFETCH 1
 #endif
@@ -447,7 +451,7 @@ __device__ __forceinline__ void reconstruct_pencil(const SweepArgs& a, int pid, 
 #pragma unroll 1
   for (int t = f0 - 3; t < t_steady0 && t <= tend; ++t) step(t, Ramp{});
   if (PPM_RECON_PREFETCH && t_steady0 <= t_steady1) fetch(t_steady0);
-#pragma unroll 1
+#pragma unroll kReconUnroll
   for (int t = t_steady0; t <= t_steady1; ++t) step(t, Steady{});
 #pragma unroll 1
   for (int t = t_steady1 + 1 > t_steady0 ? t_steady1 + 1 : t_steady0; t <= tend; ++t)
@@ -1462,7 +1466,7 @@ __device__ __forceinline__ void flush_stage(const SweepArgs& a, const double* st
     const int j = q % kStageCells, p = q / kStageCells;
     const int pid = pid0 + p;
     if (j < ncells && pid < a.npencils) {
-      const int off = pencil_base(a, pid) + (c0 + j);  // sa == 1
+      const int off = pid * (int)a.s1 + (c0 + j);  // x sweep: pencils are consecutive rows
       const double* sp = stage + j * kStageLd + p;
       a.out_d[off] = sp[0];
       a.out_e[off] = sp[kStageField];
@@ -1933,12 +1937,21 @@ __global__ void __launch_bounds__(128) fallback_kernel(const __grid_constant__ B
 // fa .. fb, loads from three cells left of cb to three right of ce.  A pencil with a cell
 // that fails its check goes to the fallback pass.
 // PD: the inputs arrive through a cp.async ring PD steps ahead, as in update_pencil;
-// STAGED: the x sweep's staged stores, with plain loads a step ahead, or XT, its input
-// cells as TMA tiles.
-enum { UD = 0, UP, UU, UV, UW, UGE, UE, UPB, UDB, UUB, UG, kTransVals };
-template <int PD>
+// STAGED: the x sweep's staged stores; XT: its input cells as TMA tiles (the ring then
+// carries the face's values alone).
+#ifndef PPM_TRANS_UNROLL
+#define PPM_TRANS_UNROLL 1
+#endif
+constexpr int kTransUnroll = PPM_TRANS_UNROLL;
+enum { UPB = 0, UDB, UUB, UG, UD, UP, UU, UV, UW, UGE, UE, kTransVals };
+// values of a ring unit: with TMA tiles (XT) only the face's and the acceleration
+template <bool XT>
+__host__ __device__ constexpr int trans_vals() {
+  return XT ? UG + 1 : kTransVals;
+}
+template <int PD, bool XT>
 __host__ __device__ constexpr int trans_ring_doubles() {
-  return PD > 0 ? (PD + 1) * kTransVals * kMarchThreads : 0;
+  return (PD + 1) * trans_vals<XT>() * kMarchThreads;
 }
 constexpr int kTransTiles = 7;  // TMA tiles: d, e, u, v, w, ge, p (BatchArgs::xin)
 
@@ -1947,7 +1960,6 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
                                                  UpdateCounts& cnt, int c0, int c1, bool valid,
                                                  double* stage, int pid0, double* ring,
                                                  XTiles* xt) {
-  static_assert(!(PD > 0 && STAGED), "the ring serves the y and z sweeps");
   constexpr int NV = DUAL ? 3 : 2;
   bool live = valid, flagged = false, handed = false;
   const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
@@ -1976,20 +1988,10 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
   }
 
   // inputs of step t: cell t, the energy (and acceleration) of cell t-3, face t-2
-  double in[kTransVals];  // the next step's values (neither PD nor XT)
-#pragma unroll
-  for (int k = 0; k < kTransVals; ++k) in[k] = 0.0;
   auto fetch = [&](const int t, auto steady) {
     constexpr bool ST = decltype(steady)::value;
-    double* r = PD > 0 ? ring + (t % (PD + 1)) * (kTransVals * kMarchThreads) : nullptr;
-    auto get = [&](int k, const double* p) {
-      if (PD > 0)
-        cp_async8(r + k * kMarchThreads, p);
-      else if (STAGED && k < UPB)
-        in[k] = ldg_keep(p);
-      else
-        in[k] = __ldcs(p);
-    };
+    double* r = ring + (t % (PD + 1)) * (trans_vals<XT>() * kMarchThreads);
+    auto get = [&](int k, const double* p) { cp_async8(r + k * kMarchThreads, p); };
     if (!XT && (ST || t <= hi)) {
       const int off = base + t * sa;
       get(UD, a.in_d + off);
@@ -2010,7 +2012,7 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
       get(UDB, f + XDB * pl);
       get(UUB, f + XUB * pl);
     }
-    if (PD > 0) cp_async_commit();
+    cp_async_commit();
   };
 
   double wq0[3], wq1[3], wq2[3];  // v, w, ge of cells t-3, t-2, t-1
@@ -2055,10 +2057,19 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
     if (XT && (ST || t <= hi) && (t % kXTileCells == 0 || (!ST && t == lo)))
       x_chunk<kTransTiles>(*xt, t / kXTileCells - xt->q0, hi + 1);
     if (live) {
-      if (PD > 0) {
-        cp_async_wait<(PD > 0 ? PD - 1 : 0)>();
-        const double* r = ring + (t % (PD + 1)) * (kTransVals * kMarchThreads);
-        if (ST || t <= hi) {
+      cp_async_wait<PD - 1>();
+      const double* r = ring + (t % (PD + 1)) * (trans_vals<XT>() * kMarchThreads);
+      if (ST || t <= hi) {
+        if (XT) {
+          const double* x = x_row<kTransTiles>(*xt, t);
+          nd = x[0];
+          ne = x[kXTile];
+          nu = a.in_u ? x[2 * kXTile] : 0.0;
+          nq[0] = a.in_v ? x[3 * kXTile] : 0.0;
+          nq[1] = a.in_w ? x[4 * kXTile] : 0.0;
+          nq[2] = DUAL ? x[5 * kXTile] : 0.0;
+          np_ = x[6 * kXTile];
+        } else {
           nd = r[UD * kMarchThreads];
           np_ = r[UP * kMarchThreads];
           nu = a.in_u ? r[UU * kMarchThreads] : 0.0;
@@ -2066,38 +2077,14 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
           nq[1] = a.in_w ? r[UW * kMarchThreads] : 0.0;
           nq[2] = DUAL ? r[UGE * kMarchThreads] : 0.0;
         }
-        if (ST || (t - 3 >= cb && t - 3 <= ce)) {
-          e3 = r[UE * kMarchThreads];
-          if (GRAV) g3 = r[UG * kMarchThreads];
-        }
-        if (ST || (t - 2 >= fa && t - 2 <= fb))
-          G = Godunov{r[UPB * kMarchThreads], r[UDB * kMarchThreads], r[UUB * kMarchThreads]};
-        fetch(t + PD, steady);
-      } else {
-        if (XT) {
-          if (ST || t <= hi) {
-            const double* r = x_row<kTransTiles>(*xt, t);
-            nd = r[0];
-            ne = r[kXTile];
-            nu = a.in_u ? r[2 * kXTile] : 0.0;
-            nq[0] = a.in_v ? r[3 * kXTile] : 0.0;
-            nq[1] = a.in_w ? r[4 * kXTile] : 0.0;
-            nq[2] = DUAL ? r[5 * kXTile] : 0.0;
-            np_ = r[6 * kXTile];
-          }
-        } else {
-          nd = in[UD];
-          np_ = in[UP];
-          nu = in[UU];
-          nq[0] = in[UV];
-          nq[1] = in[UW];
-          nq[2] = in[UGE];
-          e3 = in[UE];
-        }
-        g3 = in[UG];
-        G = Godunov{in[UPB], in[UDB], in[UUB]};
-        fetch(t + 1, steady);
       }
+      if (ST || (t - 3 >= cb && t - 3 <= ce)) {
+        if (!XT) e3 = r[UE * kMarchThreads];
+        if (GRAV) g3 = r[UG * kMarchThreads];
+      }
+      if (ST || (t - 2 >= fa && t - 2 <= fb))
+        G = Godunov{r[UPB * kMarchThreads], r[UDB * kMarchThreads], r[UUB * kMarchThreads]};
+      fetch(t + PD, steady);
     }
     // ---- reconstruction of v, w, ge (reconstruct_pencil, ROLE 1)
     Prep prC = prB;
@@ -2161,7 +2148,7 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
       }
       if (C.d + (F0.df - F1.df) <= 0.0 || C.e < 0.0) {  // to the fallback pass
         if (!STAGED) {
-          if (PD > 0) cp_async_wait<0>();
+          cp_async_wait<0>();
           handed = true;
           return;
         }
@@ -2189,7 +2176,7 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
         dep = pgas2d_de_local(PEm, P, known);
         if (!known) {
           if (!STAGED) {
-            if (PD > 0) cp_async_wait<0>();
+            cp_async_wait<0>();
             handed = true;
             return;
           }
@@ -2246,23 +2233,22 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
     for (int q = 0; q < kXBuffers - 1 && (xt->q0 + q) * kXTileCells <= hi; ++q)
       x_issue<kTransTiles>(*xt, q);
   }
-  constexpr int AHEAD = PD > 0 ? PD : 1;
   if (live) {
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u) fetch(lo + u, Ramp{});
+    for (int u = 0; u < PD; ++u) fetch(lo + u, Ramp{});
   }
   const int tlast = ce + 3;
   auto max2 = [](int x, int y) { return x > y ? x : y; };
   auto min2 = [](int x, int y) { return x < y ? x : y; };
   // every range of a steady step, and of the steps it fetches for
   const int s0 = max2(max2(fa + 2, is + 3), c0 + 4);
-  const int s1 = min2(min2(hi, fb + 2), min2(ie + 3, c1 + 3)) - AHEAD;
+  const int s1 = min2(min2(hi, fb + 2), min2(ie + 3, c1 + 3)) - PD;
 #pragma unroll 1
   for (int t = lo; t < s0 && t <= tlast; ++t) {
     step(t, Ramp{});
     if (handed) return true;
   }
-#pragma unroll 1
+#pragma unroll kTransUnroll
   for (int t = s0; t <= s1; ++t) {
     step(t, Steady{});
     if (!STAGED && handed) return true;
@@ -2288,7 +2274,7 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
       flush_stage<DUAL>(a, stage, pid0, k0, k - k0 + 1);
     }
   }
-  if (PD > 0) cp_async_wait<0>();
+  cp_async_wait<0>();
   if (XT) x_drain(*xt);
   cnt.nonfinite += nonfin;
   cnt.dtmin = dtmin;
@@ -2304,15 +2290,11 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
 #ifndef PPM_TRANS_PIPE
 #define PPM_TRANS_PIPE 2
 #endif
-template <bool STAGED>
-__host__ __device__ constexpr int trans_pipe() {
-  return STAGED ? 0 : PPM_TRANS_PIPE;
-}
 constexpr int kTransXBlock = (kMarchThreads / 32) * x_warp_doubles<kTransTiles>();
 template <bool STAGED, bool XT>
 constexpr size_t trans_smem_bytes() {
   return sizeof(double) * ((XT ? kTransXBlock : 0) + (STAGED ? kStageBlock : 0) +
-                           trans_ring_doubles<trans_pipe<STAGED>()>());
+                           trans_ring_doubles<PPM_TRANS_PIPE, XT>());
 }
 
 template <bool DUAL, bool GRAV, bool ONE, bool COR, bool STAGED, bool XT>
@@ -2326,6 +2308,7 @@ __global__ void __launch_bounds__(kMarchThreads,
   __shared__ uint64_t s_xbar[XT ? (kMarchThreads / 32) * kXBuffers : 1];
   extern __shared__ __align__(128) double s_dyn[];
   double* const s_stage = s_dyn + (XT ? kTransXBlock : 0);
+  double* const s_ring = s_stage + (STAGED ? kStageBlock : 0);
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
   s_flag[threadIdx.x] = 0;
   int64_t lb;
@@ -2348,9 +2331,9 @@ __global__ void __launch_bounds__(kMarchThreads,
   UpdateCounts cnt = {0, 0, 0, 1.0e20};
   if ((STAGED || valid) && c0 < a.n) {
     const Phys P = make_phys(a);
-    if (transport_pencil<DUAL, GRAV, COR, STAGED, trans_pipe<STAGED>(), XT>(
+    if (transport_pencil<DUAL, GRAV, COR, STAGED, PPM_TRANS_PIPE, XT>(
             a, pid, P, cnt, c0, c1, valid, s_stage + warp * kStageWarp, wpid0,
-            s_dyn + threadIdx.x, &xt))
+            s_ring + threadIdx.x, &xt))
       s_flag[pl] = 1;
   }
   finish_block(B, a, g, pid, valid && c0 == 0, s_flag, pl, s_cnt, cnt);
