@@ -432,14 +432,38 @@ struct Riemann {
   bool converged; // reached |dp/p| < tolerance within numiter - 1 updates
 };
 
-__device__ __forceinline__ double acoustic_guess(const FaceState& s, double cl, double cr,
+// cl, cr = sqrt(gamma p d) of the two sides, and (tolerance build) their reciprocals; the
+// face states are at least tiny (1e-20), so the arguments are positive and normal
+struct Lagrangian {
+  double cl, cr, icl, icr;
+};
+__device__ __forceinline__ Lagrangian lagrangian(const FaceState& s, const Phys& P) {
+  Lagrangian c;
+#if PPM_FAST_ALGEBRA
+  c.cl = qsqrt_n(P.gamma * s.pl * s.dl, c.icl);
+  c.cr = qsqrt_n(P.gamma * s.pr * s.dr, c.icr);
+#else
+  c.cl = sqrt(P.gamma * s.pl * s.dl);
+  c.cr = sqrt(P.gamma * s.pr * s.dr);
+  c.icl = c.icr = 0.0;
+#endif
+  return c;
+}
+
+__device__ __forceinline__ double acoustic_guess(const FaceState& s, const Lagrangian& c,
                                                  const Phys& P) {
-  double ps = qdiv(cr * s.pl + cl * s.pr + cr * cl * (s.ul - s.ur), cr + cl);
+  const double cl = c.cl, cr = c.cr;
+  double ps = (cr * s.pl + cl * s.pr + cr * cl * (s.ul - s.ur));
+#if PPM_FAST_ALGEBRA
+  ps *= qrcp_n(cr + cl);
+#else
+  ps = ps / (cr + cl);
+#endif
   if (ps < P.pmin) ps = P.pmin;
   return ps;
 }
 
-__device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, double cl, double cr,
+__device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, const Lagrangian& c,
                                                    double ps, const Phys& P) {
   double old_ps = ps, ubl = 0.0, ubr = 0.0;
   int it = 0;
@@ -452,7 +476,7 @@ __device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, double cl
   // with y = 1/sqrt(X) and 1/z = y/c an update takes two reciprocal square roots and one
   // reciprocal (the reference's form: two roots and eight divisions).  256^3 sweep: 1138 k
   // issue cycles -> 828 k, 0.73 -> 0.58 ms (with the flux's shared reciprocals below).
-  const double icl = qrcp_n(cl), icr = qrcp_n(cr);
+  const double icl = c.icl, icr = c.icr;
   const double qp = P.qa * qrcp_n(s.pl * s.pr), gl = s.pr * qp, gr = s.pl * qp;
   const double omq = 1.0 - P.qa;
   double il = 0.0, ir = 0.0, qs = 0.0;  // 1/dpl, 1/dpr, 1/(1/dpl + 1/dpr)
@@ -476,6 +500,7 @@ __device__ __forceinline__ Riemann twoshock_newton(const FaceState& s, double cl
     }
   }
 #else
+  const double cl = c.cl, cr = c.cr;
   double dpdul = 0.0, dpdur = 0.0;
 #pragma unroll 1
   for (int n = 2; n <= kNumIter; n++) {
@@ -537,13 +562,28 @@ __device__ __forceinline__ Godunov godunov_state(const FaceState& s, double pbar
   const double X = dmax(1.0 + P.qa * (pbar * (d0 * q0) - 1.0), kTiny);
   const double c02X = c02 * X;
   const double z02 = dmax(c02X * (d0 * d0), kTiny), zd = z02 - (pbar - p0) * d0;
-  const double qz = qrcp(z02 * zd);
+  const double qz = qrcp_n(z02 * zd);  // z02 >= tiny, zd of its order
   const double idbar = id0 * (zd * zd * qz);
   const double dbar = d0 * (z02 * z02 * qz);
   const bool rare = pbar < p0;
-  const double l0 = u0 * sn + qsqrt(rare ? c02 : c02X);
-  const double cbar = qsqrt(dmax(gamma * pbar * idbar, kTiny));
+  double iroot;
+  const double l0 = u0 * sn + qsqrt_n(rare ? c02 : c02X, iroot);
+  const double cbar = qsqrt_n(dmax(gamma * pbar * idbar, kTiny), iroot);
   const double lbar = rare ? sn * ubar + cbar : l0;
+  // inside a rarefaction fan only where the face lies between its head and tail
+  double pb = pbar, db = dbar, ub = ubar;
+  if (l0 < 0.0) {
+    pb = p0; db = d0; ub = u0;
+  } else if (!(lbar >= 0.0)) {
+    double frac = l0 - lbar;
+    if (frac < kTiny) frac = kTiny;
+    frac = qdiv(0.0 - lbar, frac);
+    frac = dmin(dmax(frac, 0.0), 1.0);
+    const double rest = 1.0 - frac;
+    pb = fma(p0, frac, __dmul_rn(pbar, rest));
+    db = fma(d0, frac, __dmul_rn(dbar, rest));
+    ub = fma(u0, frac, __dmul_rn(ubar, rest));
+  }
 #else
   double c0 = sqrt(dmax(gamma * p0 / d0, kTiny));
   double z0 = c0 * d0 * sqrt(dmax(1.0 + P.qa * (pbar / p0 - 1.0), kTiny));
@@ -557,7 +597,6 @@ __device__ __forceinline__ Godunov godunov_state(const FaceState& s, double pbar
     l0 = u0 * sn + z0 / d0;
     lbar = l0;
   }
-#endif
   double frac = l0 - lbar;
   if (frac < kTiny) frac = kTiny;
   frac = qdiv(0.0 - lbar, frac);
@@ -571,6 +610,7 @@ __device__ __forceinline__ Godunov godunov_state(const FaceState& s, double pbar
   if (l0 < 0.0) {
     pb = p0; db = d0; ub = u0;
   }
+#endif
   return Godunov{pb, db, ub};
 }
 
@@ -591,7 +631,7 @@ __device__ __forceinline__ Flux godunov_flux(const Godunov& G, const AdvState& s
   const double dub = ub * db;
 #if PPM_FAST_ALGEBRA
   const double ke = fma(ub, ub, fma(vb, vb, __dmul_rn(wb, wb)));
-  const double eb = fma(0.5, ke, qdiv(pb, P.gm1 * db));
+  const double eb = fma(0.5, ke, __dmul_rn(pb, qrcp_n(P.gm1 * db)));
   const double efl = fma(dub, eb, __dmul_rn(pb, ub)), ufl = fma(dub, ub, pb);
 #else
   const double eb = pb / (P.gm1 * db) + 0.5 * (ub * ub + vb * vb + wb * wb);
@@ -766,11 +806,8 @@ __device__ __forceinline__ Cell euler_update(const Cell& c, const Flux& F0, cons
                                              double ges, double gr, const Phys& P, bool& fatal) {
   Cell o;
   double dnu = c.d + (F0.df - F1.df);
-  double dnuinv = qrcp(dnu);
-  if (P.small_rho > 0.0) {
-    dnu = dmax(dnu, P.small_rho);
-    dnuinv = qrcp(dnu);
-  }
+  if (P.small_rho > 0.0) dnu = dmax(dnu, P.small_rho);
+  const double dnuinv = qrcp(dnu);
   double uold = c.u;
   o.u = (c.u * c.d + (F0.uf - F1.uf)) * dnuinv;
   o.v = (c.v * c.d + (F0.vf - F1.vf)) * dnuinv;
@@ -791,6 +828,27 @@ __device__ __forceinline__ Cell euler_update(const Cell& c, const Flux& F0, cons
   return o;
 }
 
+// x/y > eta.  The tolerance build compares x with eta*y instead (y >= 0, or the other way
+// round), as the quotient itself is not needed.
+__device__ __forceinline__ bool over(double x, double y, double eta) {
+#if PPM_FAST_ALGEBRA
+  const double t = eta * y;
+  return y >= 0.0 ? x > t : x < t;
+#else
+  return x / y > eta;
+#endif
+}
+
+// max(ge, pmin/((gamma-1) d)); the tolerance build divides only where the floor may hold
+// (the factor leaves room for the rounding of the product)
+__device__ __forceinline__ double pressure_floor(double ge, double d, const Phys& P) {
+  const double gd = P.gm1 * d;
+#if PPM_FAST_ALGEBRA
+  if (ge * gd > 1.000001 * P.pmin) return ge;
+#endif
+  return dmax(ge, qdiv(P.pmin, gd));
+}
+
 // ----------------------------------------------------- pgas2d_dual.F:70-117 (one cell)
 // de_m / de_p: dslice*eslice of the clamped left / right neighbours, the left one
 // already rewritten by this routine (the loop is sequential along the pencil).
@@ -798,9 +856,9 @@ __device__ __forceinline__ void pgas2d_dual(Cell& c, double de_m, double de_p, c
   double ke = 0.5 * (c.u * c.u + c.v * c.v + c.w * c.w);
   double ge1 = c.e - ke;
   double demax = dmax(dmax(c.d * c.e, de_m), de_p);
-  if (qdiv(ge1 * c.d, demax) > P.eta2) c.ge = ge1;
-  double ge2 = (qdiv(ge1, c.e) > P.eta1) ? ge1 : c.ge;
-  ge2 = dmax(ge2, qdiv(P.pmin, P.gm1 * c.d));
+  if (over(ge1 * c.d, demax, P.eta2)) c.ge = ge1;
+  double ge2 = over(ge1, c.e, P.eta1) ? ge1 : c.ge;
+  ge2 = pressure_floor(ge2, c.d, P);
   c.e = c.e - ge1 + ge2;
 }
 
@@ -814,10 +872,10 @@ __device__ __forceinline__ double pgas2d_de_local(const Cell& c, const Phys& P, 
   double ke = 0.5 * (c.u * c.u + c.v * c.v + c.w * c.w);
   double ge1 = c.e - ke;
   const double own = c.d * c.e;
-  const bool rebuilt = qdiv(ge1, c.e) > P.eta1;
+  const bool rebuilt = over(ge1, c.e, P.eta1);
   known = rebuilt || (own > 0.0 && qdiv(ge1 * c.d, own) <= 0.5 * P.eta2);
   double ge2 = rebuilt ? ge1 : c.ge;
-  ge2 = dmax(ge2, qdiv(P.pmin, P.gm1 * c.d));
+  ge2 = pressure_floor(ge2, c.d, P);
   return c.d * (c.e - ge1 + ge2);
 }
 

@@ -92,6 +92,18 @@ __device__ __forceinline__ double qrsqrt_n(double x) {
 #endif
 }
 
+// sqrt(x) and 1/sqrt(x) of a positive normal x
+__device__ __forceinline__ double qsqrt_n(double x, double& inv) {
+#if PPM_FAST_DIVSQRT
+  inv = qrsqrt_n(x);
+  return x * inv;
+#else
+  const double r = sqrt(x);
+  inv = 1.0 / r;
+  return r;
+#endif
+}
+
 // a/b
 __device__ __forceinline__ double qdiv(double a, double b) {
 #if PPM_FAST_DIVSQRT

@@ -612,20 +612,19 @@ __global__ void __launch_bounds__(RT, (LEARNED ? PPM_RIEMANN_LEARNED_MINBLOCKS
   }
   unsigned trips = 0;  // Newton updates of this lane's face (both starts when rejected)
   if (valid) {
-    const double cl = qsqrt(P.gamma * s.pl * s.dl);
-    const double cr = qsqrt(P.gamma * s.pr * s.dr);
-    const double ps = acoustic_guess(s, cl, cr, P);
+    const Lagrangian lc = lagrangian(s, P);
+    const double ps = acoustic_guess(s, lc, P);
     Riemann rs;
     unsigned spent = 0;
     if (LEARNED) {
-      rs = twoshock_newton(s, cl, cr, guess_pressure(ps, y, d2, P.pmin), P);
+      rs = twoshock_newton(s, lc, guess_pressure(ps, y, d2, P.pmin), P);
       if (!rs.converged) {
         spent = (unsigned)rs.iters;
-        rs = twoshock_newton(s, cl, cr, ps, P);
+        rs = twoshock_newton(s, lc, ps, P);
         atomicAdd(&s_rejected, 1u);
       }
     } else {
-      rs = twoshock_newton(s, cl, cr, ps, P);
+      rs = twoshock_newton(s, lc, ps, P);
       if (a.log && a.log_stride > 0) {
         const unsigned long long h =
             ((unsigned long long)idx + 0x9E3779B97F4A7C15ull * (unsigned long long)(g + 1)) *
@@ -843,9 +842,8 @@ __global__ void __launch_bounds__(kFaceThreads, PPM_FACE_MINBLOCKS)
   const int64_t idx = (int64_t)(c - is) * np + pid;
   unsigned trips = 0;
   if (face_ok) {
-    const double clr = qsqrt(P.gamma * st.pl * st.dl);
-    const double crr = qsqrt(P.gamma * st.pr * st.dr);
-    rs = twoshock_newton(st, clr, crr, acoustic_guess(st, clr, crr, P), P);
+    const Lagrangian lc = lagrangian(st, P);
+    rs = twoshock_newton(st, lc, acoustic_guess(st, lc, P), P);
     trips = (unsigned)rs.iters;
     if (a.log && a.log_stride > 0) {
       const unsigned long long h =
@@ -1435,6 +1433,71 @@ __device__ __forceinline__ double cell_dt1(const SweepArgs& a, const Cell& o, do
                   (cs + fabs(velocity3 - a.vg[2])) / dx[2]);
 }
 
+// Whether a cell can hold the block's smallest dt1 = aye/S, S the sum of (cs + |v - vg|)/dx:
+// S is estimated to 20 bits (one approximate root, no division) and compared, by the upper
+// word of the double, with the largest estimate of the block's cells so far (best, shared
+// memory).  A cell more than 4 units of that word below it cannot be the smallest, so its
+// calc_dt (IEEE root and divisions, a sixth of the last sweep's update) is left out.  The
+// reciprocal widths are the pencil's (w1, w2 across the sweep).
+struct CflFilter {
+  double ix, i1, i2, gu, gv, gw;
+  int* best;
+  bool on, has_v, has_w;
+};
+constexpr int kCflMargin = 16;  // units of the upper word: at least 7.6e-6, the estimate 2e-6
+__device__ __forceinline__ CflFilter cfl_filter(const SweepArgs& a, int t1, int t2, int* best) {
+  CflFilter f;
+  const int dim = a.dim;
+  f.on = a.cfl_min_bits && best && a.uniform && a.aye > 0.0 && a.eos_type == 0 && !a.presfree;
+  f.best = best;
+  // the axes of (u, v, w): (x, y, z), (y, z, x), (z, x, y); of (t1, t2): (y, z), (x, z),
+  // (x, y)
+  const double w1 = a.cw1 ? a.cw1[t1] : 1.0, w2 = a.cw2 ? a.cw2[t2] : 1.0;
+  f.ix = qrcp(a.uc.dx);
+  f.i1 = qrcp(dim == 1 ? w2 : w1);
+  f.i2 = qrcp(dim == 1 ? w1 : w2);
+  f.gu = a.vg[dim];
+  f.gv = a.vg[(dim + 1) % 3];
+  f.gw = a.vg[(dim + 2) % 3];
+  f.has_v = (dim + 1) % 3 < a.rank;
+  f.has_w = (dim + 2) % 3 < a.rank;
+  return f;
+}
+template <bool DUAL>
+__device__ __forceinline__ bool cfl_candidate(const CflFilter& f, const SweepArgs& a,
+                                              const Cell& o, const Phys& P) {
+  if (!f.on) return true;
+  const double ge = DUAL ? o.ge : o.e - 0.5 * (o.u * o.u + o.v * o.v + o.w * o.w);
+  double p = dmax(P.gm1 * o.d * ge, P.pmin);
+  p = dmax(p, a.min_support * P.gm1 * o.d * o.d);
+  const double gp = P.gamma * p;
+  const double cs = gp * fm_rsqrt_approx(gp * o.d);
+  double S = (cs + fabs(o.u - f.gu)) * f.ix;
+  if (f.has_v) S += (cs + fabs(o.v - f.gv)) * f.i1;
+  if (f.has_w) S += (cs + fabs(o.w - f.gw)) * f.i2;
+  const int hi = __double2hiint(S), top = *(volatile int*)f.best;
+  if (hi > top && hi < 0x7FF00000) atomicMax(f.best, hi);
+  return hi >= top - kCflMargin;  // infinities and positive NaN included
+}
+
+// The smallest dt1 of stored cells c0 .. c1 of a pencil: for the pencils of a block in which
+// another one was flagged, whose cells may have set the block's best and then dropped out.
+template <bool DUAL>
+__device__ __noinline__ double stored_dt1(const SweepArgs& a, int pid, int c0, int c1) {
+  const Phys P = make_phys(a);
+  const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
+  double best = 1.0e20;
+  if (t1 < a.ts1 || t1 > a.te1 || t2 < a.ts2 || t2 > a.te2) return best;
+  for (int c = c0 > a.is ? c0 : a.is; c <= c1 && c <= a.ie; ++c) {
+    const int64_t off = (int64_t)t1 * a.s1 + t2 * a.s2 + c * a.sa;
+    const Cell o = {a.out_d[off], a.out_e[off], a.out_u ? a.out_u[off] : 0.0,
+                    a.out_v ? a.out_v[off] : 0.0, a.out_w ? a.out_w[off] : 0.0,
+                    DUAL ? a.out_ge[off] : 0.0};
+    best = dmin(best, cell_dt1<DUAL>(a, o, a.coef[c].dx, t1, t2, P));
+  }
+  return best;
+}
+
 // Output staging of the x sweep.  Its pencils run along the contiguous axis, so a warp
 // storing one cell per pencil writes 32 separate sectors; instead every thread stores
 // its cells into shared memory, and every kStageCells cells each warp writes out its
@@ -1496,12 +1559,14 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
                                               UpdateCounts& cnt, int c0, int c1,
                                               bool valid = true,
                                               double* stage = nullptr, int pid0 = 0,
-                                              double* ring = nullptr, XTiles* xt = nullptr) {
+                                              double* ring = nullptr, XTiles* xt = nullptr,
+                                              int* best = nullptr) {
   bool live = valid, flagged = false;
   const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
   const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
   // the pencil's cells are active across the sweep (calc_dt covers active cells only)
   const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
+  const CflFilter flt = cfl_filter(a, t1, t2, best);
   double dtmin = 1.0e20;
   const int sa = (int)a.sa, np = (int)a.npencils;
   const double qdx = P.dt / a.uc.dx;  // dt/dx of every cell (a.uniform)
@@ -1671,7 +1736,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
           dep = o.d * o.e;
         }
         if (!isfinite(o.d) || !isfinite(o.e)) nonfin += 1;
-        if (cfl && (ST || (c >= is && c <= ie)))
+        if (cfl && (ST || (c >= is && c <= ie)) && cfl_candidate<DUAL>(flt, a, o, P))
           dtmin = dmin(dtmin, cell_dt1<DUAL>(a, o, a.uniform ? a.uc.dx : a.coef[c].dx, t1, t2, P));
         if (STAGED && PPM_X_STAGE_STORES) {
           double* sp = stage + (c % kStageCells) * kStageLd + (threadIdx.x & 31);
@@ -1797,15 +1862,19 @@ constexpr size_t update_smem_bytes() {
 
 // The end of an update or transport block: flagged pencils onto the fallback list (their
 // counts and time step come from the fallback pass), the other threads' counts and the
-// block's smallest time step.  first: the thread of its pencil that lists it.
+// block's smallest time step.  held: this thread holds cells c0 .. c1 of pencil pid.
+// FILTER: the block's cells went through the CflFilter.
+template <bool DUAL, bool FILTER>
 __device__ __forceinline__ void finish_block(const BatchArgs& B, const SweepArgs& a, int g,
-                                             int pid, bool first, const unsigned char* s_flag,
-                                             int pl, unsigned long long* s_cnt,
+                                             int pid, int c0, int c1, bool held,
+                                             const unsigned char* s_flag, int pl,
+                                             unsigned long long* s_cnt,
                                              const UpdateCounts& cnt) {
   double my_dt = 1.0e20;
   __syncthreads();
+  const bool any = FILTER && __syncthreads_or(s_flag[threadIdx.x]) != 0;
   if (s_flag[pl]) {
-    if (first) {
+    if (held && c0 == 0) {
       const unsigned long long slot = atomicAdd(&B.counters[kCntFlagged], 1ull);
       B.flagged[slot] = ((int64_t)g << 40) | pid;
     }
@@ -1813,6 +1882,7 @@ __device__ __forceinline__ void finish_block(const BatchArgs& B, const SweepArgs
     if (cnt.fatal) atomicAdd(&s_cnt[0], (unsigned long long)cnt.fatal);
     if (cnt.nonfinite) atomicAdd(&s_cnt[1], (unsigned long long)cnt.nonfinite);
     my_dt = cnt.dtmin;
+    if (FILTER && any && held && a.cfl_min_bits) my_dt = stored_dt1<DUAL>(a, pid, c0, c1);
   }
   if (a.cfl_min_bits) {  // warp minimum, one atomic per warp (every lane reaches this)
 #pragma unroll
@@ -1840,6 +1910,7 @@ __global__ void __launch_bounds__(kMarchThreads,
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
   __shared__ unsigned long long s_cnt[2];
   __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
+  __shared__ int s_best;                           // see CflFilter
   __shared__ uint64_t s_xbar[XT ? (kMarchThreads / 32) * kXBuffers : 1];
   extern __shared__ __align__(128) double s_dyn[];
   double* const s_xtile = s_dyn;                                // XT: kXWarp per warp
@@ -1847,6 +1918,7 @@ __global__ void __launch_bounds__(kMarchThreads,
   double* const s_ring = s_dyn;                                 // y, z: the input ring
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
   s_flag[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_best = 0;
   int64_t lb;
   const int g = locate<ONE>(B.upd_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
@@ -1871,10 +1943,10 @@ __global__ void __launch_bounds__(kMarchThreads,
     const Phys P = make_phys(a);
     if (update_pencil<DUAL, GRAV, false, STAGED, update_pipe<ONE, STAGED>(), XT, RS>(
             a, pid, P, cnt, c0, c1, valid, s_stage + warp * kStageWarp, wpid0,
-            s_ring + threadIdx.x, &xt))
+            s_ring + threadIdx.x, &xt, &s_best))
       s_flag[pl] = 1;
   }
-  finish_block(B, a, g, pid, valid && c0 == 0, s_flag, pl, s_cnt, cnt);
+  finish_block<DUAL, false>(B, a, g, pid, c0, c1, valid && c0 < a.n, s_flag, pl, s_cnt, cnt);
 }
 
 // The transport path's planes of one pencil made the fallback pass's: its advected states,
@@ -1959,12 +2031,13 @@ template <bool DUAL, bool GRAV, bool COR, bool STAGED, int PD, bool XT>
 __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, const Phys& P,
                                                  UpdateCounts& cnt, int c0, int c1, bool valid,
                                                  double* stage, int pid0, double* ring,
-                                                 XTiles* xt) {
+                                                 XTiles* xt, int* best) {
   constexpr int NV = DUAL ? 3 : 2;
   bool live = valid, flagged = false, handed = false;
   const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
   const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
   const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
+  const CflFilter flt = cfl_filter(a, t1, t2, best);
   double dtmin = 1.0e20;
   const int sa = (int)a.sa, np = (int)a.npencils;
   const int n = a.n, is = a.is, ie = a.ie;
@@ -2193,7 +2266,7 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
           dep = o.d * o.e;
         }
         if (!isfinite(o.d) || !isfinite(o.e)) nonfin += 1;
-        if (cfl && (ST || (k >= is && k <= ie)))
+        if (cfl && (ST || (k >= is && k <= ie)) && cfl_candidate<DUAL>(flt, a, o, P))
           dtmin = dmin(dtmin, cell_dt1<DUAL>(a, o, COR && !a.uniform ? a.coef[k].dx : a.uc.dx,
                                              t1, t2, P));
         store(k, o);
@@ -2305,12 +2378,14 @@ __global__ void __launch_bounds__(kMarchThreads,
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
   __shared__ unsigned long long s_cnt[2];
   __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
+  __shared__ int s_best;                           // see CflFilter
   __shared__ uint64_t s_xbar[XT ? (kMarchThreads / 32) * kXBuffers : 1];
   extern __shared__ __align__(128) double s_dyn[];
   double* const s_stage = s_dyn + (XT ? kTransXBlock : 0);
   double* const s_ring = s_stage + (STAGED ? kStageBlock : 0);
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
   s_flag[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_best = 0;
   int64_t lb;
   const int g = locate<ONE>(B.upd_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
@@ -2333,10 +2408,10 @@ __global__ void __launch_bounds__(kMarchThreads,
     const Phys P = make_phys(a);
     if (transport_pencil<DUAL, GRAV, COR, STAGED, PPM_TRANS_PIPE, XT>(
             a, pid, P, cnt, c0, c1, valid, s_stage + warp * kStageWarp, wpid0,
-            s_ring + threadIdx.x, &xt))
+            s_ring + threadIdx.x, &xt, &s_best))
       s_flag[pl] = 1;
   }
-  finish_block(B, a, g, pid, valid && c0 == 0, s_flag, pl, s_cnt, cnt);
+  finish_block<DUAL, true>(B, a, g, pid, c0, c1, valid && c0 < a.n, s_flag, pl, s_cnt, cnt);
 }
 
 // ------------------------------------------------------------------ stage 5 (colours)
