@@ -130,16 +130,22 @@ __device__ __forceinline__ void load_face_advected(const SweepArgs& a, int64_t i
 // Slope-correction coefficients of every cell is-1 .. ie+1 of a pencil: calcdiss's
 // flattening (calcdiss.F:213-224 with type 1 :407-438 or type 3 :486-564) from the
 // sweep's pressure, velocity, density and total energy, and inteuler's density
-// steepening (inteuler.F:166-193).  Thread per pencil, marching; the flattening's
-// flattemp values are computed once each and kept for the max of eq. A2.
+// steepening (inteuler.F:166-193).  A thread marches a segment of a pencil (the
+// reconstruction's split: on whole pencils a 96^3 sweep's 82 blocks took 0.23 ms); the
+// flattening's flattemp values are computed once each and kept for the max of eq. A2.
 template <bool ONE>
 __global__ void __launch_bounds__(kMarchThreads) corrections_kernel(const __grid_constant__ BatchArgs B) {
   pdl_begin();
   int64_t lb;
-  const int g = locate<ONE>(B.march_prefix, B.ngrids, lb);
+  const int g = locate<ONE>(B.seg_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
-  const int64_t pid = lb * kMarchThreads + threadIdx.x;
-  if (pid >= a.npencils) return;
+  // cells first .. last of this thread's segment (the reconstruction's split)
+  const int64_t pid = (lb << a.pw_log2) + (threadIdx.x & ((1 << a.pw_log2) - 1));
+  const int segs = kMarchThreads >> a.pw_log2, cells = a.ie - a.is + 3;
+  const int per = (cells + segs - 1) / segs;
+  const int first = a.is - 1 + (int)(threadIdx.x >> a.pw_log2) * per;
+  if (pid >= a.npencils || first > a.ie + 1) return;
+  const int last = first + per - 1 < a.ie + 1 ? first + per - 1 : a.ie + 1;
   const int64_t base = (pid % a.n1) * a.s1 + (pid / a.n1) * a.s2;
   const int64_t sa = a.sa, np = a.npencils;
   const int is = a.is, ie = a.ie;
@@ -169,10 +175,10 @@ __global__ void __launch_bounds__(kMarchThreads) corrections_kernel(const __grid
   };
   double fm = 0.0, f0 = 0.0;
   if (a.flatten) {
-    fm = ftemp(is - 2);
-    f0 = ftemp(is - 1);
+    fm = ftemp(first - 1);
+    f0 = ftemp(first);
   }
-  for (int c = is - 1; c <= ie + 1; ++c) {
+  for (int c = first; c <= last; ++c) {
     const int64_t o = (int64_t)(c - (is - 1)) * np + pid;
     if (a.flatten) {  // eq. A2: the max with the neighbour on the high-pressure side
       const double fp = ftemp(c + 1);
@@ -2443,31 +2449,54 @@ __global__ void __launch_bounds__(kMarchThreads,
 constexpr double kColourFloor = 1.0e-35;        // color_floor, fortran.def:8
 constexpr double kMinColour = 1.0e-5 * kTiny;   // min_color, euler.F:104-105
 
-// CPT colours per thread: each thread marches one pencil for colours c0 .. c0+CPT-1 of
-// its block's chunk, sharing the cell and face data between them.
-template <bool DUAL, bool ONE, int CPT>
+// CPT colours per thread: each thread marches one pencil segment (cells k0 .. k1, faces
+// k0 .. k1+1) for colours c0 .. c0+CPT-1 of its block's chunk, sharing the cell and face
+// data between them.  The update is in place, and a segment reads three cells of each
+// neighbour: a block holds every segment of its pencils, and each thread copies those six
+// into shared memory before any of them writes.
+// UNI: one cell width along the sweep (see pm_slope and pm_parabola).
+// 96^3 with nine colours, tolerance build: 0.71 ms a sweep on whole pencils (738 blocks, a
+// wave and a quarter of serial marches), 0.34 in segments with the tolerance build's
+// shared factors.
+template <bool DUAL, bool ONE, int CPT, bool UNI>
 __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
     colour_kernel(const __grid_constant__ BatchArgs B) {
   pdl_begin();
+  __shared__ double s_halo[6 * CPT][kMarchThreads];  // cells k0-3 .. k0-1, k1+1 .. k1+3
   const int nc = B.ncolour;
   const int nchunk = (nc + CPT - 1) / CPT;
   const int64_t mb = blockIdx.x / nchunk;
   const int chunk = (int)(blockIdx.x - mb * nchunk);
   int64_t lb = mb;
-  const int g = ONE ? 0 : batch_locate(B.march_prefix, B.ngrids, mb, lb);
+  const int g = ONE ? 0 : batch_locate(B.seg_prefix, B.ngrids, mb, lb);
   PPM_BIND_RECORD(a, g)
-  const int64_t pid = lb * kMarchThreads + threadIdx.x;
-  if (pid >= a.npencils) return;
-  const Phys P = make_phys(a);
-  const int64_t base = (pid % a.n1) * a.s1 + (pid / a.n1) * a.s2;
-  const int64_t sa = a.sa;
+  const int pid = (int)(lb << a.pw_log2) + (threadIdx.x & ((1 << a.pw_log2) - 1));
   const int is = a.is, ie = a.ie;
-  const int64_t np = a.npencils, plane = a.plane;
+  const int segs = kMarchThreads >> a.pw_log2, per = (ie - is + segs) / segs;
+  const int k0 = is + (int)(threadIdx.x >> a.pw_log2) * per;
+  const int k1 = k0 + per - 1 < ie ? k0 + per - 1 : ie;
+  const bool mine = pid < a.npencils && k0 <= ie;
+  const int sa = (int)a.sa;
+  const int base = mine ? pencil_base(a, pid) : 0;
   const int c0 = chunk * CPT;
   const int ncol = nc - c0 < CPT ? nc - c0 : CPT;  // colours of this chunk
   double* q[CPT];
 #pragma unroll
   for (int u = 0; u < CPT; ++u) q[u] = u < ncol ? a.col[c0 + u] : nullptr;
+  if (mine && segs > 1) {
+#pragma unroll
+    for (int u = 0; u < CPT; ++u)
+      if (u < ncol)
+        for (int k = 0; k < 3; ++k) {
+          s_halo[6 * u + k][threadIdx.x] = q[u][base + (k0 - 3 + k) * sa];
+          s_halo[6 * u + 3 + k][threadIdx.x] = q[u][base + (k1 + 1 + k) * sa];
+        }
+  }
+  if (segs > 1) __syncthreads();
+  if (!mine) return;
+  const Phys P = make_phys(a);
+  const int np = (int)a.npencils;
+  const int64_t plane = a.plane;
 
   int64_t cap = 0, cap_end = 0;
   if (a.ncaptures > 0) {
@@ -2478,6 +2507,7 @@ __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
     }
     cap = cap_end = lo;
     while (cap_end < a.ncaptures && a.captures[cap_end].pencil == pid) ++cap_end;
+    while (cap < cap_end && a.captures[cap].face < k0) ++cap;
   }
 
   double wq0[CPT], wq1[CPT], wq2[CPT];  // colour of cells t-3, t-2, t-1
@@ -2489,47 +2519,56 @@ __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
     wq0[u] = wq1[u] = wq2[u] = dqm1[u] = qlm1[u] = colla[u] = coll0[u] = fm[u] = 0.0;
   double wu0 = 0.0, wu1 = 0.0, wu2 = 0.0;  // normal velocity of cells t-3, t-2, t-1
   Prep prA = {0, 0, 0, 0, 0}, prB = {0, 0, 0, 0, 0};  // cells t-2, t-1
-  const int tend = ie + 3;
 #pragma unroll 1
-  for (int t = 0; t <= tend; ++t) {
-    const int64_t off = base + (int64_t)t * sa;
+  for (int t = k0 - 3; t <= k1 + 3; ++t) {
+    const int off = base + t * sa;
     double nq[CPT];
 #pragma unroll
-    for (int u = 0; u < CPT; ++u) nq[u] = u < ncol ? q[u][off] : 0.0;
+    for (int u = 0; u < CPT; ++u) {
+      nq[u] = 0.0;
+      if (u < ncol) {
+        if (segs > 1 && t < k0)
+          nq[u] = s_halo[6 * u + t - k0 + 3][threadIdx.x];
+        else if (segs > 1 && t > k1)
+          nq[u] = s_halo[6 * u + 2 + t - k1][threadIdx.x];
+        else
+          nq[u] = q[u][off];
+      }
+    }
     const double nu = ldg0(a.in_u, off);
     Prep prC = prB;
-    if (t >= is - 1 && t <= ie + 1)
-      prC = a.presfree ? cell_prep<true>(__ldg(a.in_d + off), __ldg(a.pres + off), nu,
-                                         a.coef[t].dx2i, P)
-                       : cell_prep(__ldg(a.in_d + off), __ldg(a.pres + off), nu,
-                                   a.coef[t].dx2i, P);
+    if (t >= k0 - 1 && t <= k1 + 1) {
+      const double dx2i = UNI ? a.uc.dx2i : a.coef[t].dx2i;
+      prC = a.presfree ? cell_prep<true>(__ldg(a.in_d + off), __ldg(a.pres + off), nu, dx2i, P)
+                       : cell_prep(__ldg(a.in_d + off), __ldg(a.pres + off), nu, dx2i, P);
+    }
     double dqN[CPT], qlN[CPT];  // slope and left edge of cell t-1
 #pragma unroll
     for (int u = 0; u < CPT; ++u) dqN[u] = qlN[u] = 0.0;
     {
       const int c = t - 1;
-      if (c >= is - 2 && c <= ie + 2) {
-        const Coef cf = a.coef[c];
+      if (c >= k0 - 2 && c <= k1 + 2) {
+        const Coef& cf = UNI ? a.uc : a.coef[c];
 #pragma unroll
         for (int u = 0; u < CPT; ++u) {
-          dqN[u] = pm_slope(wq1[u], wq2[u], nq[u], cf.c1, cf.c2);
-          if (c >= is - 1) qlN[u] = pm_edge(wq1[u], wq2[u], dqm1[u], dqN[u], cf.c3, cf.c4, cf.c5, cf.c6);
+          dqN[u] = pm_slope<UNI>(wq1[u], wq2[u], nq[u], cf.c1, cf.c2);
+          if (c >= k0 - 1) qlN[u] = pm_edge(wq1[u], wq2[u], dqm1[u], dqN[u], cf.c3, cf.c4, cf.c5, cf.c6);
         }
       }
     }
     {
       const int c = t - 2;  // parabola of cell c; face c
-      if (c >= is - 1 && c <= ie + 1) {
-        const double fl = a.flatten != 0 ? a.flat[(int64_t)(c - (is - 1)) * np + pid] : 0.0;
+      if (c >= k0 - 1 && c <= k1 + 1) {
+        const double fl = a.flatten != 0 ? a.flat[(c - (is - 1)) * np + pid] : 0.0;
         Para pa[CPT];
 #pragma unroll
         for (int u = 0; u < CPT; ++u)
           pa[u] = a.flatten != 0
                       ? pm_parabola<false, true>(wq0[u], wq1[u], wq2[u], qlm1[u], qlN[u], 0.0,
                                                  0.0, 0.0, fl)
-                      : pm_parabola(wq0[u], wq1[u], wq2[u], qlm1[u], qlN[u]);
-        if (c >= is) {
-          const int64_t fidx = (int64_t)(c - is) * np + pid;
+                      : pm_parabola<false, false, UNI>(wq0[u], wq1[u], wq2[u], qlm1[u], qlN[u]);
+        if (c >= k0) {
+          const int fidx = (c - is) * np + pid;
           const double* fc = a.fcol + fidx;
           const double dla = fc[CDLA * plane], dl0 = fc[CDL0 * plane];
           const double dra = fc[CDRA * plane], dr0 = fc[CDR0 * plane];
@@ -2550,12 +2589,28 @@ __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
             if (ub > 0.0) dsl = a.fstate[SDL * plane + fidx];
             else dsr = a.fstate[SDR * plane + fidx];
           }
-          const double dx = a.coef[c].dx;
+          const double dx = UNI ? a.uc.dx : a.coef[c].dx;
+#if PPM_FAST_ALGEBRA
+          // tolerance mode: every colour's scale factors of the face once (the quotients
+          // below have the same factors for all of them)
+          const bool la = wu0 <= 0.0, ra = wu1 >= 0.0;
+          double fl_s = dlc * qrcp(la ? dla : dl0), fr_s = drc * qrcp(ra ? dra : dr0);
+          if (ovl) fl_s *= dla * qrcp(dlc);
+          if (ovr) fr_s *= dra * qrcp(drc);
+          const double qx = qdiv(P.dt, dx);
+          const double gl_s = qx * ub * db * qrcp(ub > 0.0 ? dsl : dsr);
+#endif
           int64_t cq = cap;  // this face's capture requests (the same for every colour)
 #pragma unroll
           for (int u = 0; u < CPT; ++u) {
             if (u >= ncol) break;
             const double colra = pm_C(pa[u], prA.char2), colr0 = pm_B(pa[u], prA.c0);
+#if PPM_FAST_ALGEBRA
+            const double cls = dmax((la ? colla[u] : coll0[u]) * fl_s, kColourFloor);
+            const double crs = dmax((ra ? colra : colr0) * fr_s, kColourFloor);
+            const double cf = hll ? qx * (w[0] * (w[1] * cls) + w[2] * (w[3] * crs))
+                                  : gl_s * (ub > 0.0 ? cls : crs);
+#else
             double cls = (wu0 <= 0.0) ? colla[u] * dlc / dla : coll0[u] * dlc / dl0;
             double crs = (wu1 >= 0.0) ? colra * drc / dra : colr0 * drc / dr0;
             if (ovl) cls = cls * dla / dlc;
@@ -2571,19 +2626,21 @@ __global__ void __launch_bounds__(kMarchThreads, PPM_COLOUR_MINBLOCKS)
               cf = P.dt * ub * colb;
             }
             cf = cf / dx;
-            for (cq = cap; cq < cap_end && a.captures[cq].face <= c; ++cq) {
+#endif
+            // capture: the segment's own faces k0 .. k1, and ie+1 by the last one
+            for (cq = cap; cq < cap_end && (c <= k1 || k1 == ie) && a.captures[cq].face <= c; ++cq) {
               const FluxCapture& rq = a.captures[cq];
               if (rq.face == c) a.col_capture[(rq.dst / 6) * nc + c0 + u] = cf;
             }
-            if (c - 1 >= is && c - 1 <= ie) {
+            if (c > k0) {
               const double v = wq0[u] + (fm[u] - cf);
-              q[u][base + (int64_t)(c - 1) * sa] = dmax(v, kMinColour);
+              q[u][base + (c - 1) * sa] = dmax(v, kMinColour);
             }
             fm[u] = cf;
           }
           cap = cq;
         }
-        if (c <= ie) {
+        if (c <= k1) {
 #pragma unroll
           for (int u = 0; u < CPT; ++u) {
             colla[u] = pm_A(pa[u], prA.char1);
@@ -2679,6 +2736,22 @@ void launch_riemann_plain(const BatchArgs& B, unsigned rb, cudaStream_t st) {
     launch_riemann_rt<DUAL, ONE, STATE, kRiemannThreads>(B, rb, st);
 }
 
+template <bool DUAL, bool ONE>
+void launch_colours(const BatchArgs& B, cudaStream_t st) {
+  constexpr int cpt = PPM_COLOURS_PER_THREAD;
+  const int64_t chunks = (B.ncolour + cpt - 1) / cpt;
+  const bool wide = B.seg_blocks * B.ncolour >= PPM_COLOUR_WIDE_BLOCKS;
+  const int64_t blocks = B.seg_blocks * (wide ? chunks : B.ncolour);
+  if (wide && !B.uneven)
+    launch_chain(colour_kernel<DUAL, ONE, cpt, true>, blocks, kMarchThreads, 0, st, B);
+  else if (wide)
+    launch_chain(colour_kernel<DUAL, ONE, cpt, false>, blocks, kMarchThreads, 0, st, B);
+  else if (!B.uneven)
+    launch_chain(colour_kernel<DUAL, ONE, 1, true>, blocks, kMarchThreads, 0, st, B);
+  else
+    launch_chain(colour_kernel<DUAL, ONE, 1, false>, blocks, kMarchThreads, 0, st, B);
+}
+
 template <bool DUAL, bool GRAV, bool ONE>
 void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
                    cudaStream_t st, cudaEvent_t* ev, bool learned, bool staged) {
@@ -2691,7 +2764,7 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     const bool cor = B.corrections || B.uneven;
     const unsigned rb = (unsigned)riemann_blocks;
     if (B.corrections)
-      launch_chain(corrections_kernel<ONE>, march_blocks, kMarchThreads, 0, st, B);
+      launch_chain(corrections_kernel<ONE>, sb, kMarchThreads, 0, st, B);
     if (cor)
       launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads, 0, st, B);
     else
@@ -2746,7 +2819,7 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
   }
   if (B.ncolour > 0) cudaMemsetAsync(B.hll_flags, 0, (size_t)B.hll_bytes, st);
   const bool cor = B.corrections || B.ncolour > 0 || B.presfree || B.uneven;
-  if (B.corrections) launch_chain(corrections_kernel<ONE>, march_blocks, kMarchThreads, 0, st, B);
+  if (B.corrections) launch_chain(corrections_kernel<ONE>, sb, kMarchThreads, 0, st, B);
   if (B.both_roles) {
     launch_chain(clear_sweep_kernel, 1, 1, 0, st, B);
     mark(1);
@@ -2813,13 +2886,7 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     launch_chain(fallback_kernel<DUAL, GRAV, ONE>, 64, 128, 0, st, B);
   }
   if (B.ncolour > 0) {
-    constexpr int cpt = PPM_COLOURS_PER_THREAD;
-    const int64_t chunks = (B.ncolour + cpt - 1) / cpt;
-    if (march_blocks * B.ncolour < PPM_COLOUR_WIDE_BLOCKS)
-      launch_chain(colour_kernel<DUAL, ONE, 1>, march_blocks * B.ncolour, kMarchThreads, 0, st,
-                   B);
-    else
-      launch_chain(colour_kernel<DUAL, ONE, cpt>, march_blocks * chunks, kMarchThreads, 0, st, B);
+    launch_colours<DUAL, ONE>(B, st);
   }
   mark(5);
 }

@@ -65,6 +65,21 @@ def test_dual_energy_select_parameters(ctx, eta1, eta2):
     _steps(ctx, g, hp, random_state(g, hp, seed=9, mach=8.0))
 
 
+# colours are updated in place by the segments of a pencil; flattening and steepening
+# coefficients come in the same split
+@pytest.mark.parametrize("shape,ncol", [((9,), 1), ((130,), 3), ((40, 37), 2), ((17, 33, 20), 5)])
+@pytest.mark.parametrize("flatten,steepen", [(0, 0), (3, 1)])
+def test_colours_in_segments(ctx, shape, ncol, flatten, steepen):
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=True, flatten=flatten, steepen=steepen)
+    g = H.Grid.uniform(shape)
+    f = random_state(g, hp, seed=11)
+    rng = np.random.default_rng(12)
+    for n in range(ncol):
+        f[f"col{n}"] = f["d"] * (0.2 + 0.5 * rng.random(g.shape))
+    H.fill_ghosts(g, f, "periodic")
+    _steps(ctx, g, hp, f)
+
+
 # cell widths that differ along the sweep take the general reconstruction
 def test_uneven_cell_widths(ctx):
     hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.3, dual=True)
