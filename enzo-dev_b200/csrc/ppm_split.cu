@@ -1509,12 +1509,13 @@ __device__ __noinline__ double stored_dt1(const SweepArgs& a, int pid, int c0, i
 // its cells into shared memory, and every kStageCells cells each warp writes out its
 // 32 pencils' cells with consecutive lanes on consecutive cells of a pencil (warp-local:
 // no block barrier).  Layout per warp [field][cell][lane], the cell row padded
-// (kStageLd) so that the flush reads hit distinct banks.
+// (kStageLd) so that the flush reads hit distinct banks: a half warp reads 4 lanes of each of
+// 4 cells, 8 banks apart with rows of 36.
 #ifndef PPM_X_STAGE_STORES
 #define PPM_X_STAGE_STORES 1
 #endif
 #ifndef PPM_STAGE_LD
-#define PPM_STAGE_LD (32 + 8)
+#define PPM_STAGE_LD (32 + 4)
 #endif
 #ifndef PPM_STAGE_CELLS
 #define PPM_STAGE_CELLS 4
