@@ -1,0 +1,41 @@
+"""Host-memory calls: pageable fields go through the context's pinned pieces (threads above
+4 MB a call), pinned fields directly; the fields are the device call's either way."""
+import numpy as np
+import pytest
+
+from ppm_b200 import capi
+from ppm_b200 import harness as H
+from parity_util import random_state
+
+pytestmark = pytest.mark.gpu
+
+
+# below and above the size worth the threads, pieces with ragged ends, more than the staging
+# memory holds at once (64 MiB), colours
+@pytest.mark.parametrize("shape,ncol", [((20, 18, 16), 0), ((40, 41, 43), 0), ((64, 64, 64), 3),
+                                        ((120, 121, 122), 0)])
+@pytest.mark.parametrize("grav", [False, True])
+def test_pageable_pinned_and_device_fields_agree(shape, ncol, grav):
+    torch = pytest.importorskip("torch")
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=True, gravity=grav)
+    g = H.Grid.uniform(shape)
+    f = random_state(g, hp, seed=4)
+    rng = np.random.default_rng(1)
+    for n in range(ncol):
+        f[f"col{n}"] = f["d"] * (0.1 + rng.random(g.shape))
+    acc = [0.1 * rng.standard_normal(g.shape) for _ in range(3)] if grav else None
+    c = capi.Context(0)
+    dev = {k: torch.from_numpy(v).cuda() for k, v in f.items()}
+    acc_dev = [torch.from_numpy(a).cuda() for a in acc] if grav else None
+    host = {k: v.copy() for k, v in f.items()}
+    pinned = {k: torch.from_numpy(v.copy()).pin_memory() for k, v in f.items()}
+    pinned_np = {k: v.numpy() for k, v in pinned.items()}
+    for cyc in range(2):
+        c.solve_ppm_de(g, hp, 1e-3, cyc, dev, memory=capi.MEM_DEVICE, accel=acc_dev)
+        c.solve_ppm_de(g, hp, 1e-3, cyc, host, accel=acc)
+        c.solve_ppm_de(g, hp, 1e-3, cyc, pinned_np, accel=acc)
+        for k in f:
+            ref = dev[k].cpu().numpy()
+            assert np.array_equal(host[k], ref), (cyc, k)
+            assert np.array_equal(pinned_np[k], ref), (cyc, k)
+    c.close()
