@@ -17,6 +17,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -68,7 +69,7 @@ def build(force: bool = False, verbose: bool = False, variant: str = "exact") ->
     obj_dir.mkdir(parents=True, exist_ok=True)
     headers = list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
     newest_header = max(p.stat().st_mtime for p in headers)
-    objs = []
+    objs, cmds = [], []
     for src in SOURCES:
         obj = obj_dir / (Path(src).stem + ".o")
         stale = (force or not obj.exists() or obj.stat().st_mtime < newest_header
@@ -78,8 +79,10 @@ def build(force: bool = False, verbose: bool = False, variant: str = "exact") ->
                    "-c", str(CSRC / src), "-o", str(obj)]
             if verbose:
                 cmd += ["-Xptxas", "-v"]
-            subprocess.run(cmd, check=True)
+            cmds.append(cmd)
         objs.append(str(obj))
+    with ThreadPoolExecutor(len(SOURCES)) as pool:
+        list(pool.map(lambda c: subprocess.run(c, check=True), cmds))
     tmp = lib.with_suffix(".so.tmp")
     subprocess.run([nvcc(), *ARCH, "-shared", "-o", str(tmp), *objs, "-lcudart",
                     "-Xlinker", f"--version-script={EXPORTS_MAP}"], check=True)
@@ -88,7 +91,8 @@ def build(force: bool = False, verbose: bool = False, variant: str = "exact") ->
 
 
 def build_all(force: bool = False, verbose: bool = False) -> list:
-    return [build(force, verbose, name) for name in VARIANTS]
+    with ThreadPoolExecutor(len(VARIANTS)) as pool:
+        return list(pool.map(lambda name: build(force, verbose, name), VARIANTS))
 
 
 if __name__ == "__main__":
