@@ -939,7 +939,7 @@ def run_ours(args):
     cells = g.active_cells
     value = cells * world * args.steps / (ms * 1e-3)
 
-    # roofline of the dominant unit, one directional sweep (its five kernels, timed with
+    # roofline of the dominant unit, one directional sweep (its kernels, timed with
     # events on the launching stream): algorithmic bytes per sweep = 104 B per active
     # cell (every field read once and written once), over its average duration
     peak, peak_src = measured_peak_hbm()
@@ -948,7 +948,7 @@ def run_ours(args):
     tr, tr_src = committed_traffic(variant)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": (tr * cells if tr else None),
-                "kernel": "directional sweep (reconstruct x2, riemann, update, fallback)",
+                "kernel": "directional sweep (reconstruct, riemann, transport or update, fallback)",
                 "avg_launch_ms": avg_sweep_s * 1e3,
                 "stage_ms_per_sweep": {k: v / max(nsweep, 1) for k, v in stages.items()},
                 "sweep_share_of_step": sweep_ms / ms, "peak_source": peak_src,

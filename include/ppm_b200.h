@@ -382,8 +382,11 @@ long long ppm_b200_launch_count(ppm_b200_context *ctx);
    and the number of timed sweep launches since the last read, and resets them. */
 int ppm_b200_profile(ppm_b200_context *ctx, int enable);
 int ppm_b200_profile_read(ppm_b200_context *ctx, double *sweep_ms, long long *sweep_launches);
-/* Per-kernel split of the last ppm_b200_profile_read: summed ms of the five kernels of
-   a sweep (reconstruct d/p/u, reconstruct v/w/ge, Riemann, update, HLL fallback pass). */
+/* Per-stage split of the last ppm_b200_profile_read: summed ms of the stages of a sweep
+   (reconstruct d/p/u, reconstruct v/w/ge, Riemann, update, HLL fallback pass).  On large
+   two-shock batches one transport kernel reconstructs v/w/ge and updates: its time is the
+   update's and the second entry is empty.  On small batches both reconstructions are one
+   launch, in the second entry. */
 int ppm_b200_profile_stages(ppm_b200_context *ctx, double stage_ms[5]);
 
 /* grid::ComovingExpansionTerms for PPM (Grid_ComovingExpansionTerms.C:36-99 with
