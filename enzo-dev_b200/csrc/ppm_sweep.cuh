@@ -347,9 +347,8 @@ inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select,
 
 // The record's shared coefficients, from its coefficient table on the host.
 inline void set_uniform(SweepArgs& a, const double* width, const Coef* table) {
-  a.uniform = 1;
-  for (int i = 1; i < a.n; ++i)
-    if (std::memcmp(&width[i], &width[0], sizeof(double)) != 0) a.uniform = 0;
+  // every width equal to the next: one comparison (a level prepares hundreds of grids)
+  a.uniform = a.n < 2 || std::memcmp(width, width + 1, (size_t)(a.n - 1) * sizeof(double)) == 0;
   a.uc = table[a.is];
 }
 
