@@ -2224,7 +2224,10 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
       double ges = 0.0;
       if (DUAL) {
         const double pcent = dmax(P.gm1 * C.ge * C.d, kTiny);
-        ges = (COR && !a.uniform ? P.dt / a.coef[c].dx : qdx) * pcent * (F0.ub - F1.ub);
+        // rounded, as update_pencil carries it from step to step: fused into the energy's sum
+        // it would give other bits than the separate kernels
+        ges = __dmul_rn(__dmul_rn(COR && !a.uniform ? P.dt / a.coef[c].dx : qdx, pcent),
+                        F0.ub - F1.ub);
       }
       if (C.d + (F0.df - F1.df) <= 0.0 || C.e < 0.0) {  // to the fallback pass
         if (!STAGED) {
