@@ -1444,17 +1444,21 @@ __device__ __forceinline__ double cell_dt1(const SweepArgs& a, const Cell& o, do
 // word of the double, with the largest estimate of the block's cells so far (best, shared
 // memory).  A cell more than 4 units of that word below it cannot be the smallest, so its
 // calc_dt (IEEE root and divisions, a sixth of the last sweep's update) is left out.  The
-// reciprocal widths are the pencil's (w1, w2 across the sweep).
+// reciprocal widths are the pencil's (w1, w2 across the sweep).  active: the pencil is
+// active across the sweep; only then are there widths to read (a staged warp's lanes past
+// the last pencil come here too, with t2 past the table's end).
 struct CflFilter {
   double ix, i1, i2, gu, gv, gw;
   int* best;
   bool on, has_v, has_w;
 };
 constexpr int kCflMargin = 16;  // units of the upper word: at least 7.6e-6, the estimate 2e-6
-__device__ __forceinline__ CflFilter cfl_filter(const SweepArgs& a, int t1, int t2, int* best) {
-  CflFilter f;
+__device__ __forceinline__ CflFilter cfl_filter(const SweepArgs& a, int t1, int t2, int* best,
+                                                bool active) {
+  CflFilter f = {};
+  f.on = active && best && a.uniform && a.aye > 0.0 && a.eos_type == 0 && !a.presfree;
+  if (!f.on) return f;
   const int dim = a.dim;
-  f.on = a.cfl_min_bits && best && a.uniform && a.aye > 0.0 && a.eos_type == 0 && !a.presfree;
   f.best = best;
   // the axes of (u, v, w): (x, y, z), (y, z, x), (z, x, y); of (t1, t2): (y, z), (x, z),
   // (x, y)
@@ -1573,7 +1577,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
   const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
   // the pencil's cells are active across the sweep (calc_dt covers active cells only)
   const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
-  const CflFilter flt = cfl_filter(a, t1, t2, best);
+  const CflFilter flt = cfl_filter(a, t1, t2, best, cfl);
   double dtmin = 1.0e20;
   const int sa = (int)a.sa, np = (int)a.npencils;
   const double qdx = P.dt / a.uc.dx;  // dt/dx of every cell (a.uniform)
@@ -2044,7 +2048,7 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
   const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
   const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
   const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
-  const CflFilter flt = cfl_filter(a, t1, t2, best);
+  const CflFilter flt = cfl_filter(a, t1, t2, best, cfl);
   double dtmin = 1.0e20;
   const int sa = (int)a.sa, np = (int)a.npencils;
   const int n = a.n, is = a.is, ie = a.ie;

@@ -30,6 +30,10 @@ def _dev(f, torch):
     ((20, 12, 10), True, False, True),
     ((24, 18), True, False, False),
     ((40,), False, False, False),
+    # x sweep staged with lanes past the last pencil (72 pencils of 32 a warp), which have no
+    # cell widths to read
+    ((16, 2, 3), True, False, False),
+    ((16, 2, 3), False, True, False),
 ])
 def test_folded_time_step_equals_calc_dt(torch, shape, dual, grav, fallback_cells):
     hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.45, dual=dual, gravity=grav)
