@@ -2327,8 +2327,9 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
   const int tlast = ce + 3;
   auto max2 = [](int x, int y) { return x > y ? x : y; };
   auto min2 = [](int x, int y) { return x < y ? x : y; };
-  // every range of a steady step, and of the steps it fetches for
-  const int s0 = max2(max2(fa + 2, is + 3), c0 + 4);
+  // every range of a steady step, and of the steps it fetches for (the cell it stores, t-4, is
+  // an active one: is + 4)
+  const int s0 = max2(max2(fa + 2, is + 4), c0 + 4);
   const int s1 = min2(min2(hi, fb + 2), min2(ie + 3, c1 + 3)) - PD;
 #pragma unroll 1
   for (int t = lo; t < s0 && t <= tlast; ++t) {
