@@ -40,15 +40,14 @@ def _heat_ghosts(g, f, hp):
 
 
 # cells with a negative total energy; without the dual-energy select they keep it through
-# every sweep of a step this small, so the last sweep flags their pencils too (the call then
-# reports the negative energy)
+# every sweep of a step this small, so the last sweep flags their pencils too
 def _bad_cells(g, f, torch, n=30):
     gen = torch.Generator().manual_seed(n)
     for _ in range(n):
         k, j, i = (int(torch.randint(3, s - 3, (1,), generator=gen)) if s > 6 else 0
                    for s in g.shape)
-        f["te"][k, j, i] = -1e-3
-    return n
+        f["te"][k, j, i] = -1.0
+    return int((f["te"] == -1.0).sum())
 
 
 # even and odd sides (TMA tiles and the ring in the x sweep), two dimensions; every sweep last
@@ -69,8 +68,7 @@ def test_single_grid(torch, variant, shape, dual, bad):
     ctx.set_cfl(nxt, courant=hp.cfl, **kw)
     for cyc in range(g.rank):
         fd = {k: torch.from_numpy(v.copy()).cuda() for k, v in f.items()}
-        rc, st = ctx.solve_ppm_de(g, hp, DT, cyc, fd, memory=capi.MEM_DEVICE, check=False)
-        assert rc == (capi.ERR_NEGATIVE if bad else capi.OK)
+        rc, st = ctx.solve_ppm_de(g, hp, DT, cyc, fd, memory=capi.MEM_DEVICE)
         assert st["fallbacks"] >= n * g.rank  # n in each sweep
         ref = ctx.compute_timestep(g, hp, fd, memory=capi.MEM_DEVICE, **kw)
         assert nxt.item() == ref, (cyc, nxt.item(), ref)
@@ -86,10 +84,10 @@ def test_level(torch, variant, graphs, dual, bad):
     grids = [H.Grid.uniform(s) for s in shapes]
     assert sum(g.size for g in grids) >= 750000
     host = [random_state(g, hp, seed=60 + k, mach=0.5) for k, g in enumerate(grids)]
+    n = 0
     for g, f in zip(grids, host):
         _heat_ghosts(g, f, hp)
-        if bad:
-            _bad_cells(g, f, torch, n=3)
+        n += _bad_cells(g, f, torch, n=3) if bad else 0
     ctx = capi.Context(0, variant=variant)
     ctx.set_graphs(graphs)
     dt = torch.zeros(1, dtype=torch.float64, device="cuda")
@@ -104,9 +102,8 @@ def test_level(torch, variant, graphs, dual, bad):
             for k in f:
                 f[k].copy_(torch.from_numpy(h[k]))
         torch.cuda.synchronize()
-        rc, _ = ctx.solve_level(grids, hp, 0.0, cyc, fs, dt_device=dt, want_stats=True,
-                                check=False)
-        assert rc == (capi.ERR_NEGATIVE if bad else capi.OK)
+        rc, st = ctx.solve_level(grids, hp, 0.0, cyc, fs, dt_device=dt, want_stats=True)
+        assert st["fallbacks"] >= 3 * n
         ref = ctx.compute_timestep_level(grids, hp, fs)
         assert nxt.item() == ref, (cyc, nxt.item(), ref)
     ctx.close()
