@@ -1442,8 +1442,12 @@ __device__ __forceinline__ double cell_dt1(const SweepArgs& a, const Cell& o, do
 // Whether a cell can hold the block's smallest dt1 = aye/S, S the sum of (cs + |v - vg|)/dx:
 // S is estimated to 20 bits (one approximate root, no division) and compared, by the upper
 // word of the double, with the largest estimate of the block's cells so far (best, shared
-// memory).  A cell more than 4 units of that word below it cannot be the smallest, so its
-// calc_dt (IEEE root and divisions, a sixth of the last sweep's update) is left out.  The
+// memory).  A cell more than kCflMargin units of that word below it cannot be the smallest, so its
+// calc_dt (IEEE root and divisions, a sixth of the last sweep's update) is left out.  A pencil
+// the fallback pass rewrites may have put a state into best that it no longer has, so a
+// block with such a pencil looks at its stored cells again (stored_dt1).  In the transport
+// kernel only: on small grids it costs more than it saves (update kernel with and without:
+// 24 patches 576 / 570 us a step, 37x24x53 with HLLC 175 / 169).  The
 // reciprocal widths are the pencil's (w1, w2 across the sweep).  active: the pencil is
 // active across the sweep; only then are there widths to read (a staged warp's lanes past
 // the last pencil come here too, with t2 past the table's end).
@@ -1570,14 +1574,12 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
                                               UpdateCounts& cnt, int c0, int c1,
                                               bool valid = true,
                                               double* stage = nullptr, int pid0 = 0,
-                                              double* ring = nullptr, XTiles* xt = nullptr,
-                                              int* best = nullptr) {
+                                              double* ring = nullptr, XTiles* xt = nullptr) {
   bool live = valid, flagged = false;
   const int t2 = pid / a.n1, t1 = pid - t2 * a.n1;
   const int base = live ? t1 * (int)a.s1 + t2 * (int)a.s2 : 0;
   // the pencil's cells are active across the sweep (calc_dt covers active cells only)
   const bool cfl = a.cfl_min_bits && t1 >= a.ts1 && t1 <= a.te1 && t2 >= a.ts2 && t2 <= a.te2;
-  const CflFilter flt = cfl_filter(a, t1, t2, best, cfl);
   double dtmin = 1.0e20;
   const int sa = (int)a.sa, np = (int)a.npencils;
   const double qdx = P.dt / a.uc.dx;  // dt/dx of every cell (a.uniform)
@@ -1747,7 +1749,7 @@ __device__ __forceinline__ bool update_pencil(const SweepArgs& a, int pid, const
           dep = o.d * o.e;
         }
         if (!isfinite(o.d) || !isfinite(o.e)) nonfin += 1;
-        if (cfl && (ST || (c >= is && c <= ie)) && cfl_candidate<DUAL>(flt, a, o, P))
+        if (cfl && (ST || (c >= is && c <= ie)))
           dtmin = dmin(dtmin, cell_dt1<DUAL>(a, o, a.uniform ? a.uc.dx : a.coef[c].dx, t1, t2, P));
         if (STAGED && PPM_X_STAGE_STORES) {
           double* sp = stage + (c % kStageCells) * kStageLd + (threadIdx.x & 31);
@@ -1921,7 +1923,6 @@ __global__ void __launch_bounds__(kMarchThreads,
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");
   __shared__ unsigned long long s_cnt[2];
   __shared__ unsigned char s_flag[kMarchThreads];  // pencils handed to the fallback pass
-  __shared__ int s_best;                           // see CflFilter
   __shared__ uint64_t s_xbar[XT ? (kMarchThreads / 32) * kXBuffers : 1];
   extern __shared__ __align__(128) double s_dyn[];
   double* const s_xtile = s_dyn;                                // XT: kXWarp per warp
@@ -1929,7 +1930,6 @@ __global__ void __launch_bounds__(kMarchThreads,
   double* const s_ring = s_dyn;                                 // y, z: the input ring
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0ull;
   s_flag[threadIdx.x] = 0;
-  if (threadIdx.x == 0) s_best = 0;
   int64_t lb;
   const int g = locate<ONE>(B.upd_prefix, B.ngrids, lb);
   PPM_BIND_RECORD(a, g)
@@ -1954,7 +1954,7 @@ __global__ void __launch_bounds__(kMarchThreads,
     const Phys P = make_phys(a);
     if (update_pencil<DUAL, GRAV, false, STAGED, update_pipe<ONE, STAGED>(), XT, RS>(
             a, pid, P, cnt, c0, c1, valid, s_stage + warp * kStageWarp, wpid0,
-            s_ring + threadIdx.x, &xt, &s_best))
+            s_ring + threadIdx.x, &xt))
       s_flag[pl] = 1;
   }
   finish_block<DUAL, false>(B, a, g, pid, c0, c1, valid && c0 < a.n, s_flag, pl, s_cnt, cnt);

@@ -84,3 +84,43 @@ def test_folded_time_step_of_a_level_with_graphs(torch):
         assert dt.item() == ref, (cyc, dt.item(), ref)
         ctx.set_boundary_level(grids, fs, True)
     ctx.close()
+
+
+# A pencil cut into segments of eight cells, whose bad cell b (its density runs out along the
+# last sweep) lies two cells from a segment border: the fallback changes the energy of cell
+# b+1, hence the dual-energy select of cell b+2, which another segment has stored by then with
+# the hot gas energy it no longer has.  The signal speed of that state must not keep the true
+# fastest cell (another pencil of the block, the last cell of its segment) out of the minimum.
+@pytest.mark.parametrize("u,dt,ub,db,dc,dm,de,up", [
+    (2.2498, 0.0089198, 0.0, 0.63657, 0.38141, 1.1054, 6.8954, True),
+    (1.4972, 0.012593, 0.0, 2.2955, 2.0466, 1.5901, 7.4858, False),
+    (1.3202, 0.017501, 0.0, 2.4083, 2.3949, 2.8732, 8.024, False),
+    (2.5989, 0.0093248, 0.0, 0.53066, 0.38457, 2.1178, 8.5972, False),
+])
+@pytest.mark.parametrize("variant", ["exact", "fast"])
+def test_folded_time_step_beside_a_flagged_pencil(torch, variant, u, dt, ub, db, dc, dm, de, up):
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=True)
+    g = H.Grid.uniform((20, 64), width=(20 / 64, 1.0))
+    bad, hot = 10, 13  # pencils along y
+    b, step = (22, 1) if up else (25, -1)
+    d, v = np.ones(g.shape), np.full(g.shape, 6.0)
+    v[:, :, (bad, hot)] = 0.0
+    v[0, b, bad], v[0, b - step, bad] = step * u, step * u * ub
+    d[0, b, bad], d[0, b + step, bad], d[0, b - step, bad] = db, dc, dm
+    d[0, b + 2 * step, bad] = 0.03
+    d[0, 39, hot] = 0.045
+    ge = 1.5 / d  # one pressure: nothing moves along x
+    te = ge + 0.5 * v ** 2
+    te[0, b + 2 * step, bad] = 0.1 * de / 0.03  # the select's threshold between the two
+    zero = np.zeros(g.shape)
+    f = dict(d=d, te=te, v1=zero, v2=v, v3=zero, ge=ge)
+    ctx = capi.Context(0, variant=variant)
+    nxt = torch.zeros(1, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.set_cfl(nxt, courant=hp.cfl)
+    fd = _dev(f, torch)
+    rc, st = ctx.solve_ppm_de(g, hp, dt, 0, fd, memory=capi.MEM_DEVICE)
+    assert st["fallbacks"] > 0
+    assert fd["ge"][0, b + 2 * step, bad].item() < 30.0  # selected again (50 before)
+    assert nxt.item() == ctx.compute_timestep(g, hp, fd, memory=capi.MEM_DEVICE)
+    ctx.close()
