@@ -555,16 +555,16 @@ __device__ __forceinline__ Godunov godunov_state(const FaceState& s, double pbar
   }
 #if PPM_FAST_ALGEBRA
   // tolerance mode: 1/d0 and 1/p0 from one reciprocal; z0^2 = c0^2 d0^2 X without its
-  // root; dbar = d0 z0^2/(z0^2 - (pbar - p0) d0) and its reciprocal from one reciprocal
-  // of the two factors; of c0 and z0/d0 = c0 sqrt(X) only the one that l0 takes
+  // root; dbar = d0 z0^2/(z0^2 - (pbar - p0) d0) and its reciprocal (two reciprocals: the
+  // product of the two factors, (gamma p d)^2, would leave the range of a double where the
+  // reference's expressions do not); of c0 and z0/d0 = c0 sqrt(X) only the one that l0 takes
   const double q0 = qrcp_n(d0 * p0), id0 = p0 * q0;
   const double c02 = dmax(gamma * p0 * id0, kTiny);
   const double X = dmax(1.0 + P.qa * (pbar * (d0 * q0) - 1.0), kTiny);
   const double c02X = c02 * X;
   const double z02 = dmax(c02X * (d0 * d0), kTiny), zd = z02 - (pbar - p0) * d0;
-  const double qz = qrcp_n(z02 * zd);  // z02 >= tiny, zd of its order
-  const double idbar = id0 * (zd * zd * qz);
-  const double dbar = d0 * (z02 * z02 * qz);
+  const double idbar = id0 * (zd * qrcp_n(z02));  // z02 >= tiny, zd of its order
+  const double dbar = d0 * (z02 * qrcp_n(zd));
   const bool rare = pbar < p0;
   double iroot;
   const double l0 = u0 * sn + qsqrt_n(rare ? c02 : c02X, iroot);
