@@ -784,7 +784,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   fused = fused && !uneven;  // the face kernel is the plain path's: one cell width
   const bool transport = solver_code(p) == 0 && p->pressure_free != 1 && nc == 0 && !fused &&
                          ppm::use_transport(total_cells);
-  const bool local_select = !p->dual_energy || p->eta1 <= 0.25 * p->eta2;
+  const bool local_select = ppm::select_is_local(p->dual_energy != 0, p->eta1, p->eta2);
   for (int k = 0; k < ng; ++k) {
     ppm::set_segments(rec[k], total_pencils, local_select, transport);
     gpre[k + 1] = gpre[k] + ppm::segment_blocks(rec[k], rec[k].pw_log2);

@@ -866,8 +866,8 @@ __device__ __forceinline__ void pgas2d_dual(Cell& c, double de_m, double de_p, c
 // They enter only through demax >= d*e of the cell itself, in the test ge1*d/demax > eta2
 // that replaces ge by ge1.  The total energy does not depend on that test where
 // ge1/e > eta1 (it is rebuilt from ge1 either way), nor where ge1*d/(d*e) is below eta2
-// (then no larger demax can pass it; half of eta2 leaves room for rounding).  known =
-// false: neither holds, and the neighbours decide.
+// (then, with eta2 >= 0, no larger demax can pass it; half of eta2 leaves room for
+// rounding).  known = false: neither holds, and the neighbours decide.
 __device__ __forceinline__ double pgas2d_de_local(const Cell& c, const Phys& P, bool& known) {
   double ke = 0.5 * (c.u * c.u + c.v * c.v + c.w * c.w);
   double ge1 = c.e - ke;

@@ -253,7 +253,8 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   const int64_t riemann_blocks =
       (int64_t)(a.ie - a.is + 2) * ((a.npencils + ppm::kRiemannThreads - 1) / ppm::kRiemannThreads);
   const bool transport = ppm::use_transport(a.npencils * a.n);
-  ppm::set_segments(a, a.npencils, !p->dual_energy || p->eta1 <= 0.25 * p->eta2, transport);
+  ppm::set_segments(a, a.npencils, ppm::select_is_local(p->dual_energy != 0, p->eta1, p->eta2),
+                    transport);
   ppm::set_uniform(a, in->cell_width[dim], table.data());
   const int64_t seg_blocks = ppm::segment_blocks(a, a.pw_log2);
   const int64_t upd_blocks = ppm::segment_blocks(a, a.uw_log2);

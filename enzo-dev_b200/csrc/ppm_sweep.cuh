@@ -314,9 +314,14 @@ inline bool use_both_roles(int64_t seg_blocks, bool transport) {
 inline int64_t segment_blocks(const SweepArgs& a, int log_w) {
   return (a.npencils + (int64_t(1) << log_w) - 1) >> log_w;
 }
-// a: a record with its geometry; batch_pencils: pencils of all grids of the launch.
-// local_select: pgas2d_dual's energy of a cell may be formed without its left neighbour
-// (see update_pencil); without it the update needs whole pencils.
+// pgas2d_dual's energy of a cell may be formed without its left neighbour (see
+// pgas2d_de_local, which needs 0 <= eta2: then a neighbour's energy can only keep the test
+// from passing); otherwise the update needs whole pencils.
+inline bool select_is_local(bool dual, double eta1, double eta2) {
+  return !dual || (eta2 >= 0.0 && eta1 <= 0.25 * eta2);
+}
+// a: a record with its geometry; batch_pencils: pencils of all grids of the launch;
+// local_select: select_is_local.
 inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select,
                          bool transport) {
   int whole = 0;

@@ -65,6 +65,20 @@ def test_dual_energy_select_parameters(ctx, eta1, eta2):
     _steps(ctx, g, hp, random_state(g, hp, seed=9, mach=8.0))
 
 
+# a negative eta2: an internal energy below zero passes the test beside a neighbour of larger
+# energy where it would not by itself, so the pencils stay whole
+@pytest.mark.parametrize("seed,eta1,eta2", [(3, -0.3, -0.3), (5, -1.0, -1.0), (8, -0.3, -0.3),
+                                            (12, -2.0, -0.6)])
+def test_dual_energy_select_of_negative_thresholds(ctx, seed, eta1, eta2):
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.1, dual=True, eta1=eta1, eta2=eta2)
+    g = H.Grid.uniform((1000,))
+    f = random_state(g, hp, seed=seed, mach=8.0)
+    rng = np.random.default_rng(seed)
+    low = rng.random(g.shape) < 0.6
+    f["te"][low] = (0.5 * f["v1"] ** 2 * rng.uniform(0.1, 0.7, g.shape))[low]
+    _steps(ctx, g, hp, f, cycles=1)
+
+
 # colours are updated in place by the segments of a pencil; flattening and steepening
 # coefficients come in the same split
 @pytest.mark.parametrize("shape,ncol", [((9,), 1), ((130,), 3), ((40, 37), 2), ((17, 33, 20), 5)])
