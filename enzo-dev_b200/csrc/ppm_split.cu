@@ -1491,7 +1491,7 @@ __device__ __forceinline__ bool cfl_candidate(const CflFilter& f, const SweepArg
   if (f.has_w) S += (cs + fabs(o.w - f.gw)) * f.i2;
   const int hi = __double2hiint(S), top = *(volatile int*)f.best;
   if (hi > top && hi < 0x7FF00000) atomicMax(f.best, hi);
-  return hi >= top - kCflMargin;  // infinities and positive NaN included
+  return hi >= top - kCflMargin || hi < 0;  // infinities and NaN included (0 pressure: 0/0)
 }
 
 // The smallest dt1 of stored cells c0 .. c1 of a pencil: for the pencils of a block in which

@@ -107,3 +107,24 @@ def test_level(torch, variant, graphs, dual, bad):
         ref = ctx.compute_timestep_level(grids, hp, fs)
         assert nxt.item() == ref, (cyc, nxt.item(), ref)
     ctx.close()
+
+
+# without a pressure floor a cold cell's pressure is zero (its total energy less than its
+# kinetic one after the step): it still moves, and may be the fastest
+@pytest.mark.parametrize("variant", ["exact", "fast"])
+def test_cells_without_pressure(torch, variant):
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=False, tiny_number=0.0)
+    g = H.Grid.uniform((900, 900))
+    f = random_state(g, hp, seed=2, mach=1e4)
+    ctx = capi.Context(0, variant=variant)
+    nxt = torch.zeros(1, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.set_cfl(nxt, courant=hp.cfl)
+    fd = {k: torch.from_numpy(v.copy()).cuda() for k, v in f.items()}
+    dt = ctx.compute_timestep(g, hp, fd, memory=capi.MEM_DEVICE)
+    rc, _ = ctx.solve_ppm_de(g, hp, dt, 0, fd, memory=capi.MEM_DEVICE, check=False)
+    assert rc in (capi.OK, capi.ERR_NEGATIVE)
+    cold = fd["te"] - 0.5 * (fd["v1"] ** 2 + fd["v2"] ** 2) <= 0.0
+    assert int(cold[0, 3:-3, 3:-3].sum()) > 1000
+    assert nxt.item() == ctx.compute_timestep(g, hp, fd, memory=capi.MEM_DEVICE)
+    ctx.close()
