@@ -1197,9 +1197,10 @@ struct HostPieces {
   }
 };
 
-// Pageable memory of a size worth the threads.
-bool pageable(const void* p, size_t call_bytes) {
-  if (call_bytes < kPiecesLeast) return false;
+// Pageable memory of a size worth the threads.  Not on the per-thread default stream, which
+// is another stream in each of them: the copies would not be ordered with the kernels.
+bool pageable(const ppm_b200_context* ctx, const void* p, size_t call_bytes) {
+  if (call_bytes < kPiecesLeast || ctx->stream == cudaStreamPerThread) return false;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
@@ -1299,7 +1300,7 @@ int stage_in(ppm_b200_context* ctx, const ppm_b200_params* p, ppm_b200_grid* g, 
   size_t call_bytes = bytes * (size_t)fs.ncol;
   for (int k = 0; k < 6; ++k) call_bytes += src[k] ? bytes : 0;
   auto bring = [&](void* dst, const void* host) -> int {
-    if (pageable(host, call_bytes)) {
+    if (pageable(ctx, host, call_bytes)) {
       pieces.add(const_cast<void*>(host), dst, bytes);
       return PPM_B200_OK;
     }
@@ -1347,7 +1348,7 @@ int stage_out(ppm_b200_context* ctx, const ppm_b200_params* p, ppm_b200_grid* g,
   size_t call_bytes = bytes * (size_t)fs.ncol;
   for (int k = 0; k < 6; ++k) call_bytes += dst[k] && fs.f[k] ? bytes : 0;
   auto send = [&](void* host, void* dev) -> int {
-    if (pageable(host, call_bytes)) {
+    if (pageable(ctx, host, call_bytes)) {
       pieces.add(host, dev, bytes);
       return PPM_B200_OK;
     }

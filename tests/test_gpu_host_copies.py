@@ -5,7 +5,7 @@ import pytest
 
 from ppm_b200 import capi
 from ppm_b200 import harness as H
-from parity_util import random_state
+from parity_util import copy_fields, random_state
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +39,24 @@ def test_pageable_pinned_and_device_fields_agree(shape, ncol, grav):
             assert np.array_equal(host[k], ref), (cyc, k)
             assert np.array_equal(pinned_np[k], ref), (cyc, k)
     c.close()
+
+
+# a context on a stream of the caller's: the legacy and the per-thread default stream (whose
+# handles, 1 and 2, name the calling thread's own stream) and a created one
+@pytest.mark.parametrize("stream", [1, 2, "created"])
+def test_host_fields_on_the_callers_stream(stream):
+    torch = pytest.importorskip("torch")
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=True)
+    g = H.Grid.uniform((64, 64, 64))
+    f = random_state(g, hp, seed=4)
+    own = torch.cuda.Stream()
+    ref, ctx = capi.Context(0), capi.Context(0, stream=own.cuda_stream if stream == "created"
+                                             else stream)
+    a, b = copy_fields(f), copy_fields(f)
+    for cyc in range(3):
+        ref.solve_ppm_de(g, hp, 1e-3, cyc, a)
+        ctx.solve_ppm_de(g, hp, 1e-3, cyc, b)
+        for k in f:
+            assert np.array_equal(a[k], b[k]), (cyc, k)
+    ctx.close()
+    ref.close()
