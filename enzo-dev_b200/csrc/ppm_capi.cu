@@ -1218,7 +1218,14 @@ int copy_pieces(ppm_b200_context* ctx, const HostPieces& w, bool to_device) {
     if (ctx->pinned) CK(cudaFreeHost(ctx->pinned));
     ctx->pinned = nullptr;
     ctx->pinned_bytes = 0;
-    CK(cudaMallocHost(&ctx->pinned, slots * kPiece));
+    if (cudaMallocHost(&ctx->pinned, slots * kPiece) != cudaSuccess) {
+      cudaGetLastError();  // no pinned memory to be had: the driver's own staging
+      ctx->pinned = nullptr;
+      for (const HostPieces::Piece& p : w.list)
+        CK(cudaMemcpyAsync(to_device ? p.dev : p.host, to_device ? p.host : p.dev, p.bytes,
+                           cudaMemcpyDefault, ctx->stream));
+      return PPM_B200_OK;
+    }
     ctx->pinned_bytes = slots * kPiece;
   }
   while (ctx->pinned_done.size() < slots) {

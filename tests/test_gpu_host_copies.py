@@ -1,5 +1,10 @@
 """Host-memory calls: pageable fields go through the context's pinned pieces (threads above
 4 MB a call), pinned fields directly; the fields are the device call's either way."""
+import resource
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -60,3 +65,33 @@ def test_host_fields_on_the_callers_stream(stream):
             assert np.array_equal(a[k], b[k]), (cyc, k)
     ctx.close()
     ref.close()
+
+
+# No pinned memory to be had (the process's address space is full): the call takes the
+# driver's copies.  In a process of its own.
+def no_pinned_memory():
+    import torch
+
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=True)
+    g = H.Grid.uniform((64, 64, 64))
+    f = random_state(g, hp, seed=4)
+    c = capi.Context(0)
+    pinned = {k: torch.from_numpy(v.copy()).pin_memory() for k, v in f.items()}
+    ref = {k: v.numpy() for k, v in pinned.items()}
+    c.solve_ppm_de(g, hp, 1e-3, 0, ref)  # allocates all the call needs but the staging
+    used = int(Path("/proc/self/statm").read_text().split()[0]) * resource.getpagesize()
+    soft, hard = resource.getrlimit(resource.RLIMIT_AS)
+    resource.setrlimit(resource.RLIMIT_AS, (used + (1 << 20), hard))
+    rc, _ = c.solve_ppm_de(g, hp, 1e-3, 0, f, check=False)
+    resource.setrlimit(resource.RLIMIT_AS, (soft, hard))
+    assert rc == capi.OK
+    for k in f:
+        assert np.array_equal(f[k], ref[k]), k
+    c.close()
+
+
+def test_no_pinned_memory():
+    here = Path(__file__).resolve().parent
+    code = (f"import sys; sys.path[:0] = [{str(here)!r}, {str(here.parent / 'enzo-dev_b200')!r}]; "
+            "import test_gpu_host_copies as t; t.no_pinned_memory()")
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
