@@ -67,7 +67,7 @@ struct FieldCopy {
   int64_t size;
 };
 void launch_copy_back(const FieldCopy& X, cudaStream_t st);
-void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st);
+void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained);
 void launch_cfl_finalize(const unsigned long long* min_bits, double courant, double* dt_out,
                          cudaStream_t st);
 void launch_sweep_batch(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
@@ -86,10 +86,10 @@ cudaError_t launch_guess_eval(const uint32_t* packed, const float* feats, int64_
                               cudaStream_t st);
 cudaError_t launch_guess_eval_tc(const uint32_t* words, const float* feats, int64_t n, float* y,
                                  unsigned long long* timeouts, int sms, cudaStream_t st);
-void launch_pressure_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st);
+void launch_pressure_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained);
 void launch_timestep_batch(const ElemBatch& B, int64_t blocks, double courant, double* dt_out,
                            cudaStream_t st);
-void launch_boundary_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st);
+void launch_boundary_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained);
 struct CopyBox {
   int dst, src;
   int d0[3], s0[3], ext[3];
@@ -968,9 +968,10 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   return PPM_B200_OK;
 }
 
-// clear_bits: the folded time step's minimum, reset before this sweep (null: not here)
+// chained: the sweep follows kernels of the launch chain (see ppm_launch.cuh); clear_bits: the
+// folded time step's minimum, reset before this sweep (null: not here)
 int enqueue_sweep(ppm_b200_context* ctx, const SweepPlan& plan, const ppm_b200_params* p,
-                  bool capturing, unsigned long long* clear_bits = nullptr) {
+                  bool capturing, bool chained, unsigned long long* clear_bits = nullptr) {
   cudaEvent_t* ev = nullptr;
   if (ctx->profiling && !capturing) {
     while (ctx->ev_pool.size() < ctx->ev_used + kSweepEvents) {
@@ -983,6 +984,7 @@ int enqueue_sweep(ppm_b200_context* ctx, const SweepPlan& plan, const ppm_b200_p
   }
   BatchArgs B = plan.B;
   B.clear_bits = clear_bits;
+  B.chained = chained ? 1 : 0;
   ppm::launch_sweep_batch(B, plan.march_blocks, plan.riemann_blocks, p->dual_energy != 0,
                           p->gravity != 0, ctx->stream, ev, p->learned_guess != 0,
                           plan.contiguous);
@@ -1496,19 +1498,22 @@ int copy_back(ppm_b200_context* ctx, const GridIO& x) {
   return PPM_B200_OK;
 }
 
-// cfl_first / cfl_last: this solve is the first / last of a level's waves, which share
-// one folded time step: the minimum is reset before the first wave's last sweep and the
-// time step written after the last wave's (every wave reads the old one until then).
+// cfl_first / cfl_last: this solve is the first / last of a level's waves, which share one
+// folded time step: the minimum is reset before the first wave's last sweep and the time
+// step written after the last wave's (every wave reads the old one until then).  The first
+// wave's first kernel starts the launch chain.
 int enqueue_solve(ppm_b200_context* ctx, const ppm_b200_params* p, const std::vector<GridIO>& io,
                   const SolvePlan& sp, bool capturing, bool cfl_first = true,
                   bool cfl_last = true) {
-  ppm::launch_pressure_batch(sp.pressure.B, sp.pressure.size_blocks, ctx->stream);
+  ppm::launch_pressure_batch(sp.pressure.B, sp.pressure.size_blocks, ctx->stream,
+                             ctx->own_stream || !cfl_first);
   ctx->launches += 1;
   CK(cudaGetLastError());
   unsigned long long* cfl_bits = ((unsigned long long*)ctx->misc.p) + 2;
   for (int s = 0; s < sp.nsweeps; ++s) {
     const bool cfl = ctx->cfl_dt != nullptr && s == sp.nsweeps - 1;
-    int rc = enqueue_sweep(ctx, sp.sweep[s], p, capturing, cfl && cfl_first ? cfl_bits : nullptr);
+    int rc = enqueue_sweep(ctx, sp.sweep[s], p, capturing, true,
+                           cfl && cfl_first ? cfl_bits : nullptr);
     if (rc) return rc;
     if (cfl && cfl_last) {
       ppm::launch_cfl_finalize(cfl_bits, ctx->cfl_courant, ctx->cfl_dt, ctx->stream);
@@ -1522,7 +1527,7 @@ int enqueue_solve(ppm_b200_context* ctx, const ppm_b200_params* p, const std::ve
       if (rc) return rc;
     }
   if (p->eos_type > 0) {  // energies consistent with the EOS again (Grid_SolvePPM_DE.C:155-157)
-    ppm::launch_pressure_batch(sp.pressure.B, sp.pressure.size_blocks, ctx->stream);
+    ppm::launch_pressure_batch(sp.pressure.B, sp.pressure.size_blocks, ctx->stream, true);
     ctx->launches += 1;
     CK(cudaGetLastError());
   }
@@ -2227,7 +2232,7 @@ int ppm_b200_euler_sweep(ppm_b200_context* ctx, int dim, const ppm_b200_params* 
   std::vector<int> src(1, -1), dst(1, 0);
   rc = prepare_sweep(ctx, dim, 0, p, io, src, dst, plan);
   if (rc) return rc;
-  rc = enqueue_sweep(ctx, plan, p, false);
+  rc = enqueue_sweep(ctx, plan, p, false, ctx->own_stream);
   if (rc) return rc;
   rc = scatter_captures(ctx, dim, p, g, plan, sub);
   if (rc) return rc;
@@ -2266,7 +2271,7 @@ int ppm_b200_compute_pressure(ppm_b200_context* ctx, const ppm_b200_params* p, p
   ElemPlan ep;
   rc = prepare_elem(ctx, kSlotPressure, p, io, false, nullptr, ep);
   if (rc) return rc;
-  ppm::launch_pressure_batch(ep.B, ep.size_blocks, ctx->stream);
+  ppm::launch_pressure_batch(ep.B, ep.size_blocks, ctx->stream, ctx->own_stream);
   ctx->launches += 1;
   CK(cudaGetLastError());
   if (memory == PPM_B200_MEM_HOST) {
@@ -2404,7 +2409,7 @@ static int boundary_batch(ppm_b200_context* ctx, ppm_b200_grid* grids, int ngrid
   ElemPlan ep;
   int rc = prepare_elem(ctx, kSlotBoundary, &p, io, false, bc_type, ep);
   if (rc) return rc;
-  ppm::launch_boundary_batch(ep.B, ep.row_blocks, ctx->stream);
+  ppm::launch_boundary_batch(ep.B, ep.row_blocks, ctx->stream, ctx->own_stream);
   ctx->launches += 1;
   CK(cudaGetLastError());
   return PPM_B200_OK;
@@ -2774,7 +2779,7 @@ static int expansion_batch(ppm_b200_context* ctx, const ppm_b200_params* p,
       ep.B.interpolate = 1;
     }
   }
-  ppm::launch_expansion_batch(ep.B, ep.size_blocks, ctx->stream);
+  ppm::launch_expansion_batch(ep.B, ep.size_blocks, ctx->stream, ctx->own_stream);
   ctx->launches += 1;
   CK(cudaGetLastError());
   return PPM_B200_OK;

@@ -512,8 +512,9 @@ void launch_copy_back(const FieldCopy& X, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ launchers
-void launch_pressure_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  launch_chain(B.ngrids == 1 ? pressure_kernel<true> : pressure_kernel<false>, blocks, 256, 0, st, B);
+// chained: as a link of the launch chain (see ppm_launch.cuh)
+void launch_pressure_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained) {
+  launch_link(chained, B.ngrids == 1 ? pressure_kernel<true> : pressure_kernel<false>, blocks, 256, 0, st, B);
 }
 
 void launch_timestep_batch(const ElemBatch& B, int64_t blocks, double courant, double* dt_out,
@@ -530,12 +531,12 @@ void launch_cfl_finalize(const unsigned long long* min_bits, double courant, dou
   launch_chain(timestep_finalize_kernel, 1, 32, 0, st, min_bits, courant, dt_out);
 }
 
-void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  launch_chain(B.ngrids == 1 ? expansion_kernel<true> : expansion_kernel<false>, blocks, 256, 0, st, B);
+void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained) {
+  launch_link(chained, B.ngrids == 1 ? expansion_kernel<true> : expansion_kernel<false>, blocks, 256, 0, st, B);
 }
 
-void launch_boundary_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st) {
-  launch_chain(B.ngrids == 1 ? boundary_kernel<true> : boundary_kernel<false>, blocks, 256, 0, st, B);
+void launch_boundary_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained) {
+  launch_link(chained, B.ngrids == 1 ? boundary_kernel<true> : boundary_kernel<false>, blocks, 256, 0, st, B);
 }
 
 }  // namespace ppm

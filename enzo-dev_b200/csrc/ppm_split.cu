@@ -2768,16 +2768,21 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
     if (ev) cudaEventRecord(ev[k], st);
   };
   const unsigned sb = (unsigned)B.seg_blocks;
+  // the first kernel: part of the launch chain, or behind whatever the caller queued
+  bool chained = B.chained != 0;
+  auto link = [&](auto kernel, int64_t grid, int block) {
+    launch_link(chained, kernel, grid, block, 0, st, B);
+    chained = true;
+  };
   mark(0);
   if (B.transport) {
     const bool cor = B.corrections || B.uneven;
     const unsigned rb = (unsigned)riemann_blocks;
-    if (B.corrections)
-      launch_chain(corrections_kernel<ONE>, sb, kMarchThreads, 0, st, B);
+    if (B.corrections) link(corrections_kernel<ONE>, sb, kMarchThreads);
     if (cor)
-      launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads, 0, st, B);
+      link(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads);
     else
-      launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE>, sb, kMarchThreads, 0, st, B);
+      link(reconstruct_kernel<DUAL, GRAV, 0, ONE>, sb, kMarchThreads);
     mark(1);
     mark(2);
     if (learned && B.learned_pass) {
@@ -2828,9 +2833,9 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
   }
   if (B.ncolour > 0) cudaMemsetAsync(B.hll_flags, 0, (size_t)B.hll_bytes, st);
   const bool cor = B.corrections || B.ncolour > 0 || B.presfree || B.uneven;
-  if (B.corrections) launch_chain(corrections_kernel<ONE>, sb, kMarchThreads, 0, st, B);
+  if (B.corrections) link(corrections_kernel<ONE>, sb, kMarchThreads);
   if (B.both_roles) {
-    launch_chain(clear_sweep_kernel, 1, 1, 0, st, B);
+    link(clear_sweep_kernel, 1, 1);
     mark(1);
     if (cor)
       launch_chain(reconstruct_both_kernel<DUAL, GRAV, ONE, true>, 2 * B.seg_blocks,
@@ -2839,11 +2844,11 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
       launch_chain(reconstruct_both_kernel<DUAL, GRAV, ONE, false>, 2 * B.seg_blocks,
                    kMarchThreads, 0, st, B);
   } else if (cor) {
-    launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads, 0, st, B);
+    link(reconstruct_kernel<DUAL, GRAV, 0, ONE, true>, sb, kMarchThreads);
     mark(1);
     launch_chain(reconstruct_kernel<DUAL, GRAV, 1, ONE, true>, sb, kMarchThreads, 0, st, B);
   } else {
-    launch_chain(reconstruct_kernel<DUAL, GRAV, 0, ONE>, sb, kMarchThreads, 0, st, B);
+    link(reconstruct_kernel<DUAL, GRAV, 0, ONE>, sb, kMarchThreads);
     mark(1);
     launch_chain(reconstruct_kernel<DUAL, GRAV, 1, ONE>, sb, kMarchThreads, 0, st, B);
   }

@@ -185,6 +185,7 @@ struct BatchArgs {
   int64_t upd_blocks = 0;
   int transport = 0;                 // the transport path (see transport_kernel)
   int both_roles = 0;                // both reconstructions in one launch
+  int chained = 1;                   // the sweep's first kernel is a link of the launch chain
   unsigned long long* clear_bits = nullptr;  // folded time step to reset before this sweep
   const int64_t* riemann_prefix;     // ngrids + 1
   unsigned long long* counters;      // kCounterCopies x kMaxCounters, shared by the batch
