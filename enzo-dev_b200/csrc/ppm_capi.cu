@@ -70,9 +70,8 @@ void launch_copy_back(const FieldCopy& X, cudaStream_t st);
 void launch_expansion_batch(const ElemBatch& B, int64_t blocks, cudaStream_t st, bool chained);
 void launch_cfl_finalize(const unsigned long long* min_bits, double courant, double* dt_out,
                          cudaStream_t st);
-void launch_sweep_batch(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
-                        bool dual, bool grav, cudaStream_t st, cudaEvent_t* ev, bool learned,
-                        bool contiguous);
+void launch_sweep_batch(const BatchArgs& B, int64_t riemann_blocks, bool dual, bool grav,
+                        cudaStream_t st, cudaEvent_t* ev, bool learned, bool contiguous);
 int riemann_resident_blocks(bool dual, bool one, int threads);
 // learned-start training and evaluation (ppm_mlp.cu)
 cudaError_t launch_guess_features(const double* rec, int64_t n, double gamma, double pmin,
@@ -166,7 +165,8 @@ enum {
 };
 // captured level graphs kept at most (a changed grid list leaves the old ones unused)
 constexpr size_t kMaxGraphs = 16;
-// events around a timed sweep: before each of its five kernels and after the last
+// events around a timed sweep: before each of its five stages (see ppm_b200_profile_stages)
+// and after the last
 constexpr int kSweepEvents = 6;
 
 struct ppm_b200_context {
@@ -184,7 +184,7 @@ struct ppm_b200_context {
   DevBuf ring;              // two ring sets of the six updated fields, every grid of the batch
   DevBuf pressure;          // pressure of every grid of the batch
   DevBuf face_scratch;      // interface states, fluxes and the flagged-pencil list
-  DevBuf counters;          // kMaxCounters unsigned long long
+  DevBuf counters;          // kCounterCopies x kMaxCounters unsigned long long
   DevBuf misc;              // [0] min_bits, [1] dt, [2] min_bits of the folded time step
   DevBuf captures;
   DevBuf capture_buf;
@@ -560,7 +560,7 @@ void set_x_tiles(BatchArgs& B, const SweepArgs& a) {
 // Everything one directional sweep of a batch needs on the device.
 struct SweepPlan {
   BatchArgs B;
-  int64_t march_blocks = 0, riemann_blocks = 0;
+  int64_t riemann_blocks = 0;
   std::vector<FluxCapture> reqs;    // single-grid subgrid-flux capture
   std::vector<HostCapture> hreq;
   int64_t cap_offset = 0;           // this sweep's first request in the capture buffers
@@ -724,8 +724,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   const bool persist = plain_riemann && ctx->wave_persist != 0;
   // face scratch: planes of every grid, then the flagged-pencil list
   std::vector<SweepArgs> rec(ng);
-  std::vector<int64_t> mpre(ng + 1, 0), rpre(ng + 1, 0), fpre(ng + 1, 0), gpre(ng + 1, 0),
-      upre(ng + 1, 0);
+  std::vector<int64_t> rpre(ng + 1, 0), fpre(ng + 1, 0), gpre(ng + 1, 0), upre(ng + 1, 0);
   // the fused face kernel serves the same plain two-shock path, without slope corrections
   bool fused = plain_riemann && ctx->sweep_mode == PPM_B200_SWEEP_FUSED &&
                      correction_planes(p) == 0;
@@ -769,9 +768,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
     total_pencils += a.npencils;
     total_cells += a.npencils * a.n;
     if (nc > 0) flag_bytes += (size_t)a.plane;
-    const int64_t mb = (a.npencils + ppm::kMarchThreads - 1) / ppm::kMarchThreads;
     const int64_t rb = (int64_t)(a.ie - a.is + 2) * ((a.npencils + rt - 1) / rt);
-    mpre[k + 1] = mpre[k] + mb;
     rpre[k + 1] = rpre[k] + rb;
     fpre[k + 1] = fpre[k] + ppm::face_blocks(a.npencils, a.is, a.ie);
   }
@@ -901,9 +898,6 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   // device: its record travels in the kernel parameters.
   std::vector<unsigned char> img;
   append(img, rec.data(), rec.size());
-  const size_t off_m = align256(img.size());
-  img.resize(off_m);
-  append(img, mpre.data(), mpre.size());
   const size_t off_r = align256(img.size());
   img.resize(off_r);
   append(img, rpre.data(), rpre.size());
@@ -940,7 +934,6 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.hll_bytes = (int64_t)flag_bytes;
   plan.B.grids = (const SweepArgs*)base;
   plan.B.ngrids = ng;
-  plan.B.march_prefix = (const int64_t*)(base + off_m);
   plan.B.riemann_prefix = (const int64_t*)(base + off_r);
   plan.B.seg_prefix = (const int64_t*)(base + off_g);
   plan.B.seg_blocks = gpre[ng];
@@ -950,7 +943,6 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.both_roles = ppm::use_both_roles(gpre[ng], transport) ? 1 : 0;
   plan.B.counters = (unsigned long long*)ctx->counters.p;
   plan.B.flagged = (int64_t*)(scratch + scratch_doubles);
-  plan.march_blocks = mpre[ng];
   plan.riemann_blocks = rpre[ng];
   plan.B.riemann_threads = rt;
   plan.B.persistent = persist ? 1 : 0;
@@ -985,8 +977,8 @@ int enqueue_sweep(ppm_b200_context* ctx, const SweepPlan& plan, const ppm_b200_p
   BatchArgs B = plan.B;
   B.clear_bits = clear_bits;
   B.chained = chained ? 1 : 0;
-  ppm::launch_sweep_batch(B, plan.march_blocks, plan.riemann_blocks, p->dual_energy != 0,
-                          p->gravity != 0, ctx->stream, ev, p->learned_guess != 0,
+  ppm::launch_sweep_batch(B, plan.riemann_blocks, p->dual_energy != 0, p->gravity != 0,
+                          ctx->stream, ev, p->learned_guess != 0,
                           plan.contiguous);
   ctx->launches += sweep_kernels(p, B);
   CK(cudaGetLastError());
@@ -1689,7 +1681,6 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, b.grids);
     key_put(k, b.ngrids);
     if (b.ngrids == 1) key_put(k, b.one);
-    key_put(k, b.march_prefix);
     key_put(k, b.riemann_prefix);
     key_put(k, b.seg_prefix);
     key_put(k, b.seg_blocks);
@@ -1699,7 +1690,6 @@ std::string graph_key(ppm_b200_context* ctx, const ppm_b200_params* p, const Sol
     key_put(k, b.both_roles);
     key_put(k, b.counters);
     key_put(k, b.flagged);
-    key_put(k, sp.sweep[s].march_blocks);
     key_put(k, sp.sweep[s].riemann_blocks);
     key_put(k, sp.sweep[s].contiguous);
     key_put(k, b.x_tma);

@@ -44,9 +44,8 @@
 #include "ppm_sweep.cuh"
 
 namespace ppm {
-void launch_sweep_batch(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
-                        bool dual, bool grav, cudaStream_t st, cudaEvent_t* ev, bool learned,
-                        bool contiguous);
+void launch_sweep_batch(const BatchArgs& B, int64_t riemann_blocks, bool dual, bool grav,
+                        cudaStream_t st, cudaEvent_t* ev, bool learned, bool contiguous);
 }
 
 namespace {
@@ -249,7 +248,6 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   a.fflux = planes + (size_t)ppm::kFaceVars * (size_t)a.plane;
 
   // a batch of one grid: its record and block prefix tables go into the descriptor area
-  const int64_t march_blocks = (a.npencils + ppm::kMarchThreads - 1) / ppm::kMarchThreads;
   const int64_t riemann_blocks =
       (int64_t)(a.ie - a.is + 2) * ((a.npencils + ppm::kRiemannThreads - 1) / ppm::kRiemannThreads);
   const bool transport = ppm::use_transport(a.npencils * a.n);
@@ -258,12 +256,11 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   ppm::set_uniform(a, in->cell_width[dim], table.data());
   const int64_t seg_blocks = ppm::segment_blocks(a, a.pw_log2);
   const int64_t upd_blocks = ppm::segment_blocks(a, a.uw_log2);
-  const int64_t mpre[2] = {0, march_blocks}, rpre[2] = {0, riemann_blocks},
-                gpre[2] = {0, seg_blocks}, upre[2] = {0, upd_blocks};
+  const int64_t rpre[2] = {0, riemann_blocks}, gpre[2] = {0, seg_blocks},
+                upre[2] = {0, upd_blocks};
   unsigned char img[kStaticDescBytes];
   std::memset(img, 0, sizeof(img));
   std::memcpy(img, &a, sizeof(a));
-  std::memcpy(img + 768, mpre, sizeof(mpre));
   std::memcpy(img + 832, rpre, sizeof(rpre));
   std::memcpy(img + 896, gpre, sizeof(gpre));
   std::memcpy(img + 960, upre, sizeof(upre));
@@ -273,7 +270,6 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   B.one = a;
   B.grids = reinterpret_cast<const ppm::SweepArgs*>(desc);
   B.ngrids = 1;
-  B.march_prefix = reinterpret_cast<const int64_t*>(desc + 768);
   B.riemann_prefix = reinterpret_cast<const int64_t*>(desc + 832);
   B.seg_prefix = reinterpret_cast<const int64_t*>(desc + 896);
   B.seg_blocks = seg_blocks;
@@ -285,8 +281,8 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   B.counters = counters;
   B.flagged = reinterpret_cast<int64_t*>(planes + (size_t)(ppm::kFaceVars + ppm::kFluxVars) *
                                                       (size_t)a.plane);
-  ppm::launch_sweep_batch(B, march_blocks, riemann_blocks, p->dual_energy != 0, p->gravity != 0,
-                          st, nullptr, false, dim == 0 && a.uw_log2 >= 5);
+  ppm::launch_sweep_batch(B, riemann_blocks, p->dual_energy != 0, p->gravity != 0, st,
+                          nullptr, false, dim == 0 && a.uw_log2 >= 5);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail_cuda(e, "sweep launch");
 

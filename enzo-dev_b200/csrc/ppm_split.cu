@@ -1,10 +1,16 @@
-// ppm_split.cu -- one directional sweep as three sm_100a kernels sharing a face scratch.
+// ppm_split.cu -- one directional sweep as sm_100a kernels sharing a face scratch.
 //
-//   reconstruct_kernel  (thread per pencil, marching, two roles)  inteuler + intvar: the
-//                       12 corrected interface states of every face -> fstate
+//   reconstruct_kernel  (thread per pencil segment, marching, two roles)  inteuler + intvar:
+//                       the 12 corrected interface states of every face -> fstate
 //   riemann_kernel      (thread per face)               twoshock + flux_twoshock -> fflux
-//   update_kernel       (thread per pencil, marching)  flux_twoshock's negative-state check
-//                       with the per-cell flux_hll fallback, euler, pgas2d_dual
+//   update_kernel       (thread per pencil segment, marching)  flux_twoshock's negative-state
+//                       check, euler, pgas2d_dual
+//   transport_kernel    large two-shock batches: the v/w/ge role of the reconstruction, the
+//                       fluxes and the update in one march; the Riemann kernel then leaves
+//                       the Godunov state of each face
+//   fallback_kernel     the pencils that fail the check, with the per-cell flux_hll fallback
+//
+// and, where the run has them, corrections_kernel (slopes) and colour_kernel.
 //
 // Splitting the chain at the interface states keeps each kernel's live state small.
 // The Riemann stage -- a divergent Newton iteration with a serial chain of divides and
@@ -1171,8 +1177,8 @@ __device__ __forceinline__ Cell pipe_cell(const SweepArgs& a, const double* r) {
 // ------------------------------------------------ TMA tiles of the x sweep's update
 // The x sweep's pencils run along the contiguous axis: a warp's 32 pencils are 32 rows
 // of every field.  Plain loads fetch one sector per lane per cell; instead lane 0 of
-// each warp has the tensor-memory accelerator copy the warp's [32 pencils x 2 cells]
-// tile of every input field into shared memory, two chunks ahead, completing on an
+// each warp has the tensor-memory accelerator copy the warp's [32 pencils x kXTileCells]
+// tile of every input field into shared memory, kXBuffers - 1 chunks ahead, completing on an
 // mbarrier per buffer (no multicast; the tensor maps cover this GPU's own fields).
 // Every lane waits on the chunk's barrier (bounded: after ~1 s the warp records a
 // timeout, stops copying and drains what is in flight) and reads its own row.
@@ -1226,9 +1232,9 @@ __device__ __forceinline__ void tma_load_2d(double* dst, const CUtensorMap* map,
 }
 
 struct XTiles {
-  double* buf;                  // this warp's kXBuffers x 6 tiles [field][pencil][cell]
+  double* buf;                  // this warp's tiles [buffer][field][pencil][cell]
   uint64_t* bar;                // this warp's kXBuffers mbarriers
-  const CUtensorMap* map;       // the six tensor maps (kernel parameter space)
+  const CUtensorMap* map;       // the tensor maps of the fields (kernel parameter space)
   unsigned long long* timeouts; // the batch's kCntTimeout counter
   unsigned fields;              // bit f: input field f present
   unsigned bytes;               // bytes of one chunk (all present fields)
@@ -2762,8 +2768,8 @@ void launch_colours(const BatchArgs& B, cudaStream_t st) {
 }
 
 template <bool DUAL, bool GRAV, bool ONE>
-void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
-                   cudaStream_t st, cudaEvent_t* ev, bool learned, bool staged) {
+void launch_stages(const BatchArgs& B, int64_t riemann_blocks, cudaStream_t st,
+                   cudaEvent_t* ev, bool learned, bool staged) {
   auto mark = [&](int k) {
     if (ev) cudaEventRecord(ev[k], st);
   };
@@ -2906,26 +2912,16 @@ void launch_stages(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blo
 }
 
 template <bool DUAL, bool GRAV>
-void launch_any(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
-                cudaStream_t st, cudaEvent_t* ev, bool learned, bool staged) {
+void launch_any(const BatchArgs& B, int64_t riemann_blocks, cudaStream_t st, cudaEvent_t* ev,
+                bool learned, bool staged) {
   if (B.ngrids == 1)
-    launch_stages<DUAL, GRAV, true>(B, march_blocks, riemann_blocks, st, ev, learned, staged);
+    launch_stages<DUAL, GRAV, true>(B, riemann_blocks, st, ev, learned, staged);
   else
-    launch_stages<DUAL, GRAV, false>(B, march_blocks, riemann_blocks, st, ev, learned, staged);
+    launch_stages<DUAL, GRAV, false>(B, riemann_blocks, st, ev, learned, staged);
 }
 
 }  // namespace split
 
-// One directional sweep of every grid of a batch: five launches (six with slope
-// corrections, one more with colours; the Riemann stage by B.solver and B.presfree,
-// the reconstruction's corrections variant whenever corrections, colours or
-// PressureFree need it).  The caller provides
-// each grid's fstate / fflux / plane, the prefix tables and the flagged list, and for a
-// batch of one grid also B.one (a copy of that grid's record).  ev (optional): six
-// events recorded before each kernel and after the last.  learned: start the Newton
-// iteration from the MLP guess (every record's `guess` must point at packed weights).
-// contiguous: every grid's pencils run along the contiguous axis (sa == 1, the x
-// sweep); the update kernel then stages its stores.
 // Resident blocks per SM of the persistent two-shock stage for a block size (the grid of
 // a persistent launch is this times the SM count).
 int riemann_resident_blocks(bool dual, bool one, int threads) {
@@ -2953,14 +2949,25 @@ int riemann_resident_blocks(bool dual, bool one, int threads) {
   return n > 0 ? n : 1;
 }
 
-void launch_sweep_batch(const BatchArgs& B, int64_t march_blocks, int64_t riemann_blocks,
-                        bool dual, bool grav, cudaStream_t st, cudaEvent_t* ev, bool learned,
-                        bool contiguous) {
-  const int64_t mb = march_blocks, rb = riemann_blocks;
-  if (dual && grav) split::launch_any<true, true>(B, mb, rb, st, ev, learned, contiguous);
-  else if (dual) split::launch_any<true, false>(B, mb, rb, st, ev, learned, contiguous);
-  else if (grav) split::launch_any<false, true>(B, mb, rb, st, ev, learned, contiguous);
-  else split::launch_any<false, false>(B, mb, rb, st, ev, learned, contiguous);
+// One directional sweep of every grid of a batch: four launches on the transport path
+// (reconstruct d/p/u, Riemann, transport, fallback), otherwise five (reconstruct x2, or the
+// clearing kernel and both in one; Riemann, update, fallback); one more with slope
+// corrections, one with colours, one with the tensor-core guess pass.  The Riemann stage goes
+// by B.solver and B.presfree; the reconstruction's corrections variant serves corrections,
+// colours, PressureFree and cell widths that differ.  The caller provides each grid's
+// fstate / fflux / plane, the prefix tables and the flagged list, and for a batch of one grid
+// B.one (that grid's record).  ev (optional): six events, before each of the five stages of
+// ppm_b200_profile_stages and after the last.  learned: start the Newton iteration from the
+// MLP guess (every record's `guess` must point at packed weights).  contiguous: every grid's
+// pencils run along the contiguous axis (sa == 1, the x sweep) in whole warps; the update
+// and transport kernels then stage their stores.
+void launch_sweep_batch(const BatchArgs& B, int64_t riemann_blocks, bool dual, bool grav,
+                        cudaStream_t st, cudaEvent_t* ev, bool learned, bool contiguous) {
+  const int64_t rb = riemann_blocks;
+  if (dual && grav) split::launch_any<true, true>(B, rb, st, ev, learned, contiguous);
+  else if (dual) split::launch_any<true, false>(B, rb, st, ev, learned, contiguous);
+  else if (grav) split::launch_any<false, true>(B, rb, st, ev, learned, contiguous);
+  else split::launch_any<false, false>(B, rb, st, ev, learned, contiguous);
 }
 
 }  // namespace ppm

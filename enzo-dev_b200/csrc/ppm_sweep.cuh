@@ -169,16 +169,15 @@ enum { kMarchThreads = PPM_MARCH_THREADS, kRiemannThreads = PPM_RIEMANN_THREADS 
 // One launch over a batch of grids (an AMR level, or a single grid).  Every block
 // belongs to one grid: grid g owns blocks [prefix[g], prefix[g+1]) of a stage; a
 // block finds its grid by binary search over the prefix table.
-//   reconstruction: ceil(npencils / 2^pw_log2) blocks per grid
+//   reconstruction, corrections, colours (times the colour chunks): ceil(npencils /
+//                   2^pw_log2) blocks per grid
 //   update, transport: ceil(npencils / 2^uw_log2) blocks per grid
-//   corrections, colours: ceil(npencils / kMarchThreads) blocks per grid
 //   Riemann stage:   (ie - is + 2) * ceil(npencils / kRiemannThreads) blocks per grid
 struct BatchArgs {
   SweepArgs one;                     // the record itself when ngrids == 1 (read from the
                                      // kernel parameter space, like a plain launch)
   const SweepArgs* grids;            // device array, ngrids records
   int ngrids;
-  const int64_t* march_prefix;       // ngrids + 1
   const int64_t* seg_prefix;         // ngrids + 1 (reconstruction)
   int64_t seg_blocks = 0;
   const int64_t* upd_prefix;         // ngrids + 1 (update, transport)

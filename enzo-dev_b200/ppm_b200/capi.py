@@ -51,7 +51,7 @@ EXPORTS = (
 GUESS_WEIGHTS = 4673  # W1[6][64] b1[64] W2[64][64] b2[64] w3[64] b3
 BC_CODES = {"periodic": 0, "outflow": 1, "none": 2}  # ppm_b200_set_boundary bc_type
 
-# the five kernels of one sweep, in launch order (ppm_b200_profile_stages)
+# the five stages of one sweep, in launch order (ppm_b200_profile_stages)
 SWEEP_STAGES = ("reconstruct_dpu", "reconstruct_vwge", "riemann", "update", "fallback")
 
 _dp = C.POINTER(C.c_double)
@@ -754,7 +754,7 @@ class Context:
             raise PPMError(rc, "ppm_b200_guess_eval")
 
     def profile_stages(self):
-        """{stage: ms} of the five sweep kernels, summed over the last profile_read."""
+        """{stage: ms} of the five stages of a sweep, summed over the last profile_read."""
         arr = (C.c_double * 5)()
         rc = self.L.ppm_b200_profile_stages(self.h, arr)
         if rc != OK:
