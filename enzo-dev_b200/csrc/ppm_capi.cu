@@ -783,7 +783,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
                          ppm::use_transport(total_cells);
   const bool local_select = ppm::select_is_local(p->dual_energy != 0, p->eta1, p->eta2);
   for (int k = 0; k < ng; ++k) {
-    ppm::set_segments(rec[k], total_pencils, local_select, transport);
+    ppm::set_segments(rec[k], total_pencils, local_select, transport, ctx->sms);
     gpre[k + 1] = gpre[k] + ppm::segment_blocks(rec[k], rec[k].pw_log2);
     upre[k + 1] = upre[k] + ppm::segment_blocks(rec[k], rec[k].uw_log2);
   }
@@ -940,7 +940,7 @@ int prepare_sweep(ppm_b200_context* ctx, int dim, int position, const ppm_b200_p
   plan.B.upd_prefix = (const int64_t*)(base + off_u);
   plan.B.upd_blocks = upre[ng];
   plan.B.transport = transport ? 1 : 0;
-  plan.B.both_roles = ppm::use_both_roles(gpre[ng], transport) ? 1 : 0;
+  plan.B.both_roles = ppm::use_both_roles(gpre[ng], transport, ctx->sms) ? 1 : 0;
   plan.B.counters = (unsigned long long*)ctx->counters.p;
   plan.B.flagged = (int64_t*)(scratch + scratch_doubles);
   plan.riemann_blocks = rpre[ng];

@@ -251,8 +251,10 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   const int64_t riemann_blocks =
       (int64_t)(a.ie - a.is + 2) * ((a.npencils + ppm::kRiemannThreads - 1) / ppm::kRiemannThreads);
   const bool transport = ppm::use_transport(a.npencils * a.n);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   ppm::set_segments(a, a.npencils, ppm::select_is_local(p->dual_energy != 0, p->eta1, p->eta2),
-                    transport);
+                    transport, sms);
   ppm::set_uniform(a, in->cell_width[dim], table.data());
   const int64_t seg_blocks = ppm::segment_blocks(a, a.pw_log2);
   const int64_t upd_blocks = ppm::segment_blocks(a, a.uw_log2);
@@ -276,7 +278,7 @@ extern "C" int ppm_b200_euler_sweep_static(int dim, const ppm_b200_params* p,
   B.upd_prefix = reinterpret_cast<const int64_t*>(desc + 960);
   B.upd_blocks = upd_blocks;
   B.transport = transport ? 1 : 0;
-  B.both_roles = ppm::use_both_roles(seg_blocks, transport) ? 1 : 0;
+  B.both_roles = ppm::use_both_roles(seg_blocks, transport, sms) ? 1 : 0;
   B.uneven = a.uniform ? 0 : 1;
   B.counters = counters;
   B.flagged = reinterpret_cast<int64_t*>(planes + (size_t)(ppm::kFaceVars + ppm::kFluxVars) *

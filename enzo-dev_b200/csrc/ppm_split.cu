@@ -213,11 +213,6 @@ __global__ void __launch_bounds__(kMarchThreads) corrections_kernel(const __grid
 // dual-energy override and floors; ROLE 1 reconstructs the transverse velocities and
 // the gas energy and selects their upwind states.  Each writes its own six planes.
 // Splitting the face this way halves the live state of a marching thread.
-// Four resident blocks per SM keep a 256^3 sweep's pencils in a single wave.
-#ifndef PPM_RECON_MINBLOCKS
-#define PPM_RECON_MINBLOCKS (4 * 128 / PPM_MARCH_THREADS)
-#endif
-
 #ifndef PPM_RECON0_MINBLOCKS
 #define PPM_RECON0_MINBLOCKS PPM_RECON_MINBLOCKS
 #endif
@@ -2375,12 +2370,6 @@ __device__ __forceinline__ bool transport_pencil(const SweepArgs& a, int pid, co
   return flagged;
 }
 
-#ifndef PPM_TRANS_MINBLOCKS
-#define PPM_TRANS_MINBLOCKS (2 * 128 / PPM_MARCH_THREADS)
-#endif
-#ifndef PPM_TRANS_X_MINBLOCKS
-#define PPM_TRANS_X_MINBLOCKS (2 * 128 / PPM_MARCH_THREADS)
-#endif
 #ifndef PPM_TRANS_PIPE
 #define PPM_TRANS_PIPE 2
 #endif
@@ -2392,8 +2381,7 @@ constexpr size_t trans_smem_bytes() {
 }
 
 template <bool DUAL, bool GRAV, bool ONE, bool COR, bool STAGED, bool XT>
-__global__ void __launch_bounds__(kMarchThreads,
-                                  STAGED ? PPM_TRANS_X_MINBLOCKS : PPM_TRANS_MINBLOCKS)
+__global__ void __launch_bounds__(kMarchThreads, PPM_TRANS_MINBLOCKS)
     transport_kernel(const __grid_constant__ BatchArgs B) {
   pdl_begin();
   static_assert(!XT || (ONE && STAGED), "TMA tiles serve the x sweep of a single grid");

@@ -278,19 +278,28 @@ inline void build_coef(const double* dxi_in, int n, int is0, int ie0, std::vecto
 
 // Segments of the marching stages.  A march along a whole pencil is a serial chain of n
 // steps, so a batch with few pencils leaves the chip idle and waits for the chain: the
-// pencils are cut (powers of two) until the batch has PPM_MARCH_FILL threads or a segment is
+// pencils are cut (powers of two) until the batch has march_fill threads or a segment is
 // down to kSegMin faces, each segment repeating the few cells of its neighbours that its
 // first face and its first and last cells depend on.  Whole step, whole pencils -> cut
 // (exact build unless stated): 100 cells in one dimension 501 -> 101 us, 256x192 1608 ->
 // 161, 37x24x53 with HLLC 692 -> 240, 128^3 2703 -> 1879, 189x131x157 (tolerance) 3101 ->
-// 2404.  PPM_MARCH_FILL is the chip's resident march threads (148 SMs, 4 blocks of 128): with
+// 2404.  march_fill is the chip's resident march threads (4 blocks of 128 an SM): with
 // 2, 4 and 8 times that 128^3 measured 1865, 2168 and 2170 us in its sweeps against 1835,
 // and 189x131x157 2711, 2525 and 2980 against 2339 (below 32 pencils a block the x sweep
 // loses its staged stores); batches with more pencils than that (256^3 nearly, 512^3,
 // levels) gain nothing from more threads and pay the repeated cells.
-#ifndef PPM_MARCH_FILL
-#define PPM_MARCH_FILL (148 * 4 * 128)
+// Resident blocks per SM of the reconstruction (four keep a 256^3 sweep's pencils in a single
+// wave) and of the transport kernel.
+#ifndef PPM_RECON_MINBLOCKS
+#define PPM_RECON_MINBLOCKS (4 * 128 / PPM_MARCH_THREADS)
 #endif
+#ifndef PPM_TRANS_MINBLOCKS
+#define PPM_TRANS_MINBLOCKS (2 * 128 / PPM_MARCH_THREADS)
+#endif
+inline int64_t march_fill(int sms) { return (int64_t)sms * PPM_RECON_MINBLOCKS * kMarchThreads; }
+inline int64_t transport_fill(int sms) {
+  return (int64_t)sms * PPM_TRANS_MINBLOCKS * kMarchThreads;
+}
 #ifndef PPM_SEG_MIN
 #define PPM_SEG_MIN 4
 #endif
@@ -304,13 +313,9 @@ inline void build_coef(const double* dxi_in, int n, int is0, int ie0, std::vecto
 #endif
 inline bool use_transport(int64_t batch_cells) { return batch_cells >= PPM_TRANSPORT_CELLS; }
 // Both reconstructions in one launch, where their blocks are resident together.
-inline bool use_both_roles(int64_t seg_blocks, bool transport) {
-  return !transport && 2 * seg_blocks <= 148 * 4;
+inline bool use_both_roles(int64_t seg_blocks, bool transport, int sms) {
+  return !transport && 2 * seg_blocks <= (int64_t)sms * PPM_RECON_MINBLOCKS;
 }
-// The transport kernel's resident threads: two blocks of 128 an SM.
-#ifndef PPM_TRANS_FILL
-#define PPM_TRANS_FILL (148 * 2 * 128)
-#endif
 inline int64_t segment_blocks(const SweepArgs& a, int log_w) {
   return (a.npencils + (int64_t(1) << log_w) - 1) >> log_w;
 }
@@ -322,8 +327,8 @@ inline bool select_is_local(bool dual, double eta1, double eta2) {
 }
 // a: a record with its geometry; batch_pencils: pencils of all grids of the launch;
 // local_select: select_is_local.
-inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select,
-                         bool transport) {
+inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select, bool transport,
+                         int sms) {
   int whole = 0;
   while ((1 << whole) < kMarchThreads) ++whole;
   const int faces = a.ie - a.is + 2;
@@ -337,10 +342,10 @@ inline void set_segments(SweepArgs& a, int64_t batch_pencils, bool local_select,
     }
     return segs;
   };
-  int segs = split(PPM_MARCH_FILL, a.pw_log2);
+  int segs = split(march_fill(sms), a.pw_log2);
   a.seg_faces = (faces + segs - 1) / segs;
   if (local_select) {
-    segs = split(transport ? PPM_TRANS_FILL : PPM_MARCH_FILL, a.uw_log2);
+    segs = split(transport ? transport_fill(sms) : march_fill(sms), a.uw_log2);
   } else {
     segs = 1;
     a.uw_log2 = whole;
