@@ -183,37 +183,15 @@ def measured_peak_hbm():
     return 6650.0, "fallback 6.65 TB/s"
 
 
-def profile_file(variant, kind):
-    """The committed ncu summary of a build: the exact build's at 256^3, the tolerance
-    build's at 192^3 (per active cell, so the sizes compare)."""
-    if variant == "fast":
-        return REPO / "profiles" / "sweep_fast_turbulence192.json"
-    return REPO / "profiles" / ("sweep_fp64_turbulence256.json" if kind == "fp64"
-                                else "sweep_traffic_turbulence256.json")
-
-
-def committed_fp64(variant="exact"):
-    """FP64 warp-instructions per active cell and sweep from the committed ncu summary."""
-    f = profile_file(variant, "fp64")
-    if f.exists():
-        try:
-            d = json.loads(f.read_text())
-            return float(d["fp64_warp_inst_per_cell_sweep"]), d.get("source", "")
-        except Exception:
-            return None, ""
-    return None, ""
-
-
-def committed_traffic(variant="exact"):
-    """Per-zone-sweep DRAM bytes of the sweep kernel from the committed ncu summary."""
-    f = profile_file(variant, "traffic")
-    if f.exists():
-        try:
-            d = json.loads(f.read_text())
-            return float(d["dram_bytes_per_cell_sweep"]), d.get("source", "")
-        except Exception:
-            return None, ""
-    return None, ""
+def committed_profile(variant, key):
+    """A per-active-cell figure of the committed ncu summary of one sweep on the transport
+    path, 192^3 (dram_bytes_per_cell_sweep, fp64_warp_inst_per_cell_sweep), and its source."""
+    f = REPO / "profiles" / f"sweep_transport_{variant}_turbulence192.json"
+    try:
+        d = json.loads(f.read_text())
+        return float(d[key]), d.get("source", "")
+    except Exception:
+        return None, ""
 
 
 # ---------------------------------------------------------------- CPU reference (oracle port)
@@ -945,7 +923,11 @@ def run_ours(args):
     peak, peak_src = measured_peak_hbm()
     avg_sweep_s = sweep_ms * 1e-3 / max(nsweep, 1)
     achieved = (BYTES_PER_SWEEP_CELL + 16 * args.colours) * cells / avg_sweep_s / 1e9
-    tr, tr_src = committed_traffic(variant)
+    # the committed counts are of the transport path: two-shock, no colours, a large batch
+    counted = (args.colours == 0 and args.riemann == "twoshock"
+               and g.size >= 750_000)
+    tr, tr_src = (committed_profile(variant, "dram_bytes_per_cell_sweep") if counted
+                  else (None, ""))
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": (tr * cells if tr else None),
                 "kernel": "directional sweep (reconstruct, riemann, transport or update, fallback)",
@@ -955,7 +937,8 @@ def run_ours(args):
                 "traffic_source": tr_src or None}
     # the bound that is active: FP64 issue (64 FP64 lanes = 2 warp-instructions per SM
     # and clock), from the committed per-cell instruction count and the sampled clock
-    fp, fp_src = committed_fp64(variant)
+    fp, fp_src = (committed_profile(variant, "fp64_warp_inst_per_cell_sweep") if counted
+                  else (None, ""))
     if fp:
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 1965.0

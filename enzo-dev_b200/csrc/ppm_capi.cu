@@ -1172,11 +1172,17 @@ int prepare_elem(ppm_b200_context* ctx, int slot, const ppm_b200_params* p,
 // Copies between pageable host arrays and the device.  The driver stages such a copy through
 // its own buffers on one thread, about 12 GB/s; here up to four threads copy pieces of 512 KiB
 // between the arrays and pinned memory of the context (at most kPinnedMost, kept between
-// calls, freed with it) while the copies of other pieces run on the context's stream.  A
-// 64^3 call with six fields each way and a subgrid's fluxes, 16 cores: 3.45 -> 2.42 ms
-// (pinned or registered arrays, and calls of less than kPiecesLeast, go to the driver
-// directly as before).
-constexpr size_t kPiece = 512 << 10, kPinnedMost = size_t(64) << 20, kPiecesLeast = 4 << 20;
+// calls, freed with it) while the copies of other pieces run on the context's stream.
+// Pinned or registered arrays go to the driver directly, and so does a call of less than
+// kPiecesLeast bytes each way, or kPiecesLeastIn where nothing comes back: one way the
+// driver's copies are the faster ones up to about 20 MB, but not mixed with pieces on the
+// way back.  Driver -> pieces, 16 cores, several runs (us): time step of host fields (to the
+// device only) 40^3 (4.7 MB) 302-315 -> 471-542, 64^3 (16.5) 891-1039 -> 701-1047, 80^3 (30)
+// 1586-1644 -> 1233-1376, 128^3 9431-10599 -> 4733-5720; solve 40^3 1513-1524 -> 739-888, 64^3
+// 3555-3703 -> 1639-1938 (pieces on the way back alone: 1217-1349, 2106-2519), 128^3
+// 19671-20038 -> 9911-12118.
+constexpr size_t kPiece = 512 << 10, kPinnedMost = size_t(64) << 20;
+constexpr size_t kPiecesLeast = 4 << 20, kPiecesLeastIn = 24 << 20;
 struct HostPieces {
   struct Piece {
     unsigned char* host;
@@ -1193,8 +1199,8 @@ struct HostPieces {
 
 // Pageable memory of a size worth the threads.  Not on the per-thread default stream, which
 // is another stream in each of them: the copies would not be ordered with the kernels.
-bool pageable(const ppm_b200_context* ctx, const void* p, size_t call_bytes) {
-  if (call_bytes < kPiecesLeast || ctx->stream == cudaStreamPerThread) return false;
+bool pageable(const ppm_b200_context* ctx, const void* p, size_t call_bytes, size_t least) {
+  if (call_bytes < least || ctx->stream == cudaStreamPerThread) return false;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
@@ -1276,8 +1282,10 @@ int copy_pieces(ppm_b200_context* ctx, const HostPieces& w, bool to_device) {
 // Resolve the device field set of a grid: device pointers as given, or the context's
 // device copies of host fields (copied in here; single grid only).
 // colours: also the colour fields (the sweeps; the other entry points do not read them).
+// returns: the call copies the fields back (stage_out).
 int stage_in(ppm_b200_context* ctx, const ppm_b200_params* p, ppm_b200_grid* g, int memory,
-             FieldSet& fs, const double* acc[3], bool colours = false, bool need_acc = false) {
+             FieldSet& fs, const double* acc[3], bool colours = false, bool need_acc = false,
+             bool returns = false) {
   // the accelerations: read by the sweeps alone, which need one per axis under gravity
   const bool with_acc = need_acc && p->gravity;
   if (with_acc)
@@ -1301,7 +1309,7 @@ int stage_in(ppm_b200_context* ctx, const ppm_b200_params* p, ppm_b200_grid* g, 
   size_t call_bytes = bytes * (size_t)fs.ncol;
   for (int k = 0; k < 6; ++k) call_bytes += src[k] ? bytes : 0;
   auto bring = [&](void* dst, const void* host) -> int {
-    if (pageable(ctx, host, call_bytes)) {
+    if (pageable(ctx, host, call_bytes, returns ? kPiecesLeast : kPiecesLeastIn)) {
       pieces.add(const_cast<void*>(host), dst, bytes);
       return PPM_B200_OK;
     }
@@ -1349,7 +1357,7 @@ int stage_out(ppm_b200_context* ctx, const ppm_b200_params* p, ppm_b200_grid* g,
   size_t call_bytes = bytes * (size_t)fs.ncol;
   for (int k = 0; k < 6; ++k) call_bytes += dst[k] && fs.f[k] ? bytes : 0;
   auto send = [&](void* host, void* dev) -> int {
-    if (pageable(ctx, host, call_bytes)) {
+    if (pageable(ctx, host, call_bytes, kPiecesLeast)) {
       pieces.add(host, dev, bytes);
       return PPM_B200_OK;
     }
@@ -2075,7 +2083,7 @@ int ppm_b200_solve_ppm_de(ppm_b200_context* ctx, const ppm_b200_params* p, int c
   const long long* ggs = ggs_in ? ggs_in : zero3;
   std::vector<GridIO> io(1);
   io[0].g = g;
-  rc = stage_in(ctx, p, g, memory, io[0].user, io[0].acc, true, true);
+  rc = stage_in(ctx, p, g, memory, io[0].user, io[0].acc, true, true, true);
   if (rc) return rc;
   SolvePlan sp;
   rc = prepare_solve(ctx, p, cycle_number, io, nsub, sub, ggs, sp);
@@ -2204,7 +2212,7 @@ int ppm_b200_euler_sweep(ppm_b200_context* ctx, int dim, const ppm_b200_params* 
   const long long* ggs = ggs_in ? ggs_in : zero3;
   std::vector<GridIO> io(1);
   io[0].g = g;
-  rc = stage_in(ctx, p, g, memory, io[0].user, io[0].acc, true, true);
+  rc = stage_in(ctx, p, g, memory, io[0].user, io[0].acc, true, true, true);
   if (rc) return rc;
   rc = assign_scratch(ctx, io);
   if (rc) return rc;
@@ -2536,7 +2544,7 @@ static int correct_fluxes(ppm_b200_context* ctx, const ppm_b200_params* p, ppm_b
   CK(cudaSetDevice(ctx->device));
   GridIO io;
   io.g = g;
-  int rc = stage_in(ctx, p, g, memory, io.user, io.acc, species);
+  int rc = stage_in(ctx, p, g, memory, io.user, io.acc, species, false, true);
   if (rc) return rc;
   std::vector<double*> species_ptr;
   if (species)
@@ -2788,7 +2796,7 @@ int ppm_b200_expansion_terms(ppm_b200_context* ctx, const ppm_b200_params* p, pp
   CK(cudaSetDevice(ctx->device));
   std::vector<GridIO> io(1);
   io[0].g = g;
-  rc = stage_in(ctx, p, g, memory, io[0].user, io[0].acc);
+  rc = stage_in(ctx, p, g, memory, io[0].user, io[0].acc, false, false, true);
   if (rc) return rc;
   std::vector<FieldSet> ofs(1);
   if (old) {

@@ -46,6 +46,27 @@ def test_pageable_pinned_and_device_fields_agree(shape, ncol, grav):
     c.close()
 
 
+# calls that only read the fields: the driver's copies up to a larger size, then the pieces
+@pytest.mark.parametrize("shape", [(40, 41, 43), (64, 64, 64), (90, 91, 92)])
+def test_calls_that_only_read_host_fields(shape):
+    torch = pytest.importorskip("torch")
+    hp = H.HydroParams(gamma=5.0 / 3.0, cfl=0.4, dual=True)
+    g = H.Grid.uniform(shape)
+    f = random_state(g, hp, seed=4)
+    dev = {k: torch.from_numpy(v).cuda() for k, v in f.items()}
+    c = capi.Context(0)
+    p, pd = np.zeros(g.shape), torch.zeros(g.shape, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        assert c.compute_timestep(g, hp, f) == c.compute_timestep(g, hp, dev,
+                                                                  memory=capi.MEM_DEVICE)
+        c.compute_pressure(g, hp, f, p)
+        c.compute_pressure(g, hp, dev, pd, memory=capi.MEM_DEVICE)
+        torch.cuda.synchronize()
+        assert np.array_equal(p, pd.cpu().numpy())
+    c.close()
+
+
 # a context on a stream of the caller's: the legacy and the per-thread default stream (whose
 # handles, 1 and 2, name the calling thread's own stream) and a created one
 @pytest.mark.parametrize("stream", [1, 2, "created"])
